@@ -299,6 +299,7 @@ void build_pattern(Ctx& c) {
     c.pen_coef_host = pen_coef;
     ASEND_CUDA(cudaStreamSynchronize(s));
     build_classes(c, slot_map);
+    ++c.pattern_serial;
     c.pattern_ready = true;
 }
 

@@ -97,6 +97,7 @@ struct PcgScalars {
 
 struct MgHierarchy;
 struct LearnedState;
+struct ResidentPlan;
 
 // Quadratic tetrahedron (type 10) at s: corners 0..3, mid-edge nodes 4 (0-1),
 // 5 (1-2), 6 (0-2), 7 (0-3), 8 (1-3), 9 (2-3) (element_soln_fields.rs:229-298).
@@ -194,6 +195,8 @@ struct Ctx {
     bool shell_layered = false;
     DArr<double> d_shell_abd, d_shell_msec;
     bool pattern_ready = false, assembled = false, dynamic = false;
+    int64_t pattern_serial = 0;              // counts the patterns built
+    std::shared_ptr<ResidentPlan> resident;  // resident PCG's plan of the current pattern (k_resident.cu)
     bool modal = false;  // K and M assembled apart (c_M = 0) for the frequency job
     double dt = 0, beta = 0.25, gamma = 0.5, cM = 0;
     double cD = 0;                  // damping coefficient of the Newmark operator (dt gamma cM)
@@ -334,6 +337,14 @@ void apply_operator_device(Ctx& c, int precision, const double* d_x, double* d_y
 double time_spmv(Ctx& c, int precision, int n_launch, double* bytes);
 int pcg_solve(Ctx& c, const asend_solve_opts& o, asend_solve_stats* st, bool warm, const double* d_f,
               double* d_x, int nrhs);
+// resident PCG (k_resident.cu): whether a solve of nr right-hand sides takes
+// it, and its launch (no synchronisation).  d_sc: kMaxRhs zeroed scalar sets,
+// written at its end.
+bool resident_usable(Ctx& c, const asend_solve_opts& o, int nr);
+void resident_enqueue(Ctx& c, const asend_solve_opts& o, int pc, bool warm, const double* d_f, double* d_x, double* d_r,
+                      int nr, void* d_sc);
+void pcg_precondition(Ctx& c, int pc);  // point Jacobi or nodal blocks of the current operator
+bool resident_timed_out(Ctx& c);  // after a non-finite outcome (synchronises)
 void device_dot(Ctx& c, size_t n, const double* a, const double* b, double* d_out, double* d_part);
 void device_axpy(Ctx& c, size_t n, double alpha, const double* x, double* y);
 void adjoint_contract(Ctx& c, const double* d_a, const double* d_b, double* d_g, bool accumulate);

@@ -24,7 +24,7 @@
 #include <cstring>
 #include <vector>
 
-#include "common.cuh"
+#include "resident.cuh"
 
 namespace asend {
 namespace {
@@ -149,6 +149,22 @@ __global__ void k_adjoint_step(int n, int first, double d_ad_up, double d_ad_vp,
     rhs[i] = du - d_ad_up * an;
 }
 
+// sum over the steps s and the objective DOF k of w_k u_s[dof_k] (one CTA, a
+// fixed order), in place of one host copy per step and DOF
+__global__ void __launch_bounds__(256) k_history_objective(int n_steps, size_t step_stride, int n_obj,
+                                                           const int32_t* __restrict__ dof, const double* __restrict__ w,
+                                                           const double* __restrict__ hist, double* __restrict__ L) {
+    __shared__ double sm[32];
+    double v[1] = {0.0};
+    const int64_t tot = (int64_t)n_steps * n_obj;
+    for (int64_t i = threadIdx.x; i < tot; i += blockDim.x) {
+        const int s = (int)(i / n_obj), k = (int)(i - (int64_t)s * n_obj);
+        v[0] += w[k] * hist[(size_t)s * step_stride + dof[k]];
+    }
+    block_sum<1>(v, sm);
+    if (threadIdx.x == 0) *L = v[0];
+}
+
 __global__ void k_probe(const double* __restrict__ u, int dof, double* __restrict__ hist, int step) {
     if (threadIdx.x == 0 && blockIdx.x == 0) hist[step] = u[dof];
 }
@@ -202,7 +218,22 @@ int newmark_run(Ctx& c, const asend_solve_opts& o, int n_steps, const double* am
         ~TimeSolves() { c.time_solves = saved; }
     } time_guard{c, c.time_solves};
     c.time_solves = false;
-    for (int s = 0; s < n_steps; ++s) {
+    // small enough for the resident PCG: the whole time loop in one launch
+    const bool jac = o.precond == ASEND_PC_JACOBI || o.precond == ASEND_PC_BLOCK;
+    const bool on_device = n_steps > 0 && jac && o.rel_tol > 0.0 && resident_usable(c, o, 1);
+    if (on_device) {
+        pcg_precondition(c, o.precond);
+        DArr<double> d_amp;
+        d_amp.upload(amp, n_steps, c.stream);
+        const ResidentRun r = resident_newmark(
+            c, o, NewmarkState{n_steps, probe, c.hist_fields, c1, c2, d_f0.p, d_pen.p, d_amp.p, u.p, v.p, a.p, up.p,
+                               vp.p, ap.p, du.p, du_prev.p, hist.p, c.hist_fields > 0 ? c.d_hist.p : nullptr});
+        iters_total = r.iterations;
+        relmax = r.rel_residual;
+        status = r.nonfinite ? ASEND_NONFINITE : (r.capped ? ASEND_MAX_ITER : ASEND_OK);
+        c.last_method = o.method;
+    }
+    for (int s = 0; s < (on_device ? 0 : n_steps); ++s) {
         k_dyn_residual<<<g_rows, 128, 0, c.stream>>>(rows, n, c.A.slice_off.p, c.A.row_len.p, c.A.col.p, c.A.v64.p,
                                                       c.A.m64.p, c.cM, amp[s], d_f0.p, d_pen.p, u.p, a.p, rhs.p,
                                                       c.A.d64.n ? c.A.d64.p : nullptr, v.p, c.cD);
@@ -277,17 +308,17 @@ int newmark_adjoint(Ctx& c, const asend_solve_opts& o, int n_obj, const int32_t*
     std::vector<double> w(n, 0.0);
     double L = 0.0;
     {
-        std::vector<double> us(n);
         for (int k = 0; k < n_obj; ++k) w[obj_dof[k]] += obj_w[k];
         // L from the stored displacements at the objective DOFs
-        for (int s = 0; s < N; ++s)
-            for (int k = 0; k < n_obj; ++k) {
-                double v = 0.0;
-                ASEND_CUDA(cudaMemcpyAsync(&v, c.d_hist.p + (size_t)s * F * n + obj_dof[k], sizeof(double),
-                                           cudaMemcpyDeviceToHost, c.stream));
-                ASEND_CUDA(cudaStreamSynchronize(c.stream));
-                L += obj_w[k] * v;
-            }
+        DArr<int32_t> d_dof;
+        DArr<double> d_ow, d_L;
+        d_dof.upload(obj_dof, n_obj, c.stream);
+        d_ow.upload(obj_w, n_obj, c.stream);
+        d_L.alloc(1);
+        k_history_objective<<<1, 256, 0, c.stream>>>(N, (size_t)F * n, n_obj, d_dof.p, d_ow.p, c.d_hist.p, d_L.p);
+        ++c.launches;
+        ASEND_CUDA(cudaMemcpyAsync(&L, d_L.p, sizeof(double), cudaMemcpyDeviceToHost, c.stream));
+        ASEND_CUDA(cudaStreamSynchronize(c.stream));
     }
     DArr<double> d_w, mu, v_adj, a_adj, rhs, u_adj, gE;
     d_w.upload(w, c.stream);

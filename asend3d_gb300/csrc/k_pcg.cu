@@ -494,6 +494,20 @@ double time_spmv(Ctx& c, int precision, int n_launch, double* bytes) {
     return ms / n_launch;
 }
 
+void pcg_precondition(Ctx& c, int pc) {
+    const int n = c.A.n_rows, grid = grid_rows(n);
+    if (pc == ASEND_PC_JACOBI) {
+        if (c.dinv_epoch == c.assembly_epoch && c.d_dinv.n == (size_t)c.n_dof) return;  // once per assembly
+        c.d_dinv.alloc(c.n_dof);
+        k_jacobi<<<grid, kThreads, 0, c.stream>>>(n, c.A.slice_off.p, c.A.diag.p, c.A.v64.p, c.d_dinv.p);
+        c.dinv_epoch = c.assembly_epoch;
+    } else {
+        c.d_binv.alloc((size_t)9 * n);
+        k_block_inv<<<grid, kThreads, 0, c.stream>>>(n, c.A.slice_off.p, c.A.diag.p, c.A.v64.p, c.d_binv.p);
+    }
+    ++c.launches;
+}
+
 // Batched PCG over all load cases (chunks of up to 4 sharing one matrix read).
 int pcg_solve(Ctx& c, const asend_solve_opts& o, asend_solve_stats* st, bool warm, const double* d_f,
               double* d_x, int nrhs_all) {
@@ -535,25 +549,16 @@ int pcg_solve(Ctx& c, const asend_solve_opts& o, asend_solve_stats* st, bool war
     c.d_r.alloc(std::max(c.d_r.n, tot));
     const int grid = grid_rows(n);
     c.d_partials.alloc((size_t)grid * kMaxRhs * 3);
-    // preconditioner
-    if (pc == ASEND_PC_JACOBI) {
-        if (c.dinv_epoch != c.assembly_epoch || c.d_dinv.n != (size_t)nd) {  // once per assembly
-            c.d_dinv.alloc(nd);
-            k_jacobi<<<grid, kThreads, 0, c.stream>>>(n, c.A.slice_off.p, c.A.diag.p, c.A.v64.p, c.d_dinv.p);
-            ++c.launches;
-            c.dinv_epoch = c.assembly_epoch;
-        }
-    } else {
+    if (use_learned) {
         c.d_binv.alloc((size_t)9 * n);
-        if (use_learned) {
-            learned_blocks(c, c.d_binv.p, true);
-        } else {
-            k_block_inv<<<grid, kThreads, 0, c.stream>>>(n, c.A.slice_off.p, c.A.diag.p, c.A.v64.p, c.d_binv.p);
-            ++c.launches;
-        }
+        learned_blocks(c, c.d_binv.p, true);
+    } else {
+        pcg_precondition(c, pc);
     }
     const bool mixed = o.method == ASEND_METHOD_MIXED;
-    if (mixed) {
+    const bool resident = resident_usable(c, o, std::min(kMaxRhs, nrhs_all));
+    if (resident) {  // direction and A p stay on chip
+    } else if (mixed) {
         c.d_p32.alloc((size_t)kMaxRhs * 4 * n);
         c.d_ap32.alloc((size_t)kMaxRhs * nd);
     } else {  // FP64: 2 x double2 per node; split: hi + lo float4 per node (same bytes)
@@ -579,6 +584,25 @@ int pcg_solve(Ctx& c, const asend_solve_opts& o, asend_solve_stats* st, bool war
     if (c.time_solves) ASEND_CUDA(cudaEventRecord(c.ev0, c.stream));
     for (int r0 = 0; r0 < nrhs_all; r0 += kMaxRhs) {
         const int nr = std::min(kMaxRhs, nrhs_all - r0);
+        if (resident) {  // the whole solve in one launch
+            ASEND_CUDA(cudaMemsetAsync(d_sc_p, 0, sc_need, c.stream));
+            resident_enqueue(c, o, pc, warm, d_f + (size_t)r0 * nd, d_x + (size_t)r0 * nd, c.d_r.p + (size_t)r0 * nd, nr,
+                             d_sc_p);
+            ASEND_CUDA(cudaMemcpyAsync(h_sc, d_sc_p, sc_bytes, cudaMemcpyDeviceToHost, c.stream));
+            ASEND_CUDA(cudaStreamSynchronize(c.stream));
+            for (int q = 0; q < nr; ++q) {
+                const RhsScalars& s = h_sc[q];
+                iters_max = std::max(iters_max, (int)s.iter);
+                repl_total += s.n_repl;
+                if (s.nonfinite) status = ASEND_NONFINITE;
+                if (s.bb == 0.0) continue;
+                relres_max = std::max(relres_max, std::sqrt(s.rr_last_true / s.bb));
+                if (!s.finished) status = std::max(status, (int)ASEND_MAX_ITER);
+            }
+            if (status == ASEND_NONFINITE && resident_timed_out(c))
+                throw CudaError("a grid-wide wait of the resident PCG ran out");
+            continue;
+        }
         Launcher L{c, PcgArgs{}, o.method, pc, nr};
         PcgArgs& a = L.a;
         std::memset(&a, 0, sizeof(PcgArgs));  // padding too: the bytes key the cached graph
