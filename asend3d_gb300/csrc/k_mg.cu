@@ -19,7 +19,7 @@
 //    rediscretised coarse hex8 grids it does not lock in bending;
 //  * penalty constraints enter coarse levels lumped: pen_c = P^T pen_f row sums;
 //  * smoothing: one pre- and one post-sweep of damped nodal block Jacobi;
-//  * coarsest level: explicit inverse (Gauss-Jordan, one CTA);
+//  * coarsest level: explicit inverse (Gauss-Jordan, one cluster a block);
 //  * all level arithmetic in FP32; the outer CG keeps the FP64 operator,
 //    FP64 vectors and dots, and uses the Polak-Ribiere (flexible) beta
 //    beta = -alpha (z . Ap) / (r_old . z_old), which tolerates the FP32
@@ -30,6 +30,8 @@
 #include <cmath>
 #include <memory>
 #include <utility>
+
+#include <cooperative_groups.h>
 
 #include "pcg_common.cuh"
 
@@ -151,9 +153,6 @@ void launch_k(const Ctx& c, void (*k)(KArgs...), int grid, int block, size_t sme
 // classes up to which the first coarsening uses projected class matrices
 // (27 x 576 floats each, 62 KB)
 constexpr int kMaxChildClasses = 512;
-// dynamic shared memory of the blocked coarsest inverse (227 KB per CTA less
-// the 4 KB panel inverse and static data)
-constexpr size_t kGjSmem = 220 * 1024;
 
 __device__ __forceinline__ int nid(int i, int j, int k, int ny, int nz) { return (i * (ny + 1) + j) * (nz + 1) + k; }
 
@@ -449,7 +448,7 @@ __global__ void k_smoother_blocks(int n_rows, const int64_t* __restrict__ slice_
 
 // Coarsest level: one dense matrix per block (n_b = 3 x the block's nodes,
 // at offset dense0), filled row by row (one CTA per node row), then inverted
-// in place by Gauss-Jordan (SPD, no pivoting), one CTA per block.
+// in place by Gauss-Jordan (SPD, no pivoting), one cluster per block.
 __global__ void k_dense_build(int n_rows, const int64_t* __restrict__ slice_off, const uint8_t* __restrict__ row_len,
                               const int32_t* __restrict__ col, const float* __restrict__ vals, LevelView cv,
                               const int32_t* __restrict__ pre_node, float* __restrict__ D) {
@@ -471,68 +470,21 @@ __global__ void k_dense_build(int n_rows, const int64_t* __restrict__ slice_off,
     }
 }
 
-// In-place Gauss-Jordan inverse of block blockIdx.x's matrix.  The 1024
-// threads form a 32 x 32 grid; thread (ty, tx) updates the entries (ty + 32i,
-// tx + 32j), so consecutive threads touch consecutive addresses and no index
-// is divided.  With in_smem the matrix lives in dynamic shared memory for
-// the n steps (n <= 234); otherwise it is updated in global memory.
-__global__ void __launch_bounds__(1024) k_gauss_jordan(LevelView cv, float* __restrict__ Dall, int in_smem) {
-    extern __shared__ float dyn[];
-    __shared__ float colk[1024];
-    __shared__ float rowk[1024];
-    const BlkDev& d = cv.blk[blockIdx.x];
-    const int n = 3 * (d.nx + 1) * (d.ny + 1) * (d.nz + 1);
-    float* Ag = Dall + d.dense0;
-    float* A = in_smem ? dyn : Ag;
-    if (in_smem) {
-        for (int q = threadIdx.x; q < n * n; q += blockDim.x) dyn[q] = Ag[q];
-        __syncthreads();
-    }
-    const int tx = threadIdx.x & 31, ty = threadIdx.x >> 5;
-    for (int k = 0; k < n; ++k) {
-        const float inv = 1.f / A[(size_t)k * n + k];
-        for (int i = threadIdx.x; i < n; i += blockDim.x) {
-            colk[i] = A[(size_t)i * n + k];
-            rowk[i] = A[(size_t)k * n + i] * inv;
-        }
-        __syncthreads();
-        for (int i = ty; i < n; i += 32) {
-            const float ci = colk[i];
-            float* Ar = A + (size_t)i * n;
-            if (i == k) {
-                for (int j = tx; j < n; j += 32) Ar[j] = (j == k) ? inv : rowk[j];
-            } else {
-                for (int j = tx; j < n; j += 32) Ar[j] = (j == k) ? -ci * inv : fmaf(-ci, rowk[j], Ar[j]);
-            }
-        }
-        __syncthreads();
-    }
-    // the exact inverse is symmetric: average the FP32 rounding asymmetry out,
-    // so the coarse solve (and with it the V-cycle) is a symmetric operator
-    for (int q = threadIdx.x; q < n * n; q += blockDim.x) {
-        const int i = q / n, j = q % n;
-        if (j <= i) continue;
-        const float v = 0.5f * (A[(size_t)i * n + j] + A[(size_t)j * n + i]);
-        A[(size_t)i * n + j] = v;
-        A[(size_t)j * n + i] = v;
-    }
-    __syncthreads();
-    if (in_smem)
-        for (int q = threadIdx.x; q < n * n; q += blockDim.x) Ag[q] = dyn[q];
-}
-
-// Blocked Gauss-Jordan inverse in shared memory (row stride ld, a multiple
-// of 4), 32-column panels: for panel P (rows / columns k0..k0+kb)
-//   D = A_PP^-1 (warp 0, in registers, lane = row), R = D A_P,rest (row
-//   panel), A_rest,rest -= A_rest,P R, A_rest,P = -A_rest,P D, A_PP = D,
-// which is the unblocked in-place elimination regrouped, so a panel costs
-// four CTA barriers instead of 2 kb, and the trailing update runs as 2 x 4
-// register tiles.  No pivoting: the coarse operators are SPD.
-__device__ __forceinline__ void gj_panel_inverse(float* __restrict__ A, int ld, int k0, int kb, float* __restrict__ D) {
+// Coarsest inverse: blocked Gauss-Jordan of one block's matrix (n <= 256, which
+// the coarsening rule guarantees) by a cluster of 8 CTAs, CTA r holding rows
+// 32 r .. 32 r + 31 in shared memory.  For panel P (rows / columns k0 .. k0 +
+// 31) its owner forms D = A_PP^-1 (warp 0, in registers, lane = row) and R = D
+// A_P (R_PP = D); the others copy R through distributed shared memory and set
+// A_i = A_i - A_iP R with the panel columns of A_i cleared first, which is the
+// unblocked in-place elimination regrouped.  No pivoting: the coarse operators
+// are SPD.  Bound by the serial panels; one CTA with the whole matrix took 283
+// us at n = 216, and above 234 (no longer in one CTA's shared memory) 3,460 us
+// column by column in global memory at n = 243.
+__device__ __forceinline__ void gj_panel_inverse(const float* __restrict__ rows, int ld, int k0, int kb, float* __restrict__ D) {
     const int lane = threadIdx.x & 31;
     float d[32];
 #pragma unroll
-    for (int j = 0; j < 32; ++j) d[j] = (lane < kb && j < kb) ? A[(size_t)(k0 + lane) * ld + k0 + j] : (lane == j ? 1.f : 0.f);
+    for (int j = 0; j < 32; ++j) d[j] = (lane < kb && j < kb) ? rows[lane * ld + k0 + j] : (lane == j ? 1.f : 0.f);
 #pragma unroll
     for (int p = 0; p < 32; ++p) {
         const float piv = __shfl_sync(0xffffffffu, d[p], p);
@@ -553,99 +505,95 @@ __device__ __forceinline__ void gj_panel_inverse(float* __restrict__ A, int ld, 
     for (int j = 0; j < 32; ++j) D[lane * 32 + j] = d[j];
 }
 
-__global__ void __launch_bounds__(1024) k_gauss_jordan_blk(LevelView cv, float* __restrict__ Dall, int ld) {
-    extern __shared__ float dyn[];
-    __shared__ float D[32 * 32];
-    const BlkDev& dv = cv.blk[blockIdx.x];
+constexpr int kGjCtas = 8, kGjN = 256, kGjThreads = 256;
+constexpr size_t kGjSmem = sizeof(float) * (2 * 32 * kGjN + 32 * 32);
+
+__global__ void __cluster_dims__(kGjCtas, 1, 1) __launch_bounds__(kGjThreads)
+k_gauss_jordan(LevelView cv, float* __restrict__ Dall) {
+    extern __shared__ __align__(16) float gj[];
+    float* A = gj;                  // own 32 rows
+    float* R = gj + 32 * kGjN;      // the panel's rows
+    float* D = gj + 2 * 32 * kGjN;
+    cooperative_groups::cluster_group cl = cooperative_groups::this_cluster();
+    const int r = (int)cl.block_rank(), t = threadIdx.x;
+    const BlkDev& dv = cv.blk[blockIdx.x / kGjCtas];
     const int n = 3 * (dv.nx + 1) * (dv.ny + 1) * (dv.nz + 1);
     float* Ag = Dall + dv.dense0;
-    float* A = dyn;
-    const int t = threadIdx.x, nt = blockDim.x;
-    for (int q = t; q < n * ld; q += nt) {
-        const int i = q / ld, j = q % ld;
-        A[q] = (j < n) ? Ag[(size_t)i * n + j] : 0.f;
+    for (int q = t; q < 32 * kGjN; q += kGjThreads) {
+        const int i = 32 * r + q / kGjN, j = q % kGjN;
+        A[q] = (i < n && j < n) ? Ag[(size_t)i * n + j] : 0.f;
     }
     __syncthreads();
-    for (int k0 = 0; k0 < n; k0 += 32) {
-        const int kb = min(32, n - k0);
-        if (t < 32) gj_panel_inverse(A, ld, k0, kb, D);
-        __syncthreads();
-        // row panel: A_P,j = D A_P,j for the columns j outside the panel
-        for (int j = t; j < n; j += nt) {
-            if (j >= k0 && j < k0 + kb) continue;
+    const int i0 = 4 * (t >> 5), j0 = 8 * (t & 31);  // this thread's 4 x 8 tile of the own rows
+    for (int P = 0; 32 * P < n; ++P) {
+        const int k0 = 32 * P, kb = min(32, n - k0);
+        if (r == P) {
+            if (t < 32) gj_panel_inverse(A, kGjN, k0, kb, D);
+            __syncthreads();
             float a[32];
 #pragma unroll
-            for (int q = 0; q < 32; ++q) a[q] = (q < kb) ? A[(size_t)(k0 + q) * ld + j] : 0.f;
+            for (int q = 0; q < 32; ++q) a[q] = A[q * kGjN + t];
+            const bool in_p = t >= k0 && t < k0 + 32;
 #pragma unroll 4
-            for (int p = 0; p < kb; ++p) {
+            for (int p = 0; p < 32; ++p) {
                 float s = 0.f;
 #pragma unroll
                 for (int q = 0; q < 32; ++q) s = fmaf(D[p * 32 + q], a[q], s);
-                A[(size_t)(k0 + p) * ld + j] = s;
+                R[p * kGjN + t] = in_p ? D[p * 32 + t - k0] : s;
             }
         }
-        __syncthreads();
-        // trailing block: A_ij -= sum_q A_iq R_qj, rows and columns outside
-        // the panel, 2 x 4 tiles (columns in float4 groups; ld % 4 == 0)
-        const int ncg = ld / 4, nrg = (n + 1) / 2;
-        for (int tile = t; tile < nrg * ncg; tile += nt) {
-            const int i0 = 2 * (tile / ncg), j0 = 4 * (tile % ncg);
-            if (j0 >= n) continue;
-            const bool r0 = (i0 < k0 || i0 >= k0 + kb), r1 = (i0 + 1 < n) && (i0 + 1 < k0 || i0 + 1 >= k0 + kb);
-            if (!r0 && !r1) continue;
-            float4 acc0 = *reinterpret_cast<const float4*>(A + (size_t)i0 * ld + j0);
-            float4 acc1 = (i0 + 1 < n) ? *reinterpret_cast<const float4*>(A + (size_t)(i0 + 1) * ld + j0)
-                                       : make_float4(0.f, 0.f, 0.f, 0.f);
-            for (int q = 0; q < kb; ++q) {
-                const float4 rq = *reinterpret_cast<const float4*>(A + (size_t)(k0 + q) * ld + j0);
-                const float a0 = A[(size_t)i0 * ld + k0 + q];
-                const float a1 = (i0 + 1 < n) ? A[(size_t)(i0 + 1) * ld + k0 + q] : 0.f;
-                acc0.x = fmaf(-a0, rq.x, acc0.x); acc0.y = fmaf(-a0, rq.y, acc0.y);
-                acc0.z = fmaf(-a0, rq.z, acc0.z); acc0.w = fmaf(-a0, rq.w, acc0.w);
-                acc1.x = fmaf(-a1, rq.x, acc1.x); acc1.y = fmaf(-a1, rq.y, acc1.y);
-                acc1.z = fmaf(-a1, rq.z, acc1.z); acc1.w = fmaf(-a1, rq.w, acc1.w);
-            }
-            // columns of the panel keep their old values here (they are
-            // rewritten below); columns beyond n stay zero
-            float* o0 = A + (size_t)i0 * ld + j0;
-            float* o1 = A + (size_t)(i0 + 1) * ld + j0;
-            const float v0[4] = {acc0.x, acc0.y, acc0.z, acc0.w}, v1[4] = {acc1.x, acc1.y, acc1.z, acc1.w};
+        cl.sync();  // R is complete
+        if (r != P) {
+            const float4* src = reinterpret_cast<const float4*>(cl.map_shared_rank(R, P));
 #pragma unroll
-            for (int c = 0; c < 4; ++c) {
-                const int j = j0 + c;
-                if (j >= n || (j >= k0 && j < k0 + kb)) continue;
-                if (r0) o0[c] = v0[c];
-                if (r1) o1[c] = v1[c];
-            }
+            for (int q = 0; q < 32 * kGjN / 4 / kGjThreads; ++q)
+                reinterpret_cast<float4*>(R)[q * kGjThreads + t] = src[q * kGjThreads + t];
         }
-        __syncthreads();
-        // column panel A_i,P = -A_i,P D for the rows outside the panel; the
-        // diagonal block becomes D
-        for (int i = t; i < n; i += nt) {
-            float* Ar = A + (size_t)i * ld + k0;
-            if (i >= k0 && i < k0 + kb) {
-                const int p = i - k0;
-                for (int q = 0; q < kb; ++q) Ar[q] = D[p * 32 + q];
-                continue;
-            }
-            float a[32];
+        cl.sync();  // copied: the owner's R may be overwritten with the next panel's
+        float acc[4][8];
+        if (r == P) {
 #pragma unroll
-            for (int q = 0; q < 32; ++q) a[q] = (q < kb) ? Ar[q] : 0.f;
+            for (int u = 0; u < 4; ++u)
+#pragma unroll
+                for (int w = 0; w < 8; ++w) acc[u][w] = R[(i0 + u) * kGjN + j0 + w];
+        } else {
+#pragma unroll
+            for (int u = 0; u < 4; ++u)
+#pragma unroll
+                for (int w = 0; w < 8; ++w)
+                    acc[u][w] = (j0 + w >= k0 && j0 + w < k0 + 32) ? 0.f : A[(i0 + u) * kGjN + j0 + w];
 #pragma unroll 4
-            for (int p = 0; p < kb; ++p) {
-                float s = 0.f;
+            for (int q = 0; q < 32; ++q) {
+                const float4 r0 = *reinterpret_cast<const float4*>(R + q * kGjN + j0);
+                const float4 r1 = *reinterpret_cast<const float4*>(R + q * kGjN + j0 + 4);
+                const float rv[8] = {r0.x, r0.y, r0.z, r0.w, r1.x, r1.y, r1.z, r1.w};
 #pragma unroll
-                for (int q = 0; q < 32; ++q) s = fmaf(a[q], D[q * 32 + p], s);
-                Ar[p] = -s;
+                for (int u = 0; u < 4; ++u) {
+                    const float av = A[(i0 + u) * kGjN + k0 + q];
+#pragma unroll
+                    for (int w = 0; w < 8; ++w) acc[u][w] = fmaf(-av, rv[w], acc[u][w]);
+                }
             }
         }
+        __syncthreads();  // every thread has read the panel columns of A
+#pragma unroll
+        for (int u = 0; u < 4; ++u)
+#pragma unroll
+            for (int w = 0; w < 8; ++w) A[(i0 + u) * kGjN + j0 + w] = acc[u][w];
         __syncthreads();
     }
-    // symmetrise (the exact inverse is symmetric) and store
-    for (int q = t; q < n * n; q += nt) {
-        const int i = q / n, j = q % n;
-        Ag[q] = 0.5f * (A[(size_t)i * ld + j] + A[(size_t)j * ld + i]);
+    // the exact inverse is symmetric: average the FP32 rounding asymmetry out,
+    // so the coarse solve (and with it the V-cycle) is a symmetric operator
+    cl.sync();
+    for (int q = t; q < 32 * kGjN; q += kGjThreads) {
+        const int i = 32 * r + q / kGjN, j = q % kGjN;
+        if (i >= n || j >= n || j < i) continue;
+        const float* other = cl.map_shared_rank(A, j >> 5);
+        const float v = 0.5f * (A[q] + other[(j & 31) * kGjN + i]);
+        Ag[(size_t)i * n + j] = v;
+        Ag[(size_t)j * n + i] = v;
     }
+    cl.sync();  // the other CTAs may still read this one's rows
 }
 
 // ---------------------------------------------------------------------------
@@ -2367,7 +2315,7 @@ void build_hierarchy(Ctx& c) {
         dense_tot += (size_t)nd * nd;
         H->n_coarse = std::max(H->n_coarse, nd);
     }
-    if (H->n_coarse > 1020) throw InputError("multigrid coarsest level too large");
+    if (H->n_coarse > kGjN) throw InputError("multigrid coarsest level too large");  // not by the rule above
     if (dense_tot > (size_t)INT32_MAX) throw InputError("multigrid coarsest blocks too large");
     H->dense.alloc(dense_tot);
     for (int l = 0; l < (int)H->L.size(); ++l) level_tables(c, *H, l);
@@ -2513,15 +2461,8 @@ void setup_values(Ctx& c, bool skip_l0) {
     MgLevel& Lc = *H.L.back();
     k_dense_build<<<Lc.n_nodes, 128, 0, c.stream>>>(Lc.n_nodes, Lc.A->slice_off.p, Lc.A->row_len.p, Lc.A->col.p,
                                                     Lc.A->v32.p, view_of(Lc), Lc.pre_node.p, H.dense.p);
-    const int ld = (H.n_coarse + 3) & ~3;
-    const size_t blk_smem = sizeof(float) * (size_t)H.n_coarse * ld;
-    if (blk_smem <= kGjSmem) {  // blocked elimination in shared memory
-        ASEND_CUDA(cudaFuncSetAttribute(k_gauss_jordan_blk, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                        (int)blk_smem));
-        k_gauss_jordan_blk<<<H.n_blk, 1024, blk_smem, c.stream>>>(view_of(Lc), H.dense.p, ld);
-    } else {  // larger coarsest blocks: column-by-column elimination in global memory
-        k_gauss_jordan<<<H.n_blk, 1024, 0, c.stream>>>(view_of(Lc), H.dense.p, 0);
-    }
+    ASEND_CUDA(cudaFuncSetAttribute(k_gauss_jordan, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kGjSmem));
+    k_gauss_jordan<<<H.n_blk * kGjCtas, kGjThreads, kGjSmem, c.stream>>>(view_of(Lc), H.dense.p);
     c.launches += 2;
     ASEND_CUDA(cudaGetLastError());
     H.epoch = c.assembly_epoch;
