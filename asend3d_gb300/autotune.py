@@ -84,11 +84,12 @@ def tune(solver, rel_tol=1e-8, candidates=None, give_up=3.0, repeats=2, cache: d
 def tune_product(solver, n_launch=20):
     """The fastest shape of the multigrid CG's split outer product on this
     operator: each shape's device time over n_launch back-to-back launches
-    (asend_time_mg_kernel, the kernel alone).  The shapes give bit-identical
-    results, so this changes only the time.  Installs the winner and returns
+    (asend_time_mg_kernel, the kernel alone): the default (matrix-free on
+    blocks of equal box elements) and the shapes on the assembled values, which
+    are bit-identical among each other.  Installs the winner and returns
     (variant, {variant: ms per launch})."""
     times = {}
-    for v in _lib.PRODUCT_VARIANTS:
+    for v in (_lib.PRODUCT_DEFAULT, *_lib.PRODUCT_VARIANTS):
         solver.set_product_variant(v)
         times[v] = solver.time_mg_kernel(0, _lib.METHOD_SPLIT, n_launch)[0]
     best = min(times, key=times.get)

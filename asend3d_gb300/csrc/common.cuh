@@ -98,6 +98,7 @@ struct PcgScalars {
 struct MgHierarchy;
 struct LearnedState;
 struct ResidentPlan;
+struct BoxPlan;
 
 // Quadratic tetrahedron (type 10) at s: corners 0..3, mid-edge nodes 4 (0-1),
 // 5 (1-2), 6 (0-2), 7 (0-3), 8 (1-3), 9 (2-3) (element_soln_fields.rs:229-298).
@@ -224,6 +225,10 @@ struct Ctx {
     int cls_type = 0, n_cls = 0;
     std::vector<int32_t> h_cls_of;
     DArr<int32_t> d_cls_of;          // class of each element
+    std::vector<uint8_t> cls_box;    // classes whose matrix has a box's three reflections (to 2^-48)
+    bool class_sum = false;          // the operator is sum E_e K^_cls + penalties (+ unit rows), unmodified
+    bool class_pairs = false;        // ... with K^ rounded to FP32 pairs (split-only assembly)
+    std::shared_ptr<BoxPlan> box;    // matrix-free products on such blocks (k_box.cu)
     DArr<double> cls_ke, cls_me;     // [n_cls][(3 nn)^2] stiffness, [n_cls][nn nn] mass (FP64)
     DArr<float> cls_ke32;            // FP32 copy of cls_ke (multigrid coarsening)
     DArr<float2> cls_ke2;            // cls_ke as FP32 pairs (split-only assembly)

@@ -697,6 +697,32 @@ void launch_colours(Ctx& c, T* vals, double* mvals, double cM, const ElemExtra& 
 
 }  // namespace
 
+// Whether K is unchanged by the three reflections of a box element's axes (a
+// corner goes to its mirror image, the component along the axis changes sign)
+// to 2^-48 of its largest entry, the resolution of the pair values: the
+// matrix-free products (k_box.cu) rely on it.
+bool has_reflections(const double* K) {
+    static const int corner[8][3] = {{0, 0, 0}, {1, 0, 0}, {1, 1, 0}, {0, 1, 0},
+                                     {0, 0, 1}, {1, 0, 1}, {1, 1, 1}, {0, 1, 1}};
+    static const int at[8] = {0, 1, 3, 2, 4, 5, 7, 6};  // corner with offsets (x, y, z): at[x + 2 y + 4 z]
+    double mx = 0.0;
+    for (int i = 0; i < 576; ++i) mx = std::max(mx, std::fabs(K[i]));
+    for (int ax = 0; ax < 3; ++ax) {
+        int image[8];
+        for (int a = 0; a < 8; ++a)
+            image[a] = at[(corner[a][0] ^ (ax == 0)) + 2 * (corner[a][1] ^ (ax == 1)) + 4 * (corner[a][2] ^ (ax == 2))];
+        for (int a = 0; a < 8; ++a)
+            for (int c = 0; c < 3; ++c)
+                for (int b = 0; b < 8; ++b)
+                    for (int d = 0; d < 3; ++d) {
+                        const double v = K[(3 * image[a] + c) * 24 + 3 * image[b] + d] *
+                                         (((c == ax) != (d == ax)) ? -1.0 : 1.0);
+                        if (!(std::fabs(v - K[(3 * a + c) * 24 + 3 * b + d]) <= 3.6e-15 * mx)) return false;
+                    }
+    }
+    return true;
+}
+
 // Geometry classes of a hex8 / brickIM mesh and the per-slot gather lists.
 // Two elements share a class when their corner offsets from corner 0 agree
 // to 1e-12 of the element size and their Poisson ratios are equal; their
@@ -712,6 +738,7 @@ void build_classes(Ctx& c, const std::vector<int32_t>& slot_map) {
     c.cls_me.release();
     c.cls_ke32.release();
     c.cls_ke2.release();
+    c.cls_box.clear();
     c.d_cls_of.release();
     c.d_gat_ptr.release();
     c.d_gat.release();
@@ -807,6 +834,8 @@ void build_classes(Ctx& c, const std::vector<int32_t>& slot_map) {
         ASEND_CUDA(cudaMemcpyAsync(k64.data(), c.cls_ke.p, sizeof(double) * k64.size(), cudaMemcpyDeviceToHost,
                                    c.stream));
         ASEND_CUDA(cudaStreamSynchronize(c.stream));
+        c.cls_box.assign(ncl, 0);
+        for (int cl = 0; cl < ncl; ++cl) c.cls_box[cl] = has_reflections(&k64[(size_t)cl * 576]);
         std::vector<float> k32(k64.begin(), k64.end());
         c.cls_ke32.upload(k32, c.stream);
     }
@@ -1026,6 +1055,8 @@ void assemble_operator(Ctx& c, int precision) {
     ASEND_CUDA(cudaEventElapsedTime(&ms, c.ev0, c.ev1));
     c.assembled_precision = precision;
     c.v64_valid = !split_only;
+    c.class_sum = (gather || split_only) && c.cM == 0.0;
+    c.class_pairs = split_only;
     ++c.assembly_epoch;
     c.last_assemble_ms = ms;
 }

@@ -369,13 +369,16 @@ int eigen_solve(Ctx& c, const asend_eigen_opts& eo, double* eig_out, double* fre
         c.launches += 2;
         ++c.assembly_epoch;  // preconditioners and multigrid levels follow the shifted values
     }
+    const bool class_sum = c.class_sum;
+    if (shift != 0.0) c.class_sum = false;
     struct Restore {  // puts the unshifted diagonal back, also on an exception
         Ctx& c;
         DArr<double>& saved;
-        bool on;
+        bool on, class_sum;
         void run() {
             if (!on) return;
             on = false;
+            c.class_sum = class_sum;
             const int rows = c.A.n_rows;
             k_diag_entries<<<(rows + 127) / 128, 128, 0, c.stream>>>(rows, c.A.slice_off.p, c.A.diag.p, c.A.v64.p,
                                                                     c.A.v32.p, c.A.v32lo.p, nullptr, saved.p, 2);
@@ -383,7 +386,7 @@ int eigen_solve(Ctx& c, const asend_eigen_opts& eo, double* eig_out, double* fre
             ++c.assembly_epoch;
         }
         ~Restore() { run(); }
-    } restore{c, saved, shift != 0.0};
+    } restore{c, saved, shift != 0.0, class_sum};
 
     const int cols = m_max + b;
     Basis B(c, n, cols);

@@ -33,6 +33,7 @@
 
 #include <cooperative_groups.h>
 
+#include "box.cuh"
 #include "pcg_common.cuh"
 
 namespace asend {
@@ -113,7 +114,17 @@ struct MgHierarchy {
     DArr<float> pow_omega;        // damping in use per level
     bool safe_damping = false;    // omega from the guaranteed bound (after a failed solve)
     int tail = 0;                 // first level of the fused coarse tail (0: none)
+    BoxPlan* box = nullptr;       // matrix-free finest products of the current operator (or none)
+    bool box_cycle = false;       // V-cycles take them, too (inside the CG; a V-cycle that a caller sees
+                                  // keeps the assembled values)
     DArr<float> vl_q, vl_mw, vl_t4, vl_r2, vl_w;  // learned-smoother training vectors
+};
+
+// Matrix-free finest products in the V-cycles of a scope.
+struct BoxCycle {
+    MgHierarchy& H;
+    explicit BoxCycle(MgHierarchy& h) : H(h) { H.box_cycle = true; }
+    ~BoxCycle() { H.box_cycle = false; }
 };
 
 constexpr int kPowSteps = 10;      // from a hashed start vector
@@ -505,7 +516,7 @@ __device__ __forceinline__ void gj_panel_inverse(const float* __restrict__ rows,
     for (int j = 0; j < 32; ++j) D[lane * 32 + j] = d[j];
 }
 
-constexpr int kGjCtas = 8, kGjN = 256, kGjThreads = 256;
+constexpr int kGjCtas = 8, kGjN = 256, kGjThreads = 256, kGjBlocked = 234;
 constexpr size_t kGjSmem = sizeof(float) * (2 * 32 * kGjN + 32 * 32);
 
 __global__ void __cluster_dims__(kGjCtas, 1, 1) __launch_bounds__(kGjThreads)
@@ -525,7 +536,38 @@ k_gauss_jordan(LevelView cv, float* __restrict__ Dall) {
     }
     __syncthreads();
     const int i0 = 4 * (t >> 5), j0 = 8 * (t & 31);  // this thread's 4 x 8 tile of the own rows
-    for (int P = 0; 32 * P < n; ++P) {
+    if (n > kGjBlocked) {
+        // the owner of row k stores it into every CTA's copy, two alternating
+        for (int k = 0; k < n; ++k) {
+            float* row = R + (k & 1) * kGjN;
+            if (r == k >> 5) {
+                const float v = A[(k & 31) * kGjN + t];
+#pragma unroll
+                for (int q = 0; q < kGjCtas; ++q) cl.map_shared_rank(row, q)[t] = v;
+            }
+            cl.sync();
+            const float inv = 1.f / row[k];
+            float rk[8];
+#pragma unroll
+            for (int w = 0; w < 8; ++w) rk[w] = row[j0 + w] * inv;
+            float ci[4];
+#pragma unroll
+            for (int u = 0; u < 4; ++u) ci[u] = A[(i0 + u) * kGjN + k];
+            __syncthreads();  // every thread has read column k
+#pragma unroll
+            for (int u = 0; u < 4; ++u) {
+                const bool pivot = 32 * r + i0 + u == k;
+#pragma unroll
+                for (int w = 0; w < 8; ++w) {
+                    float* e = A + (i0 + u) * kGjN + j0 + w;
+                    if (pivot) *e = j0 + w == k ? inv : rk[w];
+                    else *e = j0 + w == k ? -ci[u] * inv : fmaf(-ci[u], rk[w], *e);
+                }
+            }
+            __syncthreads();
+        }
+    }
+    for (int P = 0; n <= kGjBlocked && 32 * P < n; ++P) {
         const int k0 = 32 * P, kb = min(32, n - k0);
         if (r == P) {
             if (t < 32) gj_panel_inverse(A, kGjN, k0, kb, D);
@@ -1483,14 +1525,6 @@ __device__ __forceinline__ F2 pair_ap_dot(const PcgArgs& A, int row, const F2 (&
     return acc;
 }
 
-__device__ __forceinline__ void set_alpha(RhsScalars& s, double pAp) {
-    s.pAp = pAp;
-    s.alpha = s.rz / s.pAp;
-    const F2 a = f2_of(s.alpha);
-    s.alpha2[0] = a.h;
-    s.alpha2[1] = a.l;
-}
-
 // The register-fed split product with the pair epilogue.
 __global__ void __launch_bounds__(kThreads) k_mg_spmv_dot_pair(MgPcg M) {
     pdl_begin();
@@ -1778,8 +1812,10 @@ __global__ void __launch_bounds__(kThreads) k_mg_spmv_dot_staged(MgPcg M) {
     if (last_block_reduce<1, 1>(A, d, 0, tot) && threadIdx.x == 0) set_alpha(Sc[0], tot[0][0]);
 }
 
-// Launch of the split outer product in one of its shapes (ASEND_PRODUCT_*):
-// register-fed, or staged with G groups per stage and S stages per warp.
+// Launch of the split outer product: by default matrix-free where the blocks
+// allow it; in one of its shapes on the assembled values (ASEND_PRODUCT_*)
+// otherwise or when one is asked for: register-fed, or staged with G groups per
+// stage and S stages per warp.
 template <int G, int S>
 void launch_staged(const Ctx& c, const MgPcg& M, int grid) {
     launch_k(c, k_mg_spmv_dot_staged<G, S>, grid, kThreads, SplitStage<G, S>::smem(kThreads), M);
@@ -1804,7 +1840,11 @@ void product_attrs() {
     if (dev >= 0 && dev < 64) done[dev] = true;
 }
 
-void launch_split_product(const Ctx& c, const MgPcg& M, int grid) {
+void launch_split_product(Ctx& c, const MgPcg& M, int grid) {
+    if (c.product_variant == ASEND_PRODUCT_DEFAULT && c.mg->box) {  // 36.8 against 118 us (200 x 40 x 40)
+        box_product(c, *c.mg->box, M.a);
+        return;
+    }
     switch (c.product_variant) {
         case ASEND_PRODUCT_REGISTERS: launch_k(c, k_mg_spmv_dot_pair, grid, kThreads, 0, M); break;
         case ASEND_PRODUCT_STAGED_3x2: launch_staged<3, 2>(c, M, grid); break;
@@ -2185,6 +2225,7 @@ void build_hierarchy(Ctx& c) {
     if (b0.empty())
         throw InputError("multigrid needs structured hex8 / brickIM blocks (asend_set_block_structure or "
                          "asend_set_instance_blocks)");
+    c.box.reset();  // (the blocks may be others than the last plan's)
     auto H = std::make_shared<MgHierarchy>();
     H->n_blk = (int)b0.size();
     auto L0 = std::make_unique<MgLevel>();
@@ -2357,8 +2398,10 @@ void damp_smoother(Ctx& c, int l) {
         ASEND_CUDA(cudaMemcpyAsync(xa, L.pow_vec.p, sizeof(float) * 4 * L.n_nodes, cudaMemcpyDeviceToDevice,
                                    c.stream));
     k_pow_init<<<g, kT, 0, c.stream>>>(L.n_nodes, xa, nrm, warm ? 0 : 1);
+    BoxPlan* box = l == 0 ? H.box : nullptr;
     for (int k = 0; k < steps; ++k) {
-        k_pow_step<<<g, kT, 0, c.stream>>>(sbview(L), L.binv.p, xa, xb, nrm, k, H.pow_part.p, tk);
+        if (box) box_power(c, *box, L.binv.p, xa, xb, nrm, k, H.pow_part.p, tk);
+        else k_pow_step<<<g, kT, 0, c.stream>>>(sbview(L), L.binv.p, xa, xb, nrm, k, H.pow_part.p, tk);
         std::swap(xa, xb);
     }
     ASEND_CUDA(cudaMemcpyAsync(L.pow_vec.p, xa, sizeof(float) * 4 * L.n_nodes, cudaMemcpyDeviceToDevice, c.stream));
@@ -2397,7 +2440,7 @@ void setup_values(Ctx& c, bool skip_l0) {
     H.pow_bound.zero(c.stream);
     H.pow_omega.zero(c.stream);
     H.pow_ticket.alloc((size_t)n_lev * kPowSteps);
-    H.pow_part.alloc((size_t)grid_of(H.L[0]->n_nodes));
+    H.pow_part.alloc((size_t)std::max(grid_of(H.L[0]->n_nodes), H.box ? box_ctas(*H.box) : 0));
     {
         std::vector<double> sf(H.n_blk, c.sf);
         if (c.n_inst > 1 && (int)c.sf_inst.size() == H.n_blk) sf = c.sf_inst;
@@ -2512,6 +2555,10 @@ int lanes_for(int n_rows) {
 constexpr int kStagedRows = 8192;
 
 void level_resid(Ctx& c, MgLevel& L, const Control* ctl) {
+    if (c.mg->box && c.mg->box_cycle && &L == c.mg->L[0].get()) {
+        box_resid(c, *c.mg->box, L.b.p, reinterpret_cast<const float4*>(L.x4.p), L.r.p, ctl);
+        return;
+    }
     const int t = L.n_nodes >= kStagedRows ? 1 : lanes_for(L.n_nodes);
     const SbView A = sbview(L);
     const float4* x = reinterpret_cast<const float4*>(L.x4.p);
@@ -2535,6 +2582,11 @@ void level_resid_or_post(Ctx& c, MgLevel& L, bool post, const Control* ctl) {
 }
 
 void level_post(Ctx& c, MgLevel& L, const Control* ctl) {
+    if (c.mg->box && c.mg->box_cycle && &L == c.mg->L[0].get()) {
+        box_post(c, *c.mg->box, L.binv.p, L.b.p, reinterpret_cast<const float4*>(L.x4.p),
+                 reinterpret_cast<float4*>(L.y4.p), ctl);
+        return;
+    }
     const int t = L.n_nodes >= kStagedRows ? 1 : lanes_for(L.n_nodes);
     const SbView A = sbview(L);
     const float4* x = reinterpret_cast<const float4*>(L.x4.p);
@@ -2642,6 +2694,11 @@ void mg_invalidate_values(Ctx& c) {
 void mg_prepare(Ctx& c, bool learned) {
     product_attrs();
     if (!c.mg) build_hierarchy(c);
+    {
+        std::vector<std::array<int, 5>> blocks;
+        for (const MgBlk& b : c.mg->L[0]->blk) blocks.push_back({b.nx, b.ny, b.nz, b.node0, b.el0});
+        c.mg->box = box_plan(c, blocks);
+    }
     if (c.mg->epoch != c.assembly_epoch) {
         setup_values(c, learned);
         c.mg->l0_learned = false;
@@ -2688,6 +2745,7 @@ double mg_time_kernel(Ctx& c, int kernel, int method, int n_launch, double* byte
     mg_prepare(c);
     mg_select_smoother(c, false);
     MgHierarchy& H = *c.mg;
+    const BoxCycle box_cycle(H);
     MgLevel& L0 = *H.L[0];
     const int n = c.A.n_rows, nd = c.n_dof;
     const int grid = (method == ASEND_METHOD_SPLIT && kernel == 0) ? std::min(grid_of(n), kPersistCtas) : grid_of(n);
@@ -2696,11 +2754,15 @@ double mg_time_kernel(Ctx& c, int kernel, int method, int n_launch, double* byte
     DArr<RhsScalars> sc;
     DArr<Control> ctl;
     DArr<double> part, p, ap;
-    sc.alloc(1);
+    const int NI = std::max(1, c.n_inst);
+    DArr<uint32_t> tk;
+    sc.alloc((size_t)NI * kMaxRhs);
     ctl.alloc(1);
+    tk.alloc((size_t)NI * 4);
     sc.zero(c.stream);
     ctl.zero(c.stream);
-    part.alloc((size_t)grid * kMaxRhs * 3);
+    tk.zero(c.stream);
+    part.alloc((size_t)std::max(grid, H.box ? box_ctas(*H.box) : 0) * kMaxRhs * 3);
     p.alloc((size_t)4 * n);
     ap.alloc(nd);
     MgPcg M;
@@ -2720,6 +2782,7 @@ double mg_time_kernel(Ctx& c, int kernel, int method, int n_launch, double* byte
     a.partials = part.p;
     a.sc = sc.p;
     a.ctl = ctl.p;
+    a.tickets = NI > 1 ? tk.p : nullptr;
     M.n_inst = 1;
     // the direction's values do not change the kernels' work: zeros
     ASEND_CUDA(cudaMemsetAsync(p.p, 0, sizeof(double) * 4 * n, c.stream));
@@ -2736,6 +2799,9 @@ double mg_time_kernel(Ctx& c, int kernel, int method, int n_launch, double* byte
     if (kernel == 0) *bytes = blocks * (9.0 * ps + 4.0) + (double)n * 4.0 * ps + (double)nd * ps;
     else if (kernel == 1) *bytes = blocks * 40.0 + (double)n * 16.0 + (double)nd * 8.0;
     else *bytes = blocks * 40.0 + (double)n * (16.0 + 36.0 + 16.0) + (double)nd * 4.0;
+    if (H.box && (kernel > 0 || (method == ASEND_METHOD_SPLIT && c.product_variant == ASEND_PRODUCT_DEFAULT)))
+        *bytes = kernel == 0 ? box_product_bytes(c)
+                             : 8.0 * c.n_el + (double)n * (kernel == 1 ? 16.0 : 68.0) + (double)nd * (kernel == 1 ? 8.0 : 4.0);
     for (int w = 0; w < 3; ++w) launch();
     ASEND_CUDA(cudaEventRecord(c.ev0, c.stream));
     for (int i = 0; i < n_launch; ++i) launch();
@@ -2879,13 +2945,15 @@ int pcg_solve_mg_once(Ctx& c, const asend_solve_opts& o, asend_solve_stats* st, 
     mg_prepare(c, o.precond == ASEND_PC_MG_LEARNED);
     mg_select_smoother(c, o.precond == ASEND_PC_MG_LEARNED);
     MgHierarchy& H = *c.mg;
+    const BoxCycle box_cycle(H);
     const int n = c.A.n_rows, nd = c.n_dof;
     const int max_it = o.max_iter > 0 ? o.max_iter : nd;
     const int G = o.graph_iters > 0 ? o.graph_iters : 8;
     if (!warm) ASEND_CUDA(cudaMemsetAsync(d_x, 0, (size_t)nrhs_all * nd * sizeof(double), c.stream));
     c.d_r.alloc(std::max(c.d_r.n, (size_t)nrhs_all * nd));
     const int grid = grid_of(n);
-    c.d_partials.alloc(std::max(c.d_partials.n, (size_t)grid * kMaxRhs * 3));
+    const size_t n_part = (size_t)std::max(grid, H.box ? box_ctas(*H.box) : 0);
+    c.d_partials.alloc(std::max(c.d_partials.n, n_part * kMaxRhs * 3));
     if (mixed) {
         c.d_p32.alloc(std::max(c.d_p32.n, (size_t)kMaxRhs * 4 * n));
         c.d_ap32.alloc(std::max(c.d_ap32.n, (size_t)kMaxRhs * nd));
@@ -3004,10 +3072,11 @@ int pcg_solve_mg_once(Ctx& c, const asend_solve_opts& o, asend_solve_stats* st, 
         // G iterations as one graph, kept with the hierarchy and reused while
         // the launch arguments are the same (they fully define the graph)
         // (with everything else that changes the captured sequence: the
-        // method, the chunk length, the product shape, the tail switch and
-        // the launch overlap)
-        std::vector<uint8_t> key(sizeof(MgPcg) + 4 * sizeof(int));
+        // method, the chunk length, the product shape, the tail switch, the
+        // launch overlap and the matrix-free plan)
+        std::vector<uint8_t> key(sizeof(MgPcg) + 4 * sizeof(int) + sizeof(void*));
         std::memcpy(key.data(), &M, sizeof(MgPcg));
+        std::memcpy(key.data() + sizeof(MgPcg) + 4 * sizeof(int), &H.box, sizeof(void*));
         const int extra[4] = {o.method, G, c.product_variant, (c.mg_tail ? 1 : 0) | (c.pdl ? 2 : 0)};
         std::memcpy(key.data() + sizeof(MgPcg), extra, sizeof(extra));
         cudaGraphExec_t exec = nullptr;

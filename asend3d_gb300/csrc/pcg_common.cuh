@@ -182,6 +182,15 @@ __device__ __forceinline__ F2 f2_of(double v) {  // FP64 -> pair (FP64 pipe: con
 }
 __device__ __forceinline__ double f2_dbl(F2 a) { return (double)a.h + (double)a.l; }
 
+// alpha = r.z / p.Ap, as FP64 and as a pair
+__device__ __forceinline__ void set_alpha(RhsScalars& s, double pAp) {
+    s.pAp = pAp;
+    s.alpha = s.rz / s.pAp;
+    const F2 a = f2_of(s.alpha);
+    s.alpha2[0] = a.h;
+    s.alpha2[1] = a.l;
+}
+
 // FP64-accurate row product from FP32 hi / lo values and a split direction:
 // the running sums S and their compensations Cc (y = S + Cc).
 template <int NR>

@@ -39,7 +39,7 @@ sys.path.insert(0, str(ROOT))
 
 # the headline metric, verbatim; each line's config.workload says what was run
 # kernel of each shape of the split outer product (asend_set_product_variant)
-PRODUCT_KERNEL = {1: "k_mg_spmv_dot_pair", 2: "k_mg_spmv_dot_staged<2,3>", 3: "k_mg_spmv_dot_staged<3,2>",
+PRODUCT_KERNEL = {0: "k_box_product", 1: "k_mg_spmv_dot_pair", 2: "k_mg_spmv_dot_staged<2,3>", 3: "k_mg_spmv_dot_staged<3,2>",
                   4: "k_mg_spmv_dot_staged<2,2>", 5: "k_mg_spmv_dot_staged<4,2>"}
 METRIC = "DOF-solves/sec at 1e-8 rel. residual, learned+batched vs plain PCG, 1 GB300; HBM GB/s"
 UNIT = "DOF-solves/s"
@@ -815,9 +815,9 @@ def run_ours(a):
     # timed as they run in the step; the slowest is reported
     peak, peak_kind = measured_peak()
     kern = {}
-    names = {0: f"{PRODUCT_KERNEL[shape]} (outer FP64-accurate product, FP32 hi+lo values, + p.Ap)",
-             1: "k_vc_resid (finest-level V-cycle residual, FP32 SBELL SpMV)",
-             2: "k_vc_post (finest-level post-smoothing, FP32 SBELL SpMV + block Jacobi)"}
+    names = {0: f"{PRODUCT_KERNEL[shape]} (outer FP64-accurate product in FP32 pairs, + p.Ap)",
+             1: "k_box_resid (finest-level V-cycle residual, FP32)",
+             2: "k_box_post (finest-level post-smoothing, FP32, block Jacobi)"}
     for k in (0, 1, 2):
         ms_k, by_k = g.time_mg_kernel(k, _lib.METHOD_SPLIT, 30)
         kern[k] = {"kernel": names[k], "ms_per_launch": ms_k, "algorithmic_bytes_per_launch": by_k,

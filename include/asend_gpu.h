@@ -136,7 +136,10 @@ int asend_mg_set_damping(asend_ctx* ctx, double factor);
  * kernel variant picked at run time (e.g. by an autotuner): the values and
  * column indices are fed through registers, or staged through shared memory
  * by bulk copies with G block-column groups per stage and S stages per warp.
- * Every shape gives bit-identical results.  No counterpart in the reference
+ * These shapes on the assembled values give bit-identical results.  The
+ * default takes the product from the element moduli and the class matrix
+ * (equal to rounding) on blocks of equal box elements with diagonal penalties,
+ * and STAGED_2x3 elsewhere.  No counterpart in the reference
  * (it has no GPU kernels): it tunes the kernel that replaces the products of
  * SparseMat::vector_multiply (list_ent_meth.rs:64-79) inside
  * conj_grad_sparse (matrix_functions.rs:285-362). */
