@@ -13,13 +13,14 @@ struct BoxPlan;
 BoxPlan* box_plan(Ctx& c, const std::vector<std::array<int, 5>>& blocks /* nx ny nz node0 el0 */);
 
 // y = A p (FP32 pairs, natural layout) of the CG and the p.Ap reduction, as
-// k_mg_spmv_dot_pair on the assembled values.
-void box_product(Ctx& c, const BoxPlan& P, pcg::PcgArgs a);
+// k_mg_spmv_dot_pair on the assembled values, for nr right-hand sides whose
+// vectors follow each other.
+void box_product(Ctx& c, const BoxPlan& P, pcg::PcgArgs a, int nr, int part_stride);
 // r = b - A x; y4 = x + B^-1 (b - A x); and a power-iteration step y4 = D^-1 A x
 // / nrm[k], nrm[k + 1] = |y4|, all FP32 on node-padded x.
-void box_resid(Ctx& c, const BoxPlan& P, const float* b, const float4* x, float* r, const pcg::Control* ctl);
+void box_resid(Ctx& c, const BoxPlan& P, const float* b, const float4* x, float* r, const pcg::Control* ctl, int nr);
 void box_post(Ctx& c, const BoxPlan& P, const float* binv, const float* b, const float4* x, float4* y4,
-              const pcg::Control* ctl);
+              const pcg::Control* ctl, int nr);
 void box_power(Ctx& c, const BoxPlan& P, const float* dinv, const float4* x, float4* y4, float* nrm, int k,
                double* part, uint32_t* ticket);
 int box_ctas(const BoxPlan& P);  // CTAs of one launch (entries of a partials array)

@@ -64,7 +64,7 @@ struct BoxItem {
 struct BoxPlan {
     int64_t pattern = -1, epoch = -1;
     bool ok = false;
-    int threads = 0, halo = 0, n_items = 0, pairs = 0;
+    int threads = 0, halo = 0, n_items = 0, pairs = 0, n_rows = 0;
     DArr<BoxItem> items;
     DArr<float2> B[2];                       // [n_cls][kBoxB] pattern blocks (hi, lo) of K^ in FP64, as pairs
     DArr<int32_t> cta_inst, inst_cta0, inst_ncta;  // batched stacks: CTAs by instance
@@ -89,6 +89,7 @@ struct BoxArgs {
     const float2* pen;
     const uint8_t* pen_node;
     int halo;
+    int n_rows;
 };
 
 struct P2 {  // value h + l, not renormalised: |l| stays near 2^-24 of the operands
@@ -374,11 +375,18 @@ __device__ __forceinline__ void box_march(const BoxArgs& A, const float4* __rest
     }
 }
 
-__global__ void __launch_bounds__(kBoxThreads, 1) k_box_product(BoxArgs X, PcgArgs A) {
+__global__ void __launch_bounds__(kBoxThreads, 1) k_box_product(BoxArgs X, PcgArgs A, int n_inst,
+                                                                int part_stride) {
     pdl_begin();
     extern __shared__ __align__(16) unsigned char smem[];
+    const size_t rhs = blockIdx.y;  // this right-hand side's vectors, scalars, partials and tickets
+    A.sc += rhs;
     RhsScalars* S = A.sc + cta_instance(A) * kMaxRhs;
-    if (cta_done<1>(A, S)) return;
+    if (A.ctl->active[rhs] == 0 || S[0].done) return;
+    A.p = reinterpret_cast<float4*>(A.p) + rhs * 2 * A.n_rows;
+    A.ap = reinterpret_cast<float2*>(A.ap) + rhs * A.n_dof;
+    A.partials += rhs * part_stride * (kMaxRhs * 3);
+    A.tickets += rhs * n_inst * 4;
     F2 acc{0.f, 0.f};
     float2* ap = reinterpret_cast<float2*>(A.ap);
     box_march<P2>(X, reinterpret_cast<const float4*>(A.p), smem, [&](int row, const P2 (&y)[3], const P2 (&p)[3]) {
@@ -394,11 +402,13 @@ __global__ void __launch_bounds__(kBoxThreads, 1) k_box_product(BoxArgs X, PcgAr
     if (last_block_reduce<1, 1>(A, d, 0, tot) && threadIdx.x == 0) set_alpha(S[0], tot[0][0]);
 }
 
-__global__ void __launch_bounds__(kBoxThreads, 1) k_box_resid(BoxArgs X, const float* __restrict__ b,
-                                                              const float4* __restrict__ x, float* __restrict__ r,
+__global__ void __launch_bounds__(kBoxThreads, 1) k_box_resid(BoxArgs X, const float* b, const float4* x, float* r,
                                                               const Control* ctl) {
     pdl_begin();
-    if (ctl && ctl->all_done) return;
+    if (ctl && ctl->active[blockIdx.y] == 0) return;
+    b += (size_t)blockIdx.y * 3 * X.n_rows;
+    x += (size_t)blockIdx.y * X.n_rows;
+    r += (size_t)blockIdx.y * 3 * X.n_rows;
     extern __shared__ __align__(16) unsigned char smem[];
     box_march<float>(X, x, smem, [&](int row, const float (&y)[3], const float (&)[3]) {
 #pragma unroll
@@ -406,11 +416,13 @@ __global__ void __launch_bounds__(kBoxThreads, 1) k_box_resid(BoxArgs X, const f
     });
 }
 
-__global__ void __launch_bounds__(kBoxThreads, 1) k_box_post(BoxArgs X, const float* __restrict__ binv,
-                                                             const float* __restrict__ b, const float4* __restrict__ x,
-                                                             float4* __restrict__ y4, const Control* ctl) {
+__global__ void __launch_bounds__(kBoxThreads, 1) k_box_post(BoxArgs X, const float* __restrict__ binv, const float* b,
+                                                             const float4* x, float4* y4, const Control* ctl) {
     pdl_begin();
-    if (ctl && ctl->all_done) return;
+    if (ctl && ctl->active[blockIdx.y] == 0) return;
+    b += (size_t)blockIdx.y * 3 * X.n_rows;
+    x += (size_t)blockIdx.y * X.n_rows;
+    y4 += (size_t)blockIdx.y * X.n_rows;
     extern __shared__ __align__(16) unsigned char smem[];
     box_march<float>(X, x, smem, [&](int row, const float (&y)[3], const float (&xv)[3]) {
         const float* B = binv + 9 * (size_t)row;
@@ -562,13 +574,13 @@ void make_items(BoxPlan& P, const std::vector<std::array<int, 5>>& blocks, const
     P.n_items = (int)items.size();
 }
 
-BoxArgs args_of(const BoxPlan& P) { return BoxArgs{P.items.p, P.B[P.pairs].p, P.E.p, P.pen.p, P.pen_node.p, P.halo}; }
+BoxArgs args_of(const BoxPlan& P) { return BoxArgs{P.items.p, P.B[P.pairs].p, P.E.p, P.pen.p, P.pen_node.p, P.halo, P.n_rows}; }
 
 template <typename T, typename... K, typename... Args>
-void launch(Ctx& c, const BoxPlan& P, void (*k)(K...), Args... args) {
+void launch(Ctx& c, const BoxPlan& P, int nr, void (*k)(K...), Args... args) {
     const size_t smem = box_smem<T>(P.threads, P.halo);
     ASEND_CUDA(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-    k<<<P.n_items, P.threads, smem, c.stream>>>(args...);
+    k<<<dim3(P.n_items, nr), P.threads, smem, c.stream>>>(args...);
 }
 
 }  // namespace
@@ -643,6 +655,7 @@ BoxPlan* box_plan(Ctx& c, const std::vector<std::array<int, 5>>& blocks) {
         P->pen.alloc(c.n_dof);
         P->pen.zero(c.stream);
         P->E.alloc(c.n_el);
+        P->n_rows = c.n_nodes;
         ASEND_CUDA(cudaStreamSynchronize(c.stream));  // the host vectors go out of scope
     }
     BoxPlan& P = *c.box;
@@ -666,24 +679,24 @@ BoxPlan* box_plan(Ctx& c, const std::vector<std::array<int, 5>>& blocks) {
 
 int box_ctas(const BoxPlan& P) { return P.n_items; }
 
-void box_product(Ctx& c, const BoxPlan& P, PcgArgs a) {
+void box_product(Ctx& c, const BoxPlan& P, PcgArgs a, int nr, int part_stride) {
     if (c.n_inst > 1) {  // this launch's own map of CTAs to instances
         a.cta_inst = P.cta_inst.p;
         a.inst_cta0 = P.inst_cta0.p;
         a.inst_ncta = P.inst_ncta.p;
     }
-    launch<P2>(c, P, k_box_product, args_of(P), a);
+    launch<P2>(c, P, nr, k_box_product, args_of(P), a, std::max(1, c.n_inst), part_stride);
 }
-void box_resid(Ctx& c, const BoxPlan& P, const float* b, const float4* x, float* r, const Control* ctl) {
-    launch<float>(c, P, k_box_resid, args_of(P), b, x, r, ctl);
+void box_resid(Ctx& c, const BoxPlan& P, const float* b, const float4* x, float* r, const Control* ctl, int nr) {
+    launch<float>(c, P, nr, k_box_resid, args_of(P), b, x, r, ctl);
 }
 void box_post(Ctx& c, const BoxPlan& P, const float* binv, const float* b, const float4* x, float4* y4,
-              const Control* ctl) {
-    launch<float>(c, P, k_box_post, args_of(P), binv, b, x, y4, ctl);
+              const Control* ctl, int nr) {
+    launch<float>(c, P, nr, k_box_post, args_of(P), binv, b, x, y4, ctl);
 }
 void box_power(Ctx& c, const BoxPlan& P, const float* dinv, const float4* x, float4* y4, float* nrm, int k,
                double* part, uint32_t* ticket) {
-    launch<float>(c, P, k_box_power, args_of(P), dinv, x, y4, nrm, k, part, ticket);
+    launch<float>(c, P, 1, k_box_power, args_of(P), dinv, x, y4, nrm, k, part, ticket);
 }
 
 // moduli, direction and A p, each once

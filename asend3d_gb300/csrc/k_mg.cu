@@ -74,6 +74,8 @@ struct MgLevel {
     std::vector<MgBlk> blk;
     DArr<BlkDev> d_blk;
     DArr<int32_t> pre_node, pre_el;  // per-block starts (+ total)
+    DArr<int32_t> row_blk;        // block of each row (stacks of blocks)
+    BlkDev one;                   // the descriptor of a lone block
     DArr<int32_t> d_xs, d_lo;     // packed per block and axis
     DArr<float> d_w;
     Sbell own;                    // pattern + FP32 values (levels >= 1)
@@ -113,7 +115,6 @@ struct MgHierarchy {
     DArr<unsigned int> pow_bound; // ||D^-1 A||_inf per level (float bits)
     DArr<float> pow_omega;        // damping in use per level
     bool safe_damping = false;    // omega from the guaranteed bound (after a failed solve)
-    int tail = 0;                 // first level of the fused coarse tail (0: none)
     BoxPlan* box = nullptr;       // matrix-free finest products of the current operator (or none)
     bool box_cycle = false;       // V-cycles take them, too (inside the CG; a V-cycle that a caller sees
                                   // keeps the assembled values)
@@ -144,13 +145,13 @@ constexpr int kPersistCtas = 152 * 4;
 // context allows it (the kernel then starts while its predecessor drains and
 // waits for it in pdl_begin(); every kernel launched here calls it first).
 template <typename... KArgs, typename... Args>
-void launch_k(const Ctx& c, void (*k)(KArgs...), int grid, int block, size_t smem, Args&&... args) {
+void launch_k(const Ctx& c, void (*k)(KArgs...), dim3 grid, int block, size_t smem, Args&&... args) {
     if (!c.pdl) {
         k<<<grid, block, smem, c.stream>>>(std::forward<Args>(args)...);
         return;
     }
     cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3((unsigned)grid);
+    cfg.gridDim = grid;
     cfg.blockDim = dim3((unsigned)block);
     cfg.dynamicSmemBytes = smem;
     cfg.stream = c.stream;
@@ -649,6 +650,15 @@ struct SbView {
     const float* v;
 };
 
+// The V-cycle runs for several right-hand sides at once: blockIdx.y picks one,
+// whose level vectors follow each other.  A right-hand side none of whose
+// instances iterates any more is left alone.
+__device__ __forceinline__ bool vc_idle(const Control* ctl) { return ctl && ctl->active[blockIdx.y] == 0; }
+template <typename T>
+__device__ __forceinline__ T* rhs_of(T* v, size_t n) {
+    return v + blockIdx.y * n;
+}
+
 // Row product with three block columns in flight per step: the column
 // indices, 27 values and three gathers of a step are independent loads, so
 // their latencies overlap instead of forming one 27-long dependent chain.
@@ -719,12 +729,14 @@ __device__ __forceinline__ void sum_lanes(float (&y)[3]) {
         for (int a = 0; a < 3; ++a) y[a] += __shfl_xor_sync(0xffffffffu, y[a], o);
 }
 
-__global__ void k_vc_smooth0(int n, const float* __restrict__ binv, const float* __restrict__ b, float4* __restrict__ x,
+__global__ void k_vc_smooth0(int n, const float* __restrict__ binv, const float* b, float4* x,
                              const Control* ctl) {
     pdl_begin();
-    if (ctl && ctl->all_done) return;
+    if (vc_idle(ctl)) return;
     const int row = blockIdx.x * blockDim.x + threadIdx.x;
     if (row >= n) return;
+    b = rhs_of(b, 3 * (size_t)n);
+    x = rhs_of(x, n);
     const float* B = binv + 9 * (size_t)row;
     const float b0 = b[3 * row], b1 = b[3 * row + 1], b2 = b[3 * row + 2];
     x[row] = make_float4(B[0] * b0 + B[1] * b1 + B[2] * b2, B[3] * b0 + B[4] * b1 + B[5] * b2,
@@ -734,7 +746,7 @@ __global__ void k_vc_smooth0(int n, const float* __restrict__ binv, const float*
 __global__ void __launch_bounds__(kT) k_vc_resid(SbView A, const float* __restrict__ b, const float4* __restrict__ x,
                                                  float* __restrict__ r, const Control* ctl) {
     pdl_begin();
-    if (ctl && ctl->all_done) return;
+    if (vc_idle(ctl)) return;
     const int row = blockIdx.x * blockDim.x + threadIdx.x;
     if (row >= A.n_rows) return;
     float y[3];
@@ -862,11 +874,13 @@ __device__ __forceinline__ bool f32_staged_slices(const SbView& A, const float4*
 }
 
 // r = b - A x over the level's rows (staged)
-__global__ void __launch_bounds__(kT) k_vc_resid_staged(SbView A, const float* __restrict__ b,
-                                                        const float4* __restrict__ x, float* __restrict__ r,
+__global__ void __launch_bounds__(kT) k_vc_resid_staged(SbView A, const float* b, const float4* x, float* r,
                                                         const Control* ctl) {
     pdl_begin();
-    if (ctl && ctl->all_done) return;
+    if (vc_idle(ctl)) return;
+    b = rhs_of(b, 3 * (size_t)A.n_rows);
+    x = rhs_of(x, A.n_rows);
+    r = rhs_of(r, 3 * (size_t)A.n_rows);
     extern __shared__ __align__(128) unsigned char vc_smem[];
     f32_staged_slices<kVcG, kVcS>(A, x, vc_smem, [&](int row, const float (&y)[3]) {
 #pragma unroll
@@ -875,11 +889,13 @@ __global__ void __launch_bounds__(kT) k_vc_resid_staged(SbView A, const float* _
 }
 
 // y4 = x + B^-1 (b - A x) over the level's rows (staged)
-__global__ void __launch_bounds__(kT) k_vc_post_staged(SbView A, const float* __restrict__ binv,
-                                                       const float* __restrict__ b, const float4* __restrict__ x,
-                                                       float4* __restrict__ y4, const Control* ctl) {
+__global__ void __launch_bounds__(kT) k_vc_post_staged(SbView A, const float* __restrict__ binv, const float* b,
+                                                       const float4* x, float4* y4, const Control* ctl) {
     pdl_begin();
-    if (ctl && ctl->all_done) return;
+    if (vc_idle(ctl)) return;
+    b = rhs_of(b, 3 * (size_t)A.n_rows);
+    x = rhs_of(x, A.n_rows);
+    y4 = rhs_of(y4, A.n_rows);
     extern __shared__ __align__(128) unsigned char vc_smem[];
     f32_staged_slices<kVcG, kVcS>(A, x, vc_smem, [&](int row, const float (&y)[3]) {
         const float d0 = b[3 * row] - y[0], d1 = b[3 * row + 1] - y[1], d2 = b[3 * row + 2] - y[2];
@@ -890,31 +906,15 @@ __global__ void __launch_bounds__(kT) k_vc_post_staged(SbView A, const float* __
     });
 }
 
-// Coarse-level variants with T lanes per row: a coarse level has too few
-// rows to fill the GPU with one thread each, and a row's 27 block columns
-// then form a long chain of dependent loads; T lanes split the chain.
-template <int T>
-__global__ void __launch_bounds__(kT) k_vc_resid_t(SbView A, const float* __restrict__ b, const float4* __restrict__ x,
-                                                   float* __restrict__ r, const Control* ctl) {
+// r = b - A x (POST = false) or y4 = x + B^-1 (b - A x) on any pattern, T lanes a
+// row (a small finest level).
+template <int T, bool POST>
+__global__ void __launch_bounds__(kT) k_vc_rows_any(SbView A, const float* __restrict__ binv, const float* b,
+                                                    const float4* x, float* r, float4* y4, const Control* ctl) {
     pdl_begin();
-    if (ctl && ctl->all_done) return;
-    const int gt = blockIdx.x * blockDim.x + threadIdx.x;
-    const int row = gt / T, t = gt % T;
-    const bool ok = row < A.n_rows;
-    float y[3] = {0.f, 0.f, 0.f};
-    if (ok) sb_row_part<T>(A, row, t, x, y);
-    sum_lanes<T>(y);
-    if (!ok || t != 0) return;
-#pragma unroll
-    for (int a = 0; a < 3; ++a) r[3 * row + a] = b[3 * row + a] - y[a];
-}
-
-template <int T>
-__global__ void __launch_bounds__(kT) k_vc_post_t(SbView A, const float* __restrict__ binv, const float* __restrict__ b,
-                                                  const float4* __restrict__ x, float4* __restrict__ y4,
-                                                  const Control* ctl) {
-    pdl_begin();
-    if (ctl && ctl->all_done) return;
+    if (vc_idle(ctl)) return;
+    b = rhs_of(b, 3 * (size_t)A.n_rows);
+    x = rhs_of(x, A.n_rows);
     const int gt = blockIdx.x * blockDim.x + threadIdx.x;
     const int row = gt / T, t = gt % T;
     const bool ok = row < A.n_rows;
@@ -923,17 +923,124 @@ __global__ void __launch_bounds__(kT) k_vc_post_t(SbView A, const float* __restr
     sum_lanes<T>(y);
     if (!ok || t != 0) return;
     const float d0 = b[3 * row] - y[0], d1 = b[3 * row + 1] - y[1], d2 = b[3 * row + 2] - y[2];
-    const float* B = binv + 9 * (size_t)row;
-    const float4 xv = x[row];
-    y4[row] = make_float4(xv.x + B[0] * d0 + B[1] * d1 + B[2] * d2, xv.y + B[3] * d0 + B[4] * d1 + B[5] * d2,
-                          xv.z + B[6] * d0 + B[7] * d1 + B[8] * d2, 0.f);
+    if constexpr (!POST) {
+        r = rhs_of(r, 3 * (size_t)A.n_rows);
+        r[3 * row] = d0, r[3 * row + 1] = d1, r[3 * row + 2] = d2;
+    } else {
+        const float* B = binv + 9 * (size_t)row;
+        const float4 xv = x[row];
+        rhs_of(y4, A.n_rows)[row] =
+            make_float4(xv.x + B[0] * d0 + B[1] * d1 + B[2] * d2, xv.y + B[3] * d0 + B[4] * d1 + B[5] * d2,
+                        xv.z + B[6] * d0 + B[7] * d1 + B[8] * d2, 0.f);
+    }
+}
+
+// Coarse-level variants with T lanes per row: a coarse level has too few
+// rows to fill the GPU with one thread each, and a row's 27 block columns
+// then form a long chain of dependent loads; T lanes split the chain.  These
+// kernels are a handful of L2 round trips long, so the level's structure is
+// computed instead of loaded (the columns of a row are its neighbours in the
+// block, in node order; coarse levels keep 27 column groups a slice): for one
+// block its description comes with the launch, in a stack with one load through
+// the row's block.  Values, gathers, right-hand side and smoother block are
+// then one round trip (caches cold, 6,171 rows of 100 x 20 x 20: a product 6.5 ->
+// 5.1 us, a restriction 5.0 -> 4.0 us, a prolongation 4.1 -> 3.7 us, the coarsest
+// solve 8.8 -> 3.2 us).  The sums and their order are sb_row_part's.
+struct GeoView {
+    int n_rows;
+    const BlkDev* blk;       // descriptors; row_blk == nullptr: one block, `one`
+    const int32_t* row_blk;  // block of each row
+    BlkDev one;
+    const float* v;
+};
+
+__device__ __forceinline__ BlkDev blk_of(const GeoView& G, int row) {
+    return G.row_blk ? G.blk[G.row_blk[row]] : G.one;
+}
+
+// The share of lane t of T in row `row`'s product; false: no such row.
+template <int T>
+__device__ __forceinline__ void geo_row_part(const GeoView& G, const BlkDev& d, int row, int t,
+                                             const float4* __restrict__ x, float (&y)[3]) {
+    const int l = row - d.node0;
+    const int sj = d.nz + 1, si = (d.ny + 1) * sj;
+    const int i = l / si, j = (l - i * si) / sj, k = l - i * si - j * sj;
+    const int i0 = max(i - 1, 0), j0 = max(j - 1, 0), k0 = max(k - 1, 0);
+    const int nj = min(j + 1, d.ny) - j0 + 1, nk = min(k + 1, d.nz) - k0 + 1;
+    const int len = (min(i + 1, d.nx) - i0 + 1) * nj * nk;
+    const int first = d.node0 + i0 * si + j0 * sj + k0;
+    const float* v = G.v + (size_t)(row >> 5) * (27 * 9 * 32) + (row & 31);
+    constexpr int U = (27 + T - 1) / T;
+    constexpr int STEP = U < 4 ? U : 4;  // columns in flight
+    y[0] = y[1] = y[2] = 0.f;
+#pragma unroll
+    for (int u0 = 0; u0 < U; u0 += STEP) {
+        float m[STEP][9];
+        float4 p[STEP];
+#pragma unroll
+        for (int u = 0; u < STEP; ++u) {
+            const int q = t + (u0 + u) * T;
+            if (q < len) {
+                const int qk = q / nk, c = first + (qk / nj) * si + (qk % nj) * sj + (q - qk * nk);
+                p[u] = x[c];
+#pragma unroll
+                for (int w = 0; w < 9; ++w) m[u][w] = v[((size_t)q * 9 + w) * 32];
+            }
+        }
+#pragma unroll
+        for (int u = 0; u < STEP; ++u) {
+            const int q = t + (u0 + u) * T;
+            if (q < len) {
+#pragma unroll
+                for (int a = 0; a < 3; ++a)
+                    y[a] = fmaf(m[u][a * 3], p[u].x, fmaf(m[u][a * 3 + 1], p[u].y, fmaf(m[u][a * 3 + 2], p[u].z, y[a])));
+            }
+        }
+    }
+}
+
+// r = b - A x (POST = false) or y4 = x + B^-1 (b - A x)
+template <int T, bool POST>
+__global__ void __launch_bounds__(kT) k_vc_rows(GeoView G, const float* __restrict__ binv, const float* b,
+                                                const float4* x, float* r, float4* y4, const Control* ctl) {
+    pdl_begin();
+    if (vc_idle(ctl)) return;
+    b = rhs_of(b, 3 * (size_t)G.n_rows);
+    x = rhs_of(x, G.n_rows);
+    const int gt = blockIdx.x * blockDim.x + threadIdx.x;
+    const int row = gt / T, t = gt % T;
+    const bool ok = row < G.n_rows, lead = ok && t == 0;
+    float y[3] = {0.f, 0.f, 0.f}, bv[3] = {0.f, 0.f, 0.f}, B[9];
+    float4 xv = make_float4(0.f, 0.f, 0.f, 0.f);
+    if (lead) {
+#pragma unroll
+        for (int a = 0; a < 3; ++a) bv[a] = b[3 * row + a];
+        if constexpr (POST) {
+            xv = x[row];
+#pragma unroll
+            for (int q = 0; q < 9; ++q) B[q] = binv[9 * (size_t)row + q];
+        }
+    }
+    if (ok) geo_row_part<T>(G, blk_of(G, row), row, t, x, y);
+    sum_lanes<T>(y);
+    if (!lead) return;
+    if constexpr (!POST) {
+        r = rhs_of(r, 3 * (size_t)G.n_rows);
+#pragma unroll
+        for (int a = 0; a < 3; ++a) r[3 * row + a] = bv[a] - y[a];
+    } else {
+        y4 = rhs_of(y4, G.n_rows);
+        const float d0 = bv[0] - y[0], d1 = bv[1] - y[1], d2 = bv[2] - y[2];
+        y4[row] = make_float4(xv.x + B[0] * d0 + B[1] * d1 + B[2] * d2, xv.y + B[3] * d0 + B[4] * d1 + B[5] * d2,
+                              xv.z + B[6] * d0 + B[7] * d1 + B[8] * d2, 0.f);
+    }
 }
 
 __global__ void __launch_bounds__(kT) k_vc_post(SbView A, const float* __restrict__ binv, const float* __restrict__ b,
                                                 const float4* __restrict__ x, float4* __restrict__ y4,
                                                 const Control* ctl) {
     pdl_begin();
-    if (ctl && ctl->all_done) return;
+    if (vc_idle(ctl)) return;
     const int row = blockIdx.x * blockDim.x + threadIdx.x;
     if (row >= A.n_rows) return;
     float y[3];
@@ -1133,285 +1240,142 @@ __global__ void k_scale_blocks(int n, float* __restrict__ binv, const float* __r
     if (i == 0) *omega_out = omega;
 }
 
+// Transfers.  Along an axis a coarse node m lies on the fine node 2 m (the last
+// one on the fine end), or on m where the axis is not coarsened, so positions
+// and weights (1/2 from the neighbours across a cell of two) are computed.
+__device__ __forceinline__ int fine_of(int m, int nc, int nf) { return nc == nf ? m : min(2 * m, nf); }
+
 // x_f[i] += sum_I w_iI y_c[I] over the fine level's nodes (a fine node outside
-// every block -- padding between instances -- is left alone); cv describes
-// the coarse level, pre_fnode the fine blocks' first nodes.
-__device__ __forceinline__ void prolong_row(const LevelView& cv, const BlkDev& d, int f, const float4* __restrict__ yc,
-                                            float4* __restrict__ xf) {
-    const int fl = f - d.fnode0;
-    if (fl >= (d.fnx + 1) * (d.fny + 1) * (d.fnz + 1)) return;
-    const int i = fl / ((d.fny + 1) * (d.fnz + 1)), j = (fl / (d.fnz + 1)) % (d.fny + 1), k = fl % (d.fnz + 1);
-    const int li = cv.lo[d.ol0 + i], lj = cv.lo[d.ol1 + j], lk = cv.lo[d.ol2 + k];
-    const float wi = cv.w[d.ol0 + i], wj = cv.w[d.ol1 + j], wk = cv.w[d.ol2 + k];
+// every block -- padding between instances -- is left alone); G describes the
+// coarse level's blocks (with their finer blocks), row_blk the fine rows'.
+__global__ void k_vc_prolong(GeoView G, int n_fine, const float4* yc, float4* xf, const Control* ctl) {
+    pdl_begin();
+    if (vc_idle(ctl)) return;
+    const int f = blockIdx.x * blockDim.x + threadIdx.x;
+    if (f >= n_fine) return;
+    yc = rhs_of(yc, G.n_rows);
+    xf = rhs_of(xf, n_fine);
     float4 acc = xf[f];
+    const BlkDev d = blk_of(G, f);
+    const int fl = f - d.fnode0, sj = d.fnz + 1, si = (d.fny + 1) * sj;
+    if (fl >= (d.fnx + 1) * si) return;
+    const int at[3] = {fl / si, (fl % si) / sj, fl % sj};
+    const int nf[3] = {d.fnx, d.fny, d.fnz}, nc[3] = {d.nx, d.ny, d.nz};
+    int lo[3];
+    bool mid[3];  // between two coarse nodes
 #pragma unroll
-    for (int di = 0; di < 2; ++di) {
-        const float a = di ? wi : 1.f - wi;
-        if (a == 0.f) continue;
+    for (int ax = 0; ax < 3; ++ax) {
+        const bool co = nc[ax] != nf[ax];
+        lo[ax] = !co ? at[ax] : (at[ax] == nf[ax] ? nc[ax] : at[ax] >> 1);
+        mid[ax] = co && (at[ax] & 1) && at[ax] < nf[ax];
+    }
+    const int base = d.node0 + nid(lo[0], lo[1], lo[2], d.ny, d.nz);
+    float4 y[8];
 #pragma unroll
-        for (int dj = 0; dj < 2; ++dj) {
-            const float b = dj ? wj : 1.f - wj;
-            if (b == 0.f) continue;
+    for (int q = 0; q < 8; ++q) {
+        const int di = q >> 2, dj = (q >> 1) & 1, dk = q & 1;
+        if ((!di || mid[0]) && (!dj || mid[1]) && (!dk || mid[2]))
+            y[q] = yc[base + (di * (d.ny + 1) + dj) * (d.nz + 1) + dk];
+    }
 #pragma unroll
-            for (int dk = 0; dk < 2; ++dk) {
-                const float c = dk ? wk : 1.f - wk;
-                if (c == 0.f) continue;
-                const float4 y = yc[d.node0 + nid(li + di, lj + dj, lk + dk, d.ny, d.nz)];
-                const float ww = a * b * c;
-                acc.x += ww * y.x;
-                acc.y += ww * y.y;
-                acc.z += ww * y.z;
-            }
+    for (int q = 0; q < 8; ++q) {
+        const int di = q >> 2, dj = (q >> 1) & 1, dk = q & 1;
+        if ((!di || mid[0]) && (!dj || mid[1]) && (!dk || mid[2])) {
+            const float ww = (mid[0] ? 0.5f : 1.f) * (mid[1] ? 0.5f : 1.f) * (mid[2] ? 0.5f : 1.f);
+            acc.x += ww * y[q].x;
+            acc.y += ww * y[q].y;
+            acc.z += ww * y[q].z;
         }
     }
     xf[f] = acc;
 }
 
-__global__ void k_vc_prolong(LevelView cv, const int32_t* __restrict__ pre_fnode, int n_fine,
-                             const float4* __restrict__ yc, float4* __restrict__ xf, const Control* ctl) {
+// Coarsest solve y = A_b^-1 b per block: one warp per row (eight loads a lane
+// in flight: a 256-wide row in one pass), kDenseRows rows a CTA.  y is
+// node-padded.
+constexpr int kDenseRows = 8;
+__global__ void __launch_bounds__(32 * kDenseRows) k_vc_dense(GeoView G, const float* __restrict__ ainv, const float* b,
+                                                              float* y4, const Control* ctl) {
     pdl_begin();
-    if (ctl && ctl->all_done) return;
-    const int f = blockIdx.x * blockDim.x + threadIdx.x;
-    if (f >= n_fine) return;
-    prolong_row(cv, cv.blk[find_blk(pre_fnode, cv.n_blk, f)], f, yc, xf);
-}
-
-// Coarsest solve y = A_b^-1 b per block (CTA = block): one warp per row,
-// lanes stride the row (coalesced), shuffle reduction.  y is node-padded.
-// sb: shared staging of the block's b (at least n floats); the CTA's threads
-// all call this (it synchronises them).
-__device__ __forceinline__ void dense_block(const BlkDev& d, const float* __restrict__ ainv, const float* __restrict__ b,
-                                            float* __restrict__ y4, float* sb) {
+    if (vc_idle(ctl)) return;
+    const int row = blockIdx.z * kDenseRows + (threadIdx.x >> 5), lane = threadIdx.x & 31;
+    const BlkDev d = G.row_blk ? G.blk[blockIdx.x] : G.one;
     const int n = 3 * (d.nx + 1) * (d.ny + 1) * (d.nz + 1);
-    const float* bb = b + 3 * (size_t)d.node0;
-    for (int i = threadIdx.x; i < n; i += blockDim.x) sb[i] = bb[i];
-    __syncthreads();
-    const float* Ab = ainv + d.dense0;
-    float* yb = y4 + 4 * (size_t)d.node0;
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, nw = blockDim.x >> 5;
-    // eight loads per lane issued together (a 256-wide row in one pass): the
-    // row's loads overlap instead of waiting on each other
-    for (int row = warp; row < n; row += nw) {
-        const float* ar = Ab + (size_t)row * n;
-        float acc = 0.f;
-        for (int j0 = 0; j0 < n; j0 += 256) {
-            float a[8];
+    if (row >= n) return;
+    const float* bb = rhs_of(b, 3 * (size_t)G.n_rows) + 3 * (size_t)d.node0;
+    const float* ar = ainv + d.dense0 + (size_t)row * n;
+    float a[8], bv[8], acc = 0.f;
 #pragma unroll
-            for (int t = 0; t < 8; ++t) {
-                const int j = j0 + lane + 32 * t;
-                a[t] = j < n ? ar[j] : 0.f;
-            }
-#pragma unroll
-            for (int t = 0; t < 8; ++t) {
-                const int j = j0 + lane + 32 * t;
-                if (j < n) acc = fmaf(a[t], sb[j], acc);
-            }
-        }
-#pragma unroll
-        for (int o = 16; o > 0; o >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, o);
-        if (lane == 0) yb[4 * (row / 3) + row % 3] = acc;
+    for (int t = 0; t < 8; ++t) {
+        const int j = lane + 32 * t;
+        a[t] = j < n ? ar[j] : 0.f;
+        bv[t] = j < n ? bb[j] : 0.f;
     }
+#pragma unroll
+    for (int t = 0; t < 8; ++t)
+        if (lane + 32 * t < n) acc = fmaf(a[t], bv[t], acc);
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, o);
+    if (lane == 0) rhs_of(y4, 4 * (size_t)G.n_rows)[4 * ((size_t)d.node0 + row / 3) + row % 3] = acc;
 }
 
-__global__ void __launch_bounds__(1024) k_vc_dense(LevelView cv, const float* __restrict__ ainv,
-                                                   const float* __restrict__ b, float* __restrict__ y4,
-                                                   const Control* ctl) {
+// Trilinear restriction R = P^T over every block at once, four lanes per coarse
+// node (a component each, the fourth idle): b_c[m] = sum over the fine nodes f
+// of w_x w_y w_z r_f, where along each axis the fine nodes next to 2 m
+// contribute with 1/2 when they lie across a cell of two.  Fixed slots let the
+// 27 loads of a lane issue together.  The coarse level's first smoothing sweep
+// x4 = B^-1 b is fused in (binv non-null).
+__global__ void __launch_bounds__(kT) k_vc_restrict(GeoView G, int n_fine, const float* in, float* out,
+                                                    const float* __restrict__ binv, float4* x4, const Control* ctl) {
     pdl_begin();
-    if (ctl && ctl->all_done) return;
-    __shared__ float sb[1024];
-    dense_block(cv.blk[blockIdx.x], ainv, b, y4, sb);
-}
-
-// Trilinear restriction R = P^T over every block at once, one coarse node per
-// thread: b_c[m] = sum over the fine nodes f of w_x w_y w_z r_f, where along
-// each axis the fine nodes between xs[m-1] and xs[m+1] contribute with the
-// prolongation weight of m (1 - w on the node's lower coarse neighbour, w on
-// the upper one).  The coarse level's first smoothing sweep x4 = B^-1 b is
-// fused in (binv non-null).
-// The taps of coarse node m on one axis: fine nodes xs[m] - 1, xs[m] and
-// xs[m] + 1, each present when it lies strictly between xs[m - 1] and
-// xs[m + 1] (coarse spacing is one or two fine cells, so no other fine node
-// has a non-zero weight); weights w[xs[m] - 1], 1 and 1 - w[xs[m] + 1], the
-// prolongation weights of m.  Fixed slots keep the taps in registers and let
-// the 27 loads of a coarse node issue together.
-struct Taps {
-    int f[3];
-    float w[3];
-    bool on[3];
-};
-__device__ __forceinline__ Taps axis_taps(const int32_t* __restrict__ xs, const float* __restrict__ w, int m,
-                                          int n_c) {
-    Taps t;
-    const int x = xs[m];
-    t.on[0] = m > 0 && x - 1 > xs[m - 1];
-    t.on[1] = true;
-    t.on[2] = m < n_c && x + 1 < xs[m + 1];
-    t.f[0] = t.on[0] ? x - 1 : x;  // an absent tap points at x: every address formed stays in range
-    t.f[1] = x;
-    t.f[2] = t.on[2] ? x + 1 : x;
-    t.w[0] = t.on[0] ? w[x - 1] : 0.f;
-    t.w[1] = 1.f;
-    t.w[2] = t.on[2] ? 1.f - w[x + 1] : 0.f;
-    return t;
-}
-
-__device__ __forceinline__ void restrict_row(const LevelView& cv, const BlkDev& d, int o, const float* __restrict__ in,
-                                             float* __restrict__ out, const float* __restrict__ binv,
-                                             float4* __restrict__ x4) {
-    const int ol = o - d.node0;
-    const int i0 = ol / ((d.ny + 1) * (d.nz + 1)), i1 = (ol / (d.nz + 1)) % (d.ny + 1), i2 = ol % (d.nz + 1);
-    const Taps tx = axis_taps(cv.xs + d.ox0, cv.w + d.ol0, i0, d.nx);
-    const Taps ty = axis_taps(cv.xs + d.ox1, cv.w + d.ol1, i1, d.ny);
-    const Taps tz = axis_taps(cv.xs + d.ox2, cv.w + d.ol2, i2, d.nz);
-    float v[3][3][3][3];
-#pragma unroll
-    for (int a = 0; a < 3; ++a)
-#pragma unroll
-        for (int b = 0; b < 3; ++b)
-#pragma unroll
-            for (int c = 0; c < 3; ++c) {
-                const bool on = tx.on[a] && ty.on[b] && tz.on[c];
-                const size_t src = 3 * (size_t)(d.fnode0 + (tx.f[a] * (d.fny + 1) + ty.f[b]) * (d.fnz + 1) + tz.f[c]);
-#pragma unroll
-                for (int q = 0; q < 3; ++q) v[a][b][c][q] = on ? in[src + q] : 0.f;
-            }
-    float s0 = 0.f, s1 = 0.f, s2 = 0.f;
-#pragma unroll
-    for (int a = 0; a < 3; ++a)
-#pragma unroll
-        for (int b = 0; b < 3; ++b) {
-            const float wab = tx.w[a] * ty.w[b];
-#pragma unroll
-            for (int c = 0; c < 3; ++c) {
-                if (!(tx.on[a] && ty.on[b] && tz.on[c])) continue;
-                const float ww = wab * tz.w[c];
-                s0 = fmaf(ww, v[a][b][c][0], s0);
-                s1 = fmaf(ww, v[a][b][c][1], s1);
-                s2 = fmaf(ww, v[a][b][c][2], s2);
-            }
-        }
-    out[3 * (size_t)o] = s0;
-    out[3 * (size_t)o + 1] = s1;
-    out[3 * (size_t)o + 2] = s2;
+    if (vc_idle(ctl)) return;
+    const int gt = blockIdx.x * blockDim.x + threadIdx.x;
+    const bool ok = (gt >> 2) < G.n_rows;
+    const int o = ok ? gt >> 2 : 0, comp = min(gt & 3, 2);
+    in = rhs_of(in, 3 * (size_t)n_fine) + comp;
+    float B[3] = {0.f, 0.f, 0.f};
     if (binv) {
-        const float* B = binv + 9 * (size_t)o;
-        x4[o] = make_float4(B[0] * s0 + B[1] * s1 + B[2] * s2, B[3] * s0 + B[4] * s1 + B[5] * s2,
-                            B[6] * s0 + B[7] * s1 + B[8] * s2, 0.f);
-    }
-}
-
-__global__ void __launch_bounds__(kT) k_vc_restrict(LevelView cv, const int32_t* __restrict__ pre_node, int n_out,
-                                                    const float* __restrict__ in, float* __restrict__ out,
-                                                    const float* __restrict__ binv, float4* __restrict__ x4,
-                                                    const Control* ctl) {
-    pdl_begin();
-    if (ctl && ctl->all_done) return;
-    const int o = blockIdx.x * blockDim.x + threadIdx.x;
-    if (o >= n_out) return;
-    restrict_row(cv, cv.blk[find_blk(pre_node, cv.n_blk, o)], o, in, out, binv, x4);
-}
-
-// ---------------------------------------------------------------------------
-// Fused coarse tail of the V-cycle.  Below a size threshold every level of an
-// instance fits one CTA, and an instance's rows couple only to its own rows
-// on every level (the stacked operator is block diagonal), so one CTA per
-// block runs the tail's residuals, restrictions, the coarsest dense solve,
-// prolongations and post-smoothing in sequence with CTA barriers between the
-// steps, in place of a dozen small grid-wide launches whose latency, not
-// their few hundred kilobytes, set their time.  Per row the arithmetic and
-// its order are those of the separate kernels (same lanes per row).
-// ---------------------------------------------------------------------------
-constexpr int kMaxTail = 8;       // levels a fused tail may hold
-constexpr int kTailNodes = 512;   // largest block (nodes) of a level in the tail
-constexpr int kTailThreads = 1024;
-constexpr int kTailMinBlocks = 16;  // instances a stack needs before its tail is fused
-
-struct TailLevel {
-    SbView A;
-    LevelView V;   // blocks of this level (with their finer blocks' maps)
-    const float* binv;
-    float* b;
-    float* r;
-    float4* x4;
-    float4* y4;
-    int lanes;     // lanes per row of this level's products (as the separate kernels)
-};
-struct TailArgs {
-    int n_lev;     // levels lt .. nl - 1; the last one is solved by its dense inverse
-    TailLevel L[kMaxTail];
-    const float* ainv;
-};
-
-// r = b - A x (post == false) or y = x + B^-1 (b - A x) (post == true) over
-// the rows [row0, row0 + nn) of one block, T lanes per row.
-template <int T>
-__device__ __forceinline__ void tail_rows(const TailLevel& L, int row0, int nn, bool post) {
-    const int tot = nn * T;
-    const float4* x = L.x4;
-    for (int base = 0; base < tot; base += blockDim.x) {  // same trip count in every thread
-        const int gt = base + threadIdx.x;
-        const int row = row0 + gt / T, t = gt % T;
-        const bool ok = gt < tot;
-        float y[3] = {0.f, 0.f, 0.f};
-        if (ok) sb_row_part<T>(L.A, row, t, x, y);
-        sum_lanes<T>(y);
-        if (!ok || t != 0) continue;
-        if (!post) {
 #pragma unroll
-            for (int a = 0; a < 3; ++a) L.r[3 * row + a] = L.b[3 * row + a] - y[a];
-        } else {
-            const float d0 = L.b[3 * row] - y[0], d1 = L.b[3 * row + 1] - y[1], d2 = L.b[3 * row + 2] - y[2];
-            const float* B = L.binv + 9 * (size_t)row;
-            const float4 xv = x[row];
-            L.y4[row] = make_float4(xv.x + B[0] * d0 + B[1] * d1 + B[2] * d2, xv.y + B[3] * d0 + B[4] * d1 + B[5] * d2,
-                                    xv.z + B[6] * d0 + B[7] * d1 + B[8] * d2, 0.f);
-        }
+        for (int q = 0; q < 3; ++q) B[q] = binv[9 * (size_t)o + 3 * comp + q];
     }
-}
-__device__ __forceinline__ void tail_level_rows(const TailLevel& L, int row0, int nn, bool post) {
-    switch (L.lanes) {
-        case 1: tail_rows<1>(L, row0, nn, post); break;
-        case 2: tail_rows<2>(L, row0, nn, post); break;
-        case 4: tail_rows<4>(L, row0, nn, post); break;
-        case 8: tail_rows<8>(L, row0, nn, post); break;
-        default: tail_rows<16>(L, row0, nn, post); break;
+    const BlkDev d = blk_of(G, o);
+    const int ol = o - d.node0, sj = d.nz + 1, si = (d.ny + 1) * sj;
+    const int m[3] = {ol / si, (ol % si) / sj, ol % sj};
+    const int nf[3] = {d.fnx, d.fny, d.fnz}, nc[3] = {d.nx, d.ny, d.nz};
+    int x[3];
+    bool on[3][3];  // axis, tap x - 1, x, x + 1
+#pragma unroll
+    for (int ax = 0; ax < 3; ++ax) {
+        x[ax] = fine_of(m[ax], nc[ax], nf[ax]);
+        on[ax][0] = m[ax] > 0 && x[ax] - fine_of(m[ax] - 1, nc[ax], nf[ax]) == 2;
+        on[ax][1] = true;
+        on[ax][2] = m[ax] < nc[ax] && fine_of(m[ax] + 1, nc[ax], nf[ax]) - x[ax] == 2;
     }
-}
-
-__global__ void __launch_bounds__(kTailThreads) k_vc_tail(TailArgs ta, const Control* ctl) {
-    pdl_begin();
-    if (ctl && ctl->all_done) return;
-    __shared__ float sb[1024];
-    const int b = blockIdx.x;
-    const int nl = ta.n_lev;
-    auto nodes = [](const BlkDev& d) { return (d.nx + 1) * (d.ny + 1) * (d.nz + 1); };
-    for (int l = 0; l + 1 < nl; ++l) {
-        const BlkDev& d = ta.L[l].V.blk[b];
-        tail_level_rows(ta.L[l], d.node0, nodes(d), false);
-        __syncthreads();
-        const TailLevel& C = ta.L[l + 1];
-        const BlkDev& dc = C.V.blk[b];
-        const bool last = (l + 2 == nl);  // the coarsest level takes no smoothing sweep
-        for (int q = threadIdx.x; q < nodes(dc); q += blockDim.x)
-            restrict_row(C.V, dc, dc.node0 + q, ta.L[l].r, C.b, last ? nullptr : C.binv, C.x4);
-        __syncthreads();
+    float v[27];
+#pragma unroll
+    for (int q = 0; q < 27; ++q) {
+        const int a = q / 9, b = q / 3 % 3, c = q % 3;
+        const size_t src = d.fnode0 + ((size_t)(x[0] + a - 1) * (d.fny + 1) + (x[1] + b - 1)) * (d.fnz + 1) + (x[2] + c - 1);
+        v[q] = on[0][a] && on[1][b] && on[2][c] ? in[3 * src] : 0.f;
     }
-    dense_block(ta.L[nl - 1].V.blk[b], ta.ainv, ta.L[nl - 1].b, reinterpret_cast<float*>(ta.L[nl - 1].y4), sb);
-    __syncthreads();
-    for (int l = nl - 2; l >= 0; --l) {
-        const TailLevel& C = ta.L[l + 1];
-        const BlkDev& dc = C.V.blk[b];
-        const int nf = (dc.fnx + 1) * (dc.fny + 1) * (dc.fnz + 1);
-        for (int q = threadIdx.x; q < nf; q += blockDim.x) prolong_row(C.V, dc, dc.fnode0 + q, C.y4, ta.L[l].x4);
-        __syncthreads();
-        const BlkDev& d = ta.L[l].V.blk[b];
-        tail_level_rows(ta.L[l], d.node0, nodes(d), true);
-        __syncthreads();
+    float s = 0.f;
+#pragma unroll
+    for (int q = 0; q < 27; ++q) {
+        const int a = q / 9, b = q / 3 % 3, c = q % 3;
+        const float ww = (a == 1 ? 1.f : 0.5f) * (b == 1 ? 1.f : 0.5f) * (c == 1 ? 1.f : 0.5f);
+        if (on[0][a] && on[1][b] && on[2][c]) s = fmaf(ww, v[q], s);
     }
+    const int lane0 = (threadIdx.x & 31) & ~3;
+    const float s0 = __shfl_sync(0xffffffffu, s, lane0), s1 = __shfl_sync(0xffffffffu, s, lane0 + 1),
+                s2 = __shfl_sync(0xffffffffu, s, lane0 + 2);
+    if (!ok || (gt & 3) == 3) return;
+    rhs_of(out, 3 * (size_t)G.n_rows)[3 * (size_t)o + comp] = s;
+    if (binv)
+        reinterpret_cast<float*>(rhs_of(x4, G.n_rows) + o)[comp] = B[0] * s0 + B[1] * s1 + B[2] * s2;
 }
 
 // ---------------------------------------------------------------------------
-// multigrid-preconditioned flexible CG kernels (one right-hand side; every
+// multigrid-preconditioned flexible CG kernels (up to 4 right-hand sides; every
 // instance of a batched stack at once, with its own scalars and tickets)
 // ---------------------------------------------------------------------------
 struct MgPcg {
@@ -1425,28 +1389,52 @@ struct MgPcg {
     const float* binv0;   // level-0 smoother blocks: the first sweep
     float4* x40;          // x4 = B^-1 r is fused into the kernels writing b0
     int n_inst;           // instances (1: a single model)
+    int part_stride;      // CTAs of the partials array per right-hand side
 };
 
-// Instances still iterating are counted in ctl->pad[0]; the one whose
-// recurrence converges last sets all_done, which ends every kernel of the
-// remaining captured iterations at once.
-__device__ __forceinline__ void retire_instance(const PcgArgs& A) {
-    if (atomicSub(&A.ctl->pad[0], 1) == 1) A.ctl->all_done = 1;
+// The kernels' second grid dimension is the right-hand side: its slice of every
+// vector, scalar set, ticket and partials array (F32: the mixed method's FP32
+// direction and A p).
+template <bool F32>
+__device__ __forceinline__ MgPcg rhs_view(MgPcg M) {
+    const size_t k = blockIdx.y, n = M.a.n_rows, nd = M.a.n_dof;
+    PcgArgs& A = M.a;
+    A.f += k * nd;
+    A.x += k * nd;
+    A.r += k * nd;
+    A.p = reinterpret_cast<char*>(A.p) + k * n * (F32 ? 16 : 32);
+    A.ap = reinterpret_cast<char*>(A.ap) + k * nd * (F32 ? 4 : 8);
+    A.partials += k * M.part_stride * (kMaxRhs * 3);
+    A.tickets += k * M.n_inst * 4;
+    A.sc += k;
+    M.xp += 2 * k * n;
+    if (M.xt) M.xt += 3 * k * n;
+    M.b0 += k * nd;
+    M.z += k * n;
+    M.x40 += k * n;
+    return M;
 }
 
-// First kernel of a captured chunk of iterations: count the instances not
-// done (all_done when none is left).
+// Nothing left to do for this CTA's instance and right-hand side.
+__device__ __forceinline__ bool mg_done(const PcgArgs& A, const RhsScalars* S) {
+    return A.ctl->active[blockIdx.y] == 0 || S[0].done;
+}
+
+// The instances still iterating are counted per right-hand side; with the last
+// one whose recurrence converges every remaining captured kernel of that
+// right-hand side ends at once.
+__device__ __forceinline__ void retire_instance(const PcgArgs& A) { atomicSub(&A.ctl->active[blockIdx.y], 1); }
+
+// First kernel of a captured chunk of iterations: count the instances not done
+// (grid: right-hand sides).
 __global__ void k_mg_count_active(MgPcg M) {
     pdl_begin();
     const PcgArgs& A = M.a;
     int n = 0;
-    for (int i = threadIdx.x; i < M.n_inst; i += blockDim.x) n += A.sc[(size_t)i * kMaxRhs].done ? 0 : 1;
+    for (int i = threadIdx.x; i < M.n_inst; i += blockDim.x) n += A.sc[(size_t)i * kMaxRhs + blockIdx.x].done ? 0 : 1;
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) n += __shfl_xor_sync(0xffffffffu, n, o);
-    if (threadIdx.x == 0) {
-        A.ctl->pad[0] = n;
-        A.ctl->all_done = (n == 0) ? 1 : 0;
-    }
+    if (threadIdx.x == 0) A.ctl->active[blockIdx.x] = n;
 }
 
 __device__ __forceinline__ void fused_smooth0(const MgPcg& M, int row, const double (&r)[3]) {
@@ -1459,9 +1447,10 @@ __device__ __forceinline__ void fused_smooth0(const MgPcg& M, int row, const dou
 template <typename TV, typename TP>
 __global__ void __launch_bounds__(kThreads) k_mg_spmv_dot(MgPcg M) {
     using PV = typename ApOf<TP>::T;
+    M = rhs_view<sizeof(TV) == 4 && std::is_same<TP, float>::value>(M);
     const PcgArgs& A = M.a;
     RhsScalars* S = A.sc + cta_instance(A) * kMaxRhs;
-    if (cta_done<1>(A, S)) return;
+    if (mg_done(A, S)) return;
     const int row = blockIdx.x * blockDim.x + threadIdx.x;
     double d[1][1] = {{0.0}};
     if (row < A.n_rows) {
@@ -1483,6 +1472,54 @@ __global__ void __launch_bounds__(kThreads) k_mg_spmv_dot(MgPcg M) {
         RhsScalars& s = S[0];
         s.pAp = tot[0][0];
         s.alpha = s.rz / s.pAp;
+    }
+}
+
+// The FP64 product with T lanes a row, for single models whose rows alone leave
+// SMs idle: one thread a row walked 27 columns one step after the other (7,930
+// rows: 52.6 us), T lanes share them.
+template <int T>
+__global__ void __launch_bounds__(kThreads) k_mg_spmv_dot_lanes(MgPcg M) {
+    M = rhs_view<false>(M);
+    const PcgArgs& A = M.a;
+    RhsScalars* S = A.sc;
+    if (mg_done(A, S)) return;
+    const int gt = blockIdx.x * blockDim.x + threadIdx.x;
+    const int row = gt / T, t = gt % T;
+    const bool ok = row < A.n_rows;
+    double y[3] = {0.0, 0.0, 0.0}, d[1][1] = {{0.0}};
+    if (ok) {
+        const int lane = row & 31, len = A.row_len[row];
+        const int64_t g0 = A.slice_off[row >> 5];
+#pragma unroll 2
+        for (int j = t; j < len; j += T) {
+            const int64_t g = g0 + j;
+            double m[9], p[3];
+            PadVec<double>::load(A.p, (size_t)A.col[g * 32 + lane], p);
+#pragma unroll
+            for (int q = 0; q < 9; ++q) m[q] = A.v64[(g * 9 + q) * 32 + lane];
+#pragma unroll
+            for (int a = 0; a < 3; ++a) y[a] = fma(m[3 * a], p[0], fma(m[3 * a + 1], p[1], fma(m[3 * a + 2], p[2], y[a])));
+        }
+    }
+#pragma unroll
+    for (int o = T / 2; o >= 1; o >>= 1)
+#pragma unroll
+        for (int a = 0; a < 3; ++a) y[a] += __shfl_xor_sync(0xffffffffu, y[a], o);
+    if (ok && t == 0) {
+        double pv[3];
+        PadVec<double>::load(A.p, row, pv);
+        double* ap = reinterpret_cast<double*>(A.ap) + 3 * (size_t)row;
+#pragma unroll
+        for (int q = 0; q < 3; ++q) {
+            ap[q] = y[q];
+            d[0][0] += pv[q] * y[q];
+        }
+    }
+    double tot[1][1];
+    if (last_block_reduce<1, 1>(A, d, 0, tot) && threadIdx.x == 0) {
+        S[0].pAp = tot[0][0];
+        S[0].alpha = S[0].rz / S[0].pAp;
     }
 }
 
@@ -1528,9 +1565,10 @@ __device__ __forceinline__ F2 pair_ap_dot(const PcgArgs& A, int row, const F2 (&
 // The register-fed split product with the pair epilogue.
 __global__ void __launch_bounds__(kThreads) k_mg_spmv_dot_pair(MgPcg M) {
     pdl_begin();
+    M = rhs_view<false>(M);
     const PcgArgs& A = M.a;
     RhsScalars* Sc = A.sc + cta_instance(A) * kMaxRhs;
-    if (cta_done<1>(A, Sc)) return;
+    if (mg_done(A, Sc)) return;
     F2 acc{0.f, 0.f};
     for (int row = blockIdx.x * blockDim.x + threadIdx.x; row < A.n_rows; row += gridDim.x * blockDim.x) {
         float Sm[1][3], Cc[1][3];
@@ -1548,15 +1586,11 @@ __global__ void __launch_bounds__(kThreads) k_mg_spmv_dot_pair(MgPcg M) {
 // FP32 pair.  Folding e into x64 there (and at the end) keeps the stored
 // solution in FP64, so the pairs' 48-bit rounding of e stays far below the
 // solve's tolerance (x itself as a pair left a noise floor near 1e-9).
-__global__ void k_zero_pairs(int n, float4* __restrict__ e) {
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i < 2 * n) e[i] = make_float4(0.f, 0.f, 0.f, 0.f);
-}
-
 // x64 += e, e = 0 for the instances whose true residual is formed next (all
 // rows when all is set)
 __global__ void __launch_bounds__(kThreads) k_fold_pairs(MgPcg M, int all) {
     pdl_begin();
+    M = rhs_view<false>(M);
     const PcgArgs& A = M.a;
     const RhsScalars* S = A.sc + cta_instance(A) * kMaxRhs;
     if (!all && !S[0].replace) return;
@@ -1609,11 +1643,14 @@ __device__ __forceinline__ void res_term(float h, float l, float xh, float xl, f
     D = __fmaf_rn(h, xr, __fmaf_rn(l, xl, D));
 }
 
+constexpr int kZeroStart = 2;  // init: the start is x = 0, so r = f
+
 // True residual r = f - A x from the operator's hi / lo values (split-only
 // assembly: no FP64 values) and the three FP32 parts of x written by the
 // fold, each term by res_term.
 __global__ void __launch_bounds__(kThreads) k_mg_residual_split(MgPcg M, int init, double tol2) {
     pdl_begin();
+    M = rhs_view<false>(M);
     const PcgArgs& A = M.a;
     RhsScalars* S = A.sc + cta_instance(A) * kMaxRhs;
     if (!init && !S[0].replace) return;
@@ -1623,7 +1660,7 @@ __global__ void __launch_bounds__(kThreads) k_mg_residual_split(MgPcg M, int ini
         const int lane = row & 31;
         float Sm[3] = {0.f, 0.f, 0.f}, Cc[3] = {0.f, 0.f, 0.f}, Dd[3] = {0.f, 0.f, 0.f};
         const int64_t g0 = A.slice_off[row >> 5];
-        const int len = A.row_len[row];
+        const int len = init == kZeroStart ? 0 : A.row_len[row];
         for (int j = 0; j < len; ++j) {
             const int64_t g = g0 + j;
             const int c = A.col[g * 32 + lane];
@@ -1677,9 +1714,10 @@ __global__ void __launch_bounds__(kThreads) k_mg_residual_split(MgPcg M, int ini
 // smoothing sweep.
 __global__ void __launch_bounds__(kThreads) k_mg_update_xr_pair(MgPcg M) {
     pdl_begin();
+    M = rhs_view<false>(M);
     const PcgArgs& A = M.a;
     RhsScalars* S = A.sc + cta_instance(A) * kMaxRhs;
-    if (cta_done<1>(A, S)) return;
+    if (mg_done(A, S)) return;
     F2 rr{0.f, 0.f};
     const F2 alpha{S[0].alpha2[0], S[0].alpha2[1]};
     for (int row = blockIdx.x * blockDim.x + threadIdx.x; row < A.n_rows; row += gridDim.x * blockDim.x) {
@@ -1725,9 +1763,10 @@ __global__ void __launch_bounds__(kThreads) k_mg_update_xr_pair(MgPcg M) {
 // after a true-residual evaluation, and p = z on a restart.
 __global__ void __launch_bounds__(kThreads) k_mg_rz_pair(MgPcg M, int mode) {
     pdl_begin();
+    M = rhs_view<false>(M);
     const PcgArgs& A = M.a;
     RhsScalars* S = A.sc + cta_instance(A) * kMaxRhs;
-    if (mode == 0 && cta_done<1>(A, S)) return;
+    if (mode == 0 && mg_done(A, S)) return;
     if (mode == 1 && !S[0].refresh) return;
     const bool restart = mode == 1 && S[0].restart;
     F2 a0{0.f, 0.f}, a1{0.f, 0.f};
@@ -1776,9 +1815,10 @@ __global__ void __launch_bounds__(kThreads) k_mg_rz_pair(MgPcg M, int mode) {
 // p = z + beta p in pairs
 __global__ void __launch_bounds__(kThreads) k_mg_update_p_pair(MgPcg M) {
     pdl_begin();
+    M = rhs_view<false>(M);
     const PcgArgs& A = M.a;
     RhsScalars* S = A.sc + cta_instance(A) * kMaxRhs;
-    if (cta_done<1>(A, S)) return;
+    if (mg_done(A, S)) return;
     const F2 beta{S[0].beta2[0], S[0].beta2[1]};
     for (int row = blockIdx.x * blockDim.x + threadIdx.x; row < A.n_rows; row += gridDim.x * blockDim.x) {
         const float4 z = M.z[row];
@@ -1800,9 +1840,10 @@ template <int G, int S>
 __global__ void __launch_bounds__(kThreads) k_mg_spmv_dot_staged(MgPcg M) {
     pdl_begin();
     extern __shared__ __align__(128) unsigned char st_smem[];
+    M = rhs_view<false>(M);
     const PcgArgs& A = M.a;
     RhsScalars* Sc = A.sc + cta_instance(A) * kMaxRhs;
-    if (cta_done<1>(A, Sc)) return;
+    if (mg_done(A, Sc)) return;
     F2 acc{0.f, 0.f};
     const bool ok = split_staged_slices<G, S>(
         A, A.p, st_smem, [&](int row, const F2 (&y)[3]) { acc = f2_add(acc, pair_ap_dot(A, row, y)); });
@@ -1817,7 +1858,7 @@ __global__ void __launch_bounds__(kThreads) k_mg_spmv_dot_staged(MgPcg M) {
 // otherwise or when one is asked for: register-fed, or staged with G groups per
 // stage and S stages per warp.
 template <int G, int S>
-void launch_staged(const Ctx& c, const MgPcg& M, int grid) {
+void launch_staged(const Ctx& c, const MgPcg& M, dim3 grid) {
     launch_k(c, k_mg_spmv_dot_staged<G, S>, grid, kThreads, SplitStage<G, S>::smem(kThreads), M);
 }
 
@@ -1840,9 +1881,9 @@ void product_attrs() {
     if (dev >= 0 && dev < 64) done[dev] = true;
 }
 
-void launch_split_product(Ctx& c, const MgPcg& M, int grid) {
+void launch_split_product(Ctx& c, const MgPcg& M, dim3 grid) {
     if (c.product_variant == ASEND_PRODUCT_DEFAULT && c.mg->box) {  // 36.8 against 118 us (200 x 40 x 40)
-        box_product(c, *c.mg->box, M.a);
+        box_product(c, *c.mg->box, M.a, (int)grid.y, M.part_stride);
         return;
     }
     switch (c.product_variant) {
@@ -1857,9 +1898,10 @@ void launch_split_product(Ctx& c, const MgPcg& M, int grid) {
 template <typename TP>
 __global__ void __launch_bounds__(kThreads) k_mg_update_xr(MgPcg M) {
     using PV = typename ApOf<TP>::T;
+    M = rhs_view<std::is_same<TP, float>::value>(M);
     const PcgArgs& A = M.a;
     RhsScalars* S = A.sc + cta_instance(A) * kMaxRhs;
-    if (cta_done<1>(A, S)) return;
+    if (mg_done(A, S)) return;
     const int row = blockIdx.x * blockDim.x + threadIdx.x;
     double d[1][1] = {{0.0}};
     if (row < A.n_rows) {
@@ -1903,9 +1945,10 @@ __global__ void __launch_bounds__(kThreads) k_mg_update_xr(MgPcg M) {
 template <typename TP>
 __global__ void __launch_bounds__(kThreads) k_mg_rz(MgPcg M, int mode) {
     using PV = typename ApOf<TP>::T;
+    M = rhs_view<std::is_same<TP, float>::value>(M);
     const PcgArgs& A = M.a;
     RhsScalars* S = A.sc + cta_instance(A) * kMaxRhs;
-    if (mode == 0 && cta_done<1>(A, S)) return;
+    if (mode == 0 && mg_done(A, S)) return;
     if (mode == 1 && !S[0].refresh) return;
     const int row = blockIdx.x * blockDim.x + threadIdx.x;
     double d[1][2] = {{0.0, 0.0}};
@@ -1943,9 +1986,10 @@ __global__ void __launch_bounds__(kThreads) k_mg_rz(MgPcg M, int mode) {
 template <typename TP>
 __global__ void __launch_bounds__(kThreads) k_mg_update_p(MgPcg M) {
     using PV = typename ApOf<TP>::T;
+    M = rhs_view<std::is_same<TP, float>::value>(M);
     const PcgArgs& A = M.a;
     RhsScalars* S = A.sc + cta_instance(A) * kMaxRhs;
-    if (cta_done<1>(A, S)) return;
+    if (mg_done(A, S)) return;
     const int row = blockIdx.x * blockDim.x + threadIdx.x;
     if (row >= A.n_rows) return;
     const double beta = S[0].beta;
@@ -1963,6 +2007,7 @@ __global__ void __launch_bounds__(kThreads) k_mg_update_p(MgPcg M) {
 template <bool PAIR_R>
 __global__ void __launch_bounds__(kThreads) k_mg_residual(MgPcg M, int init, double tol2) {
     pdl_begin();
+    M = rhs_view<false>(M);
     const PcgArgs& A = M.a;
     RhsScalars* S = A.sc + cta_instance(A) * kMaxRhs;
     if (!init && !S[0].replace) return;
@@ -1971,7 +2016,7 @@ __global__ void __launch_bounds__(kThreads) k_mg_residual(MgPcg M, int init, dou
         const int lane = row & 31;
         double y[3] = {0, 0, 0};
         const int64_t g0 = A.slice_off[row >> 5];
-        const int len = A.row_len[row];
+        const int len = init == kZeroStart ? 0 : A.row_len[row];
         for (int j = 0; j < len; ++j) {
             const int64_t g = g0 + j;
             const int c = A.col[g * 32 + lane];
@@ -2064,9 +2109,7 @@ void level_pattern(Ctx& c, MgLevel& L) {
     A.h_row_len.assign(N, 0);
     A.h_diag.assign(N, 0);
     for (int s = 0; s < A.n_slices; ++s) {
-        size_t w = 0;
-        for (int r = s * kSlice; r < std::min(N, (s + 1) * kSlice); ++r) w = std::max(w, adj[r].size());
-        A.h_slice_off[s + 1] = A.h_slice_off[s] + (int64_t)w;
+        A.h_slice_off[s + 1] = A.h_slice_off[s] + 27;  // known without the table (GeoView)
     }
     A.n_groups = A.h_slice_off[A.n_slices];
     A.h_col.assign((size_t)A.n_groups * kSlice, 0);
@@ -2159,8 +2202,26 @@ void level_tables(Ctx& c, MgHierarchy& H, int l) {
     pn[nb] = L.n_nodes;
     pe[nb] = L.n_el;
     L.d_blk.upload(dv, c.stream);
+    L.one = dv[0];
+    if (nb > 1) {
+        std::vector<int32_t> rb(L.n_nodes);
+        for (int b = 0; b < nb; ++b) std::fill(rb.begin() + pn[b], rb.begin() + pn[b + 1], b);
+        L.row_blk.upload(rb, c.stream);
+    }
     L.pre_node.upload(pn, c.stream);
     L.pre_el.upload(pe, c.stream);
+    ASEND_CUDA(cudaStreamSynchronize(c.stream));  // the host tables go out of scope
+}
+
+// The blocks of level C (with their finer blocks), found from the rows of R.
+GeoView geo_of(const MgLevel& C, const MgLevel& R) {
+    GeoView g{};
+    g.n_rows = C.n_nodes;
+    g.blk = C.d_blk.p;
+    g.row_blk = C.blk.size() > 1 ? R.row_blk.p : nullptr;
+    g.one = C.one;
+    g.v = C.own.v32.p;
+    return g;
 }
 
 LevelView view_of(const MgLevel& L) {
@@ -2360,21 +2421,6 @@ void build_hierarchy(Ctx& c) {
     if (dense_tot > (size_t)INT32_MAX) throw InputError("multigrid coarsest blocks too large");
     H->dense.alloc(dense_tot);
     for (int l = 0; l < (int)H->L.size(); ++l) level_tables(c, *H, l);
-    // fused tail: the deepest levels whose every block has <= kTailNodes
-    // nodes, if there are at least two (one besides the coarsest)
-    {
-        const int nl = (int)H->L.size();
-        int lt = nl;
-        for (int l = nl - 1; l >= 1; --l) {
-            int mx = 0;
-            for (const MgBlk& B : H->L[l]->blk) mx = std::max(mx, B.n_nodes());
-            if (mx > kTailNodes) break;
-            lt = l;
-        }
-        // only for stacks of many instances: one CTA cannot carry a lone
-        // block's small levels as fast as the grid-wide launches do
-        H->tail = (H->n_blk >= kTailMinBlocks && nl - lt >= 2 && nl - lt <= kMaxTail) ? lt : 0;
-    }
     ASEND_CUDA(cudaStreamSynchronize(c.stream));
     c.mg = H;
 }
@@ -2513,29 +2559,28 @@ void setup_values(Ctx& c, bool skip_l0) {
 
 // Restriction of level l's residual r to level l + 1's right-hand side b (and
 // its first smoothing sweep, unless l + 1 is the coarsest level).
-void restrict_to(Ctx& c, int l, const Control* ctl) {
+void restrict_to(Ctx& c, int l, const Control* ctl, int nr = 1) {
     MgHierarchy& H = *c.mg;
     MgLevel& L = *H.L[l];
     MgLevel& C = *H.L[l + 1];
     const bool last = (l + 2 == (int)H.L.size());  // the coarsest level is solved directly: no sweep
-    launch_k(c, k_vc_restrict, grid_of(C.n_nodes), kT, 0, view_of(C), C.pre_node.p, C.n_nodes, L.r.p, C.b.p,
-                                                           last ? nullptr : C.binv.p,
-                                                           reinterpret_cast<float4*>(C.x4.p), ctl);
+    launch_k(c, k_vc_restrict, dim3(grid_of(4 * C.n_nodes), nr), kT, 0, geo_of(C, C), L.n_nodes, L.r.p, C.b.p,
+             last ? nullptr : C.binv.p, reinterpret_cast<float4*>(C.x4.p), ctl);
 }
 
-void coarsest_solve(Ctx& c, const Control* ctl) {
+void coarsest_solve(Ctx& c, const Control* ctl, int nr = 1) {
     MgHierarchy& H = *c.mg;
     MgLevel& Lc = *H.L.back();
-    launch_k(c, k_vc_dense, H.n_blk, 1024, 0, view_of(Lc), H.dense.p, Lc.b.p, Lc.y4.p, ctl);
+    launch_k(c, k_vc_dense, dim3(H.n_blk, nr, (H.n_coarse + kDenseRows - 1) / kDenseRows), 32 * kDenseRows, 0,
+             geo_of(Lc, Lc), H.dense.p, Lc.b.p, Lc.y4.p, ctl);
 }
 
-void prolong_from(Ctx& c, int l, const Control* ctl) {
+void prolong_from(Ctx& c, int l, const Control* ctl, int nr = 1) {
     MgHierarchy& H = *c.mg;
     MgLevel& L = *H.L[l];
     MgLevel& C = *H.L[l + 1];
-    launch_k(c, k_vc_prolong, grid_of(L.n_nodes), kT, 0, view_of(C), L.pre_node.p, L.n_nodes,
-                                                          reinterpret_cast<const float4*>(C.y4.p),
-                                                          reinterpret_cast<float4*>(L.x4.p), ctl);
+    launch_k(c, k_vc_prolong, dim3(grid_of(L.n_nodes), nr), kT, 0, geo_of(C, L), L.n_nodes,
+             reinterpret_cast<const float4*>(C.y4.p), reinterpret_cast<float4*>(L.x4.p), ctl);
 }
 
 // One V(1,1) cycle on level 0's b.  With fused0, the caller has already
@@ -2554,108 +2599,93 @@ int lanes_for(int n_rows) {
 // products, one row per lane; smaller ones split each row over T lanes.
 constexpr int kStagedRows = 8192;
 
-void level_resid(Ctx& c, MgLevel& L, const Control* ctl) {
-    if (c.mg->box && c.mg->box_cycle && &L == c.mg->L[0].get()) {
-        box_resid(c, *c.mg->box, L.b.p, reinterpret_cast<const float4*>(L.x4.p), L.r.p, ctl);
-        return;
-    }
-    const int t = L.n_nodes >= kStagedRows ? 1 : lanes_for(L.n_nodes);
-    const SbView A = sbview(L);
-    const float4* x = reinterpret_cast<const float4*>(L.x4.p);
-    const int g = (int)(((int64_t)L.n_nodes * t + kT - 1) / kT);
-    switch (t) {
-        case 1:
-            launch_k(c, k_vc_resid_staged, std::min(grid_of(L.n_nodes), kPersistCtas), kT,
-                     (size_t)F32Stage<kVcG, kVcS>::smem(kT), A, L.b.p, x, L.r.p, ctl);
-            break;
-        case 2: launch_k(c, k_vc_resid_t<2>, g, kT, 0, A, L.b.p, x, L.r.p, ctl); break;
-        case 4: launch_k(c, k_vc_resid_t<4>, g, kT, 0, A, L.b.p, x, L.r.p, ctl); break;
-        case 8: launch_k(c, k_vc_resid_t<8>, g, kT, 0, A, L.b.p, x, L.r.p, ctl); break;
-        default: launch_k(c, k_vc_resid_t<16>, g, kT, 0, A, L.b.p, x, L.r.p, ctl); break;
-    }
-}
-
-void level_post(Ctx& c, MgLevel& L, const Control* ctl);
-void level_resid_or_post(Ctx& c, MgLevel& L, bool post, const Control* ctl) {
-    if (post) level_post(c, L, ctl);
-    else level_resid(c, L, ctl);
-}
-
-void level_post(Ctx& c, MgLevel& L, const Control* ctl) {
-    if (c.mg->box && c.mg->box_cycle && &L == c.mg->L[0].get()) {
-        box_post(c, *c.mg->box, L.binv.p, L.b.p, reinterpret_cast<const float4*>(L.x4.p),
-                 reinterpret_cast<float4*>(L.y4.p), ctl);
-        return;
-    }
-    const int t = L.n_nodes >= kStagedRows ? 1 : lanes_for(L.n_nodes);
-    const SbView A = sbview(L);
+template <bool POST>
+void launch_rows(Ctx& c, MgLevel& L, int t, const Control* ctl, int nr) {
+    const dim3 grid((unsigned)(((int64_t)L.n_nodes * t + kT - 1) / kT), nr);
+    const GeoView G = geo_of(L, L);
     const float4* x = reinterpret_cast<const float4*>(L.x4.p);
     float4* y = reinterpret_cast<float4*>(L.y4.p);
-    const int g = (int)(((int64_t)L.n_nodes * t + kT - 1) / kT);
+    auto go = [&](auto k) { launch_k(c, k, grid, kT, 0, G, L.binv.p, L.b.p, x, L.r.p, y, ctl); };
     switch (t) {
-        case 1:
-            launch_k(c, k_vc_post_staged, std::min(grid_of(L.n_nodes), kPersistCtas), kT,
-                     (size_t)F32Stage<kVcG, kVcS>::smem(kT), A, L.binv.p, L.b.p, x, y, ctl);
-            break;
-        case 2: launch_k(c, k_vc_post_t<2>, g, kT, 0, A, L.binv.p, L.b.p, x, y, ctl); break;
-        case 4: launch_k(c, k_vc_post_t<4>, g, kT, 0, A, L.binv.p, L.b.p, x, y, ctl); break;
-        case 8: launch_k(c, k_vc_post_t<8>, g, kT, 0, A, L.binv.p, L.b.p, x, y, ctl); break;
-        default: launch_k(c, k_vc_post_t<16>, g, kT, 0, A, L.binv.p, L.b.p, x, y, ctl); break;
+        case 2: go(k_vc_rows<2, POST>); break;
+        case 4: go(k_vc_rows<4, POST>); break;
+        case 8: go(k_vc_rows<8, POST>); break;
+        default: go(k_vc_rows<16, POST>); break;
     }
 }
 
-// First level of the fused coarse tail in use (nl - 1: no tail, the
-// coarsest level alone is solved by its own launch).
-int tail_level(const Ctx& c) {
-    const MgHierarchy& H = *c.mg;
-    const int nl = (int)H.L.size();
-    return (c.mg_tail && H.tail > 0) ? H.tail : nl - 1;
-}
-
-// Levels lt .. nl - 1 in one launch of k_vc_tail (one CTA per block).
-void launch_tail(Ctx& c, int lt, const Control* ctl) {
+// Residual r = b - A x (post = false) or post-smoothing y4 = x + B^-1 (b - A x) of
+// level l for nr right-hand sides: matrix-free on the finest level of a box
+// model inside the CG, staged for many rows, several lanes a row for few.
+void level_rows(Ctx& c, int l, bool post, const Control* ctl, int nr = 1) {
     MgHierarchy& H = *c.mg;
-    TailArgs ta;
-    std::memset(&ta, 0, sizeof(ta));
-    ta.n_lev = (int)H.L.size() - lt;
-    for (int i = 0; i < ta.n_lev; ++i) {
-        MgLevel& L = *H.L[lt + i];
-        TailLevel& T = ta.L[i];
-        T.A = sbview(L);
-        T.V = view_of(L);
-        T.binv = L.binv.p;
-        T.b = L.b.p;
-        T.r = L.r.p;
-        T.x4 = reinterpret_cast<float4*>(L.x4.p);
-        T.y4 = reinterpret_cast<float4*>(L.y4.p);
-        T.lanes = lanes_for(L.n_nodes);
+    MgLevel& L = *H.L[l];
+    const float4* x = reinterpret_cast<const float4*>(L.x4.p);
+    float4* y = reinterpret_cast<float4*>(L.y4.p);
+    if (l == 0 && H.box && H.box_cycle) {
+        if (post) box_post(c, *H.box, L.binv.p, L.b.p, x, y, ctl, nr);
+        else box_resid(c, *H.box, L.b.p, x, L.r.p, ctl, nr);
+        return;
     }
-    ta.ainv = H.dense.p;
-    launch_k(c, k_vc_tail, H.n_blk, kTailThreads, 0, ta, ctl);
+    const int t = L.n_nodes >= kStagedRows ? 1 : lanes_for(L.n_nodes);
+    if (t > 1 && l > 0) {
+        if (post) launch_rows<true>(c, L, t, ctl, nr);
+        else launch_rows<false>(c, L, t, ctl, nr);
+        return;
+    }
+    if (t > 1) {  // a small finest level: any pattern
+        const SbView A = sbview(L);
+        const dim3 grid((unsigned)(((int64_t)L.n_nodes * t + kT - 1) / kT), nr);
+        auto go = [&](auto k) { launch_k(c, k, grid, kT, 0, A, L.binv.p, L.b.p, x, L.r.p, y, ctl); };
+        switch (t) {
+            case 2: post ? go(k_vc_rows_any<2, true>) : go(k_vc_rows_any<2, false>); break;
+            case 4: post ? go(k_vc_rows_any<4, true>) : go(k_vc_rows_any<4, false>); break;
+            case 8: post ? go(k_vc_rows_any<8, true>) : go(k_vc_rows_any<8, false>); break;
+            default: post ? go(k_vc_rows_any<16, true>) : go(k_vc_rows_any<16, false>); break;
+        }
+        return;
+    }
+    const dim3 grid(std::min(grid_of(L.n_nodes), kPersistCtas), nr);
+    const size_t smem = (size_t)F32Stage<kVcG, kVcS>::smem(kT);
+    if (post) launch_k(c, k_vc_post_staged, grid, kT, smem, sbview(L), L.binv.p, L.b.p, x, y, ctl);
+    else launch_k(c, k_vc_resid_staged, grid, kT, smem, sbview(L), L.b.p, x, L.r.p, ctl);
 }
 
-void vcycle(Ctx& c, const Control* ctl, bool fused0) {
+void vcycle(Ctx& c, const Control* ctl, bool fused0, int nr = 1) {
     MgHierarchy& H = *c.mg;
     const int nl = (int)H.L.size();
-    const int lt = tail_level(c);
     if (!fused0 && nl > 1) {
         MgLevel& L = *H.L[0];
-        launch_k(c, k_vc_smooth0, grid_of(L.n_nodes), kT, 0, L.n_nodes, L.binv.p, L.b.p,
-                                                              reinterpret_cast<float4*>(L.x4.p), ctl);
+        launch_k(c, k_vc_smooth0, dim3(grid_of(L.n_nodes), nr), kT, 0, L.n_nodes, L.binv.p, L.b.p,
+                 reinterpret_cast<float4*>(L.x4.p), ctl);
     }
-    for (int l = 0; l < lt; ++l) {
-        level_resid(c, *H.L[l], ctl);
-        restrict_to(c, l, ctl);
+    for (int l = 0; l < nl - 1; ++l) {
+        level_rows(c, l, false, ctl, nr);
+        restrict_to(c, l, ctl, nr);
     }
-    if (lt < nl - 1) launch_tail(c, lt, ctl);
-    else coarsest_solve(c, ctl);
-    for (int l = lt - 1; l >= 0; --l) {
-        prolong_from(c, l, ctl);
-        level_post(c, *H.L[l], ctl);
+    coarsest_solve(c, ctl, nr);
+    for (int l = nl - 2; l >= 0; --l) {
+        prolong_from(c, l, ctl, nr);
+        level_rows(c, l, true, ctl, nr);
     }
 }
 
-int vcycle_launches(const Ctx& c) { return 4 * tail_level(c) + 1; }
+int vcycle_launches(const Ctx& c) { return 4 * ((int)c.mg->L.size() - 1) + 1; }
+
+// Level vectors for nr right-hand sides (grow only; the captured graphs hold
+// their addresses).
+void level_vectors(MgHierarchy& H, int nr) {
+    for (auto& Lp : H.L) {
+        MgLevel& L = *Lp;
+        if (L.b.n >= (size_t)nr * L.n_dof) continue;
+        for (auto& g : H.graphs) cudaGraphExecDestroy(g.second);
+        H.graphs.clear();
+        L.b.alloc((size_t)nr * L.n_dof);
+        L.r.alloc((size_t)nr * L.n_dof);
+        L.x4.alloc((size_t)nr * 4 * L.n_nodes);
+        L.y4.alloc((size_t)nr * 4 * L.n_nodes);
+    }
+}
 
 // L0.x4 = P C R (L0.r): the coarse-grid correction of one V-cycle alone
 // (restriction of level 0's r, the V-cycle of the coarser levels, and the
@@ -2760,7 +2790,10 @@ double mg_time_kernel(Ctx& c, int kernel, int method, int n_launch, double* byte
     ctl.alloc(1);
     tk.alloc((size_t)NI * 4);
     sc.zero(c.stream);
-    ctl.zero(c.stream);
+    Control on;
+    std::memset(&on, 0, sizeof(on));
+    on.active[0] = 1;  // or the kernels would have nothing to do
+    ctl.upload(&on, 1, c.stream);
     tk.zero(c.stream);
     part.alloc((size_t)std::max(grid, H.box ? box_ctas(*H.box) : 0) * kMaxRhs * 3);
     p.alloc((size_t)4 * n);
@@ -2782,8 +2815,9 @@ double mg_time_kernel(Ctx& c, int kernel, int method, int n_launch, double* byte
     a.partials = part.p;
     a.sc = sc.p;
     a.ctl = ctl.p;
-    a.tickets = NI > 1 ? tk.p : nullptr;
+    a.tickets = tk.p;
     M.n_inst = 1;
+    M.part_stride = 0;
     // the direction's values do not change the kernels' work: zeros
     ASEND_CUDA(cudaMemsetAsync(p.p, 0, sizeof(double) * 4 * n, c.stream));
     auto launch = [&]() {
@@ -2792,7 +2826,7 @@ double mg_time_kernel(Ctx& c, int kernel, int method, int n_launch, double* byte
             else if (method == ASEND_METHOD_SPLIT) launch_split_product(c, M, grid);
             else k_mg_spmv_dot<double, double><<<grid, kThreads, 0, c.stream>>>(M);
         } else {  // the finest level's products as the V-cycle runs them
-            level_resid_or_post(c, L0, kernel == 2, nullptr);
+            level_rows(c, 0, kernel == 2, nullptr);
         }
     };
     const double ps = (method == ASEND_METHOD_MIXED) ? 4.0 : 8.0;  // bytes per value / direction entry
@@ -2921,7 +2955,7 @@ int pcg_solve_mg_once(Ctx& c, const asend_solve_opts& o, asend_solve_stats* st, 
                       double* d_x, int nrhs_all);
 }
 
-// Multigrid-preconditioned flexible CG, one right-hand side at a time.  A
+// Multigrid-preconditioned flexible CG, up to four right-hand sides at a time.  A
 // solve that turns non-finite (a smoother damped from an eigenvalue estimate
 // that fell short of a localised top mode) is repeated from zero with every
 // level's damping taken from the guaranteed bound ||D^-1 A||_inf, which then
@@ -2952,8 +2986,11 @@ int pcg_solve_mg_once(Ctx& c, const asend_solve_opts& o, asend_solve_stats* st, 
     if (!warm) ASEND_CUDA(cudaMemsetAsync(d_x, 0, (size_t)nrhs_all * nd * sizeof(double), c.stream));
     c.d_r.alloc(std::max(c.d_r.n, (size_t)nrhs_all * nd));
     const int grid = grid_of(n);
-    const size_t n_part = (size_t)std::max(grid, H.box ? box_ctas(*H.box) : 0);
-    c.d_partials.alloc(std::max(c.d_partials.n, n_part * kMaxRhs * 3));
+    // eight lanes a row where one thread a row leaves more than half the GPU idle
+    const bool fp64_lanes = !mixed && !split && c.n_inst <= 1 && lanes_for(n) > 2;
+    const size_t n_part = (size_t)std::max({grid, H.box ? box_ctas(*H.box) : 0, fp64_lanes ? grid_of(8 * n) : 0});
+    const int nr_max = std::min(nrhs_all, kMaxRhs);
+    c.d_partials.alloc(std::max(c.d_partials.n, nr_max * n_part * kMaxRhs * 3));
     if (mixed) {
         c.d_p32.alloc(std::max(c.d_p32.n, (size_t)kMaxRhs * 4 * n));
         c.d_ap32.alloc(std::max(c.d_ap32.n, (size_t)kMaxRhs * nd));
@@ -2961,17 +2998,18 @@ int pcg_solve_mg_once(Ctx& c, const asend_solve_opts& o, asend_solve_stats* st, 
         c.d_p64.alloc(std::max(c.d_p64.n, (size_t)kMaxRhs * 4 * n));
         c.d_ap64.alloc(std::max(c.d_ap64.n, (size_t)kMaxRhs * nd));
     }
-    if (split) c.d_xpair.alloc(std::max(c.d_xpair.n, (size_t)2 * n));
-    if (split_only) c.d_xtrip.alloc(std::max(c.d_xtrip.n, (size_t)3 * n));
-    // one scalar set per instance (slot 0 of kMaxRhs), persistent so the
+    if (split) c.d_xpair.alloc(std::max(c.d_xpair.n, (size_t)nr_max * 2 * n));
+    if (split_only) c.d_xtrip.alloc(std::max(c.d_xtrip.n, (size_t)nr_max * 3 * n));
+    level_vectors(H, nr_max);
+    // one scalar set per instance and right-hand side, persistent so the
     // captured iteration graphs stay valid across solves
     const int NI = c.n_inst > 1 ? c.n_inst : 1;
     // a batched stack keeps one CTA per 128 rows (its reductions are per instance)
     const int grid_cg = (split && NI == 1) ? std::min(grid, kPersistCtas) : grid;
-    const size_t sc_need = sizeof(RhsScalars) * NI * kMaxRhs, tk_need = sizeof(uint32_t) * NI * 4;
+    const size_t sc_need = sizeof(RhsScalars) * NI * kMaxRhs, tk_need = sizeof(uint32_t) * NI * 4 * kMaxRhs;
     if (c.pcg_sc.n < sc_need) c.pcg_sc.alloc(sc_need);
     if (c.pcg_ctl.n < sizeof(Control)) c.pcg_ctl.alloc(sizeof(Control));
-    if (NI > 1 && c.pcg_tk.n < tk_need) c.pcg_tk.alloc(tk_need);
+    if (c.pcg_tk.n < tk_need) c.pcg_tk.alloc(tk_need);
     RhsScalars* d_sc = reinterpret_cast<RhsScalars*>(c.pcg_sc.p);
     Control* d_ctl = reinterpret_cast<Control*>(c.pcg_ctl.p);
     ensure_pinned_scalars(c, sc_need);
@@ -2980,12 +3018,13 @@ int pcg_solve_mg_once(Ctx& c, const asend_solve_opts& o, asend_solve_stats* st, 
     double relmax = 0.0;
     MgLevel& L0 = *H.L[0];
     ASEND_CUDA(cudaEventRecord(c.ev0, c.stream));
-    for (int r0 = 0; r0 < nrhs_all; ++r0) {
+    for (int r0 = 0; r0 < nrhs_all; r0 += kMaxRhs) {
+        const int nr = std::min(kMaxRhs, nrhs_all - r0);
         MgPcg M;
         std::memset(&M, 0, sizeof(M));  // padding too: the bytes key the cached graph
         PcgArgs& a = M.a;
         a.n_rows = n;
-        a.nrhs = 1;
+        a.nrhs = nr;
         a.n_dof = nd;
         a.slice_off = c.A.slice_off.p;
         a.row_len = c.A.row_len.p;
@@ -3005,79 +3044,80 @@ int pcg_solve_mg_once(Ctx& c, const asend_solve_opts& o, asend_solve_stats* st, 
             a.cta_inst = c.d_cta_inst.p;
             a.inst_cta0 = c.d_inst_cta0.p;
             a.inst_ncta = c.d_inst_ncta.p;
-            a.tickets = reinterpret_cast<uint32_t*>(c.pcg_tk.p);
-            ASEND_CUDA(cudaMemsetAsync(c.pcg_tk.p, 0, tk_need, c.stream));
         }
+        a.tickets = reinterpret_cast<uint32_t*>(c.pcg_tk.p);
+        ASEND_CUDA(cudaMemsetAsync(c.pcg_tk.p, 0, tk_need, c.stream));
         M.b0 = L0.b.p;
         M.z = reinterpret_cast<const float4*>(L0.y4.p);
         M.binv0 = L0.binv.p;
         M.x40 = reinterpret_cast<float4*>(L0.x4.p);
         M.n_inst = NI;
+        M.part_stride = (int)n_part;
         if (split) {  // the split method's correction e (FP32 pairs) starts at zero
             M.xp = c.d_xpair.p;
             M.xt = split_only ? c.d_xtrip.p : nullptr;
-            k_zero_pairs<<<(2 * n + kThreads - 1) / kThreads, kThreads, 0, c.stream>>>(n, M.xp);
-            ++c.launches;
+            ASEND_CUDA(cudaMemsetAsync(M.xp, 0, sizeof(float4) * 2 * n * nr, c.stream));
         }
         ASEND_CUDA(cudaMemsetAsync(d_sc, 0, sc_need, c.stream));
         ASEND_CUDA(cudaMemsetAsync(d_ctl, 0, sizeof(Control), c.stream));
         auto launch_residual = [&](int init) {
             if (split) {  // x64 += e first (the instances being replaced), then r = f - A64 x64
-                launch_k(c, k_fold_pairs, grid_cg, kThreads, 0, M, init);
+                launch_k(c, k_fold_pairs, dim3(grid_cg, nr), kThreads, 0, M, init);
                 if (split_only)
-                    launch_k(c, k_mg_residual_split, grid, kThreads, 0, M, init, o.rel_tol * o.rel_tol);
+                    launch_k(c, k_mg_residual_split, dim3(grid, nr), kThreads, 0, M, init, o.rel_tol * o.rel_tol);
                 else  // FP64-pipe bound: all 4 warps of every row tile in flight
-                    launch_k(c, k_mg_residual<true>, grid, kThreads, 0, M, init, o.rel_tol * o.rel_tol);
+                    launch_k(c, k_mg_residual<true>, dim3(grid, nr), kThreads, 0, M, init, o.rel_tol * o.rel_tol);
                 c.launches += 2;
             } else {
-                launch_k(c, k_mg_residual<false>, grid, kThreads, 0, M, init, o.rel_tol * o.rel_tol);
+                launch_k(c, k_mg_residual<false>, dim3(grid, nr), kThreads, 0, M, init, o.rel_tol * o.rel_tol);
                 ++c.launches;
             }
         };
         auto launch_iteration = [&]() {
             if (mixed) {
-                k_mg_spmv_dot<float, float><<<grid, kThreads, 0, c.stream>>>(M);
-                k_mg_update_xr<float><<<grid, kThreads, 0, c.stream>>>(M);
+                k_mg_spmv_dot<float, float><<<dim3(grid, nr), kThreads, 0, c.stream>>>(M);
+                k_mg_update_xr<float><<<dim3(grid, nr), kThreads, 0, c.stream>>>(M);
             } else if (split) {
-                launch_split_product(c, M, grid_cg);
-                launch_k(c, k_mg_update_xr_pair, grid_cg, kThreads, 0, M);
+                launch_split_product(c, M, dim3(grid_cg, nr));
+                launch_k(c, k_mg_update_xr_pair, dim3(grid_cg, nr), kThreads, 0, M);
             } else {
-                k_mg_spmv_dot<double, double><<<grid, kThreads, 0, c.stream>>>(M);
-                k_mg_update_xr<double><<<grid, kThreads, 0, c.stream>>>(M);
+                if (fp64_lanes) k_mg_spmv_dot_lanes<8><<<dim3(grid_of(8 * n), nr), kThreads, 0, c.stream>>>(M);
+                else k_mg_spmv_dot<double, double><<<dim3(grid, nr), kThreads, 0, c.stream>>>(M);
+                k_mg_update_xr<double><<<dim3(grid, nr), kThreads, 0, c.stream>>>(M);
             }
-            vcycle(c, a.ctl, true);
+            vcycle(c, a.ctl, true, nr);
             if (mixed) {
-                k_mg_rz<float><<<grid, kThreads, 0, c.stream>>>(M, 0);
-                k_mg_update_p<float><<<grid, kThreads, 0, c.stream>>>(M);
+                k_mg_rz<float><<<dim3(grid, nr), kThreads, 0, c.stream>>>(M, 0);
+                k_mg_update_p<float><<<dim3(grid, nr), kThreads, 0, c.stream>>>(M);
             } else if (split) {
-                launch_k(c, k_mg_rz_pair, grid_cg, kThreads, 0, M, 0);
-                launch_k(c, k_mg_update_p_pair, grid_cg, kThreads, 0, M);
+                launch_k(c, k_mg_rz_pair, dim3(grid_cg, nr), kThreads, 0, M, 0);
+                launch_k(c, k_mg_update_p_pair, dim3(grid_cg, nr), kThreads, 0, M);
             } else {
-                k_mg_rz<double><<<grid, kThreads, 0, c.stream>>>(M, 0);
-                k_mg_update_p<double><<<grid, kThreads, 0, c.stream>>>(M);
+                k_mg_rz<double><<<dim3(grid, nr), kThreads, 0, c.stream>>>(M, 0);
+                k_mg_update_p<double><<<dim3(grid, nr), kThreads, 0, c.stream>>>(M);
             }
         };
         // V-cycle of every instance's current b0, then rz (and p = z on a
         // restart) for the instances the residual kernel marked
         auto launch_start = [&]() {
-            vcycle(c, nullptr, false);
-            if (mixed) k_mg_rz<float><<<grid, kThreads, 0, c.stream>>>(M, 1);
-            else if (split) launch_k(c, k_mg_rz_pair, grid_cg, kThreads, 0, M, 1);
-            else k_mg_rz<double><<<grid, kThreads, 0, c.stream>>>(M, 1);
+            vcycle(c, nullptr, false, nr);
+            if (mixed) k_mg_rz<float><<<dim3(grid, nr), kThreads, 0, c.stream>>>(M, 1);
+            else if (split) launch_k(c, k_mg_rz_pair, dim3(grid_cg, nr), kThreads, 0, M, 1);
+            else k_mg_rz<double><<<dim3(grid, nr), kThreads, 0, c.stream>>>(M, 1);
             c.launches += vcycle_launches(c) + 2;
         };
-        launch_residual(1);
+        launch_residual(warm ? 1 : kZeroStart);
         launch_start();
         ASEND_CUDA(cudaGetLastError());
         // G iterations as one graph, kept with the hierarchy and reused while
         // the launch arguments are the same (they fully define the graph)
         // (with everything else that changes the captured sequence: the
-        // method, the chunk length, the product shape, the tail switch, the
-        // launch overlap and the matrix-free plan)
+        // method, the chunk length, the product shape, the launch overlap and
+        // the matrix-free plan)
         std::vector<uint8_t> key(sizeof(MgPcg) + 4 * sizeof(int) + sizeof(void*));
         std::memcpy(key.data(), &M, sizeof(MgPcg));
         std::memcpy(key.data() + sizeof(MgPcg) + 4 * sizeof(int), &H.box, sizeof(void*));
-        const int extra[4] = {o.method, G, c.product_variant, (c.mg_tail ? 1 : 0) | (c.pdl ? 2 : 0)};
+        const int extra[4] = {o.method, G, c.product_variant, (H.box_cycle ? 1 : 0) | (c.pdl ? 2 : 0)};
         std::memcpy(key.data() + sizeof(MgPcg), extra, sizeof(extra));
         cudaGraphExec_t exec = nullptr;
         for (auto& g : H.graphs)
@@ -3085,7 +3125,7 @@ int pcg_solve_mg_once(Ctx& c, const asend_solve_opts& o, asend_solve_stats* st, 
         if (!exec) {
             cudaGraph_t graph;
             ASEND_CUDA(cudaStreamBeginCapture(c.stream, cudaStreamCaptureModeThreadLocal));
-            launch_k(c, k_mg_count_active, 1, 32, 0, M);
+            launch_k(c, k_mg_count_active, nr, 32, 0, M);
             for (int i = 0; i < G; ++i) launch_iteration();
             ASEND_CUDA(cudaStreamEndCapture(c.stream, &graph));
             ASEND_CUDA(cudaGraphInstantiate(&exec, graph, 0));
@@ -3104,8 +3144,9 @@ int pcg_solve_mg_once(Ctx& c, const asend_solve_opts& o, asend_solve_stats* st, 
             ASEND_CUDA(cudaStreamSynchronize(c.stream));
             bool all_finished = true, any_replace = false, any_nonfinite = false;
             int it_now = 0;
-            for (int i = 0; i < NI; ++i) {
-                RhsScalars& s = h[(size_t)i * kMaxRhs];
+            for (int q = 0; q < NI * kMaxRhs; ++q) {
+                if (q % kMaxRhs >= nr) continue;
+                RhsScalars& s = h[q];
                 it_now = std::max(it_now, (int)s.iter);
                 if (s.nonfinite) { any_nonfinite = true; continue; }
                 if (s.finished) continue;
@@ -3136,13 +3177,14 @@ int pcg_solve_mg_once(Ctx& c, const asend_solve_opts& o, asend_solve_stats* st, 
             since_repl += G;
         }
         if (split) {  // the solution: x64 + e
-            launch_k(c, k_fold_pairs, grid_cg, kThreads, 0, M, 1);
+            launch_k(c, k_fold_pairs, dim3(grid_cg, nr), kThreads, 0, M, 1);
             ++c.launches;
         }
         ASEND_CUDA(cudaMemcpyAsync(h, d_sc, sc_bytes, cudaMemcpyDeviceToHost, c.stream));
         ASEND_CUDA(cudaStreamSynchronize(c.stream));
-        for (int i = 0; i < NI; ++i) {
-            const RhsScalars& s = h[(size_t)i * kMaxRhs];
+        for (int q = 0; q < NI * kMaxRhs; ++q) {
+            if (q % kMaxRhs >= nr) continue;
+            const RhsScalars& s = h[q];
             iters_max = std::max(iters_max, (int)s.iter);
             if (s.nonfinite) status = ASEND_NONFINITE;
             else if (!s.finished) status = std::max(status, (int)ASEND_MAX_ITER);

@@ -22,7 +22,8 @@ struct RhsScalars {
 struct Control {
     int32_t all_done;
     uint32_t ticket[4];
-    int32_t pad[3];  // pad[0]: instances still iterating (multigrid CG)
+    int32_t pad[3];  // pad[0]: right-hand sides still iterating (multigrid CG)
+    int32_t active[kMaxRhs];  // instances still iterating, per right-hand side (multigrid CG)
 };
 
 struct PcgArgs {
