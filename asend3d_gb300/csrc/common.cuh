@@ -216,6 +216,9 @@ struct Ctx {
     // A split-only assembly (precision 48) writes the operator's FP32 hi / lo
     // values and leaves the FP64 copy stale until ensure_v64() rebuilds it.
     bool v64_valid = true;
+    // a split-only assembly whose FP64 diagonal blocks have been used: the
+    // smoother takes them too (the sums of the pairs)
+    bool diag64 = false;
     float last_assemble_ms = 0.f;
 
     // ---- pattern / assembly

@@ -1055,6 +1055,7 @@ void assemble_operator(Ctx& c, int precision) {
     ASEND_CUDA(cudaEventElapsedTime(&ms, c.ev0, c.ev1));
     c.assembled_precision = precision;
     c.v64_valid = !split_only;
+    c.diag64 = false;
     c.class_sum = (gather || split_only) && c.cM == 0.0;
     c.class_pairs = split_only;
     ++c.assembly_epoch;

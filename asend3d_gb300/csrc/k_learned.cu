@@ -48,6 +48,7 @@ struct LearnedState {
     DArr<int32_t> nel_ptr, nel;        // node -> adjacent elements
     DArr<float> gpart, binv;           // per-CTA gradient partials, training blocks
     DArr<double> part;
+    DArr<double> log_E;                // log modulus less its mean, per element
     int n_samples = 0, step = 0;
     int objective = ASEND_LEARN_BLOCK;  // loss the training minimises
     bool have_weights = false;
@@ -67,21 +68,39 @@ constexpr int bW1 = 0, bW2 = bW1 + kNW1, bW3 = bW2 + kNW2, bEnd = bW3 + kNW3;
 // ---------------------------------------------------------------------------
 // features
 // ---------------------------------------------------------------------------
-__device__ __forceinline__ void diag_block(const int64_t* slice_off, const uint8_t* diag, const double* v64, int row,
-                                           double (&m)[9]) {
-    const int64_t g = slice_off[row >> 5] + diag[row];
+// The operator's FP64 values: stored, or (v64 null) the sums of the pairs, as
+// k_pairs_to64 forms them (27 blocks a row of which the features need one: 2,130 MB
+// of traffic and 726 us at 1.6 M DOF)
+struct DiagView {
+    const int64_t* slice_off;
+    const uint8_t* diag;
+    const double* v64;
+    const float* hi;
+    const float* lo;
+};
+__device__ __forceinline__ void diag_block(const DiagView& A, int row, double (&m)[9]) {
+    const int64_t g = A.slice_off[row >> 5] + A.diag[row];
     const int lane = row & 31;
 #pragma unroll
-    for (int q = 0; q < 9; ++q) m[q] = v64[(g * 9 + q) * 32 + lane];
+    for (int q = 0; q < 9; ++q) {
+        const size_t at = (g * 9 + q) * 32 + lane;
+        m[q] = A.v64 ? A.v64[at] : (double)A.hi[at] + (double)A.lo[at];
+    }
 }
 
-__global__ void k_logtrace_sum(int n, const int64_t* slice_off, const uint8_t* diag, const double* v64,
-                               double* part) {
+// log E - mean of every element, once: 8 elements share a node, and an FP64
+// logarithm costs more than the rest of a node's features
+__global__ void k_log_modulus(int n, const double* __restrict__ E, double mean_logE, double* __restrict__ out) {
+    const int e = blockIdx.x * blockDim.x + threadIdx.x;
+    if (e < n) out[e] = log(E[e]) - mean_logE;
+}
+
+__global__ void k_logtrace_sum(int n, DiagView A, double* part) {
     __shared__ double sm[32];
     double v[1] = {0.0};
     for (int row = blockIdx.x * blockDim.x + threadIdx.x; row < n; row += gridDim.x * blockDim.x) {
         double m[9];
-        diag_block(slice_off, diag, v64, row, m);
+        diag_block(A, row, m);
         v[0] += log((m[0] + m[4] + m[8]) / 3.0);
     }
     block_sum<1>(v, sm);
@@ -89,13 +108,13 @@ __global__ void k_logtrace_sum(int n, const int64_t* slice_off, const uint8_t* d
 }
 
 // features [N][16] (BF16) and the Cholesky factor of the inverse diagonal block
-__global__ void k_features(int n, const int64_t* slice_off, const uint8_t* diag, const double* v64,
-                           const int32_t* nel_ptr, const int32_t* nel, const double* E, double mean_logtr,
-                           double mean_logE, __nv_bfloat16* feat, float* cfac) {
+// Bound by FP64 arithmetic; with eight logarithms a node 498 us at 1.6 M DOF, 297 now.
+__global__ void k_features(int n, DiagView A, const int32_t* nel_ptr, const int32_t* nel, const double* log_E,
+                           double mean_logtr, __nv_bfloat16* feat, float* cfac) {
     const int row = blockIdx.x * blockDim.x + threadIdx.x;
     if (row >= n) return;
     double m[9];
-    diag_block(slice_off, diag, v64, row, m);
+    diag_block(A, row, m);
     const double tr = (m[0] + m[4] + m[8]) / 3.0;
     float f[kF];
     f[0] = (float)(m[0] / tr);
@@ -108,7 +127,7 @@ __global__ void k_features(int n, const int64_t* slice_off, const uint8_t* diag,
     double s = 0.0, s2 = 0.0, lo = 1e300, hi = -1e300;
     const int b = nel_ptr[row], e = nel_ptr[row + 1];
     for (int k = b; k < e; ++k) {
-        const double le = log(E[nel[k]]) - mean_logE;
+        const double le = log_E[nel[k]];
         s += le;
         s2 += le * le;
         lo = fmin(lo, le);
@@ -684,7 +703,7 @@ int learned_n_outputs() { return kO; }
 
 // features for the current assembly
 void learned_features(Ctx& c) {
-    ensure_v64(c);
+    c.diag64 = true;
     ensure_buffers(c);
     LearnedState& L = state(c);
     if (L.feat_epoch == c.assembly_epoch) return;
@@ -693,13 +712,15 @@ void learned_features(Ctx& c) {
     for (double e : c.E) mean_logE += std::log(e);
     mean_logE /= std::max<size_t>(1, c.E.size());
     L.part.zero(c.stream);
-    k_logtrace_sum<<<256, 256, 0, c.stream>>>(n, c.A.slice_off.p, c.A.diag.p, c.A.v64.p, L.part.p);
+    const DiagView A{c.A.slice_off.p, c.A.diag.p, c.v64_valid ? c.A.v64.p : nullptr, c.A.v32.p, c.A.v32lo.p};
+    if (L.log_E.n < (size_t)c.n_el) L.log_E.alloc((size_t)c.n_el);
+    k_logtrace_sum<<<256, 256, 0, c.stream>>>(n, A, L.part.p);
     double s = 0.0;
     ASEND_CUDA(cudaMemcpyAsync(&s, L.part.p, sizeof(double), cudaMemcpyDeviceToHost, c.stream));
+    k_log_modulus<<<lgrid(c.n_el), kLT, 0, c.stream>>>(c.n_el, c.d_E.p, mean_logE, L.log_E.p);
     ASEND_CUDA(cudaStreamSynchronize(c.stream));
-    k_features<<<lgrid(n), kLT, 0, c.stream>>>(n, c.A.slice_off.p, c.A.diag.p, c.A.v64.p, L.nel_ptr.p, L.nel.p,
-                                               c.d_E.p, s / n, mean_logE, L.feat.p, L.cfac.p);
-    c.launches += 2;
+    k_features<<<lgrid(n), kLT, 0, c.stream>>>(n, A, L.nel_ptr.p, L.nel.p, L.log_E.p, s / n, L.feat.p, L.cfac.p);
+    c.launches += 3;
     L.feat_epoch = c.assembly_epoch;
 }
 

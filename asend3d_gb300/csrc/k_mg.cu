@@ -80,8 +80,6 @@ struct MgLevel {
     DArr<float> d_w;
     Sbell own;                    // pattern + FP32 values (levels >= 1)
     Sbell* A = nullptr;
-    std::vector<int32_t> colour_ptr;
-    DArr<int32_t> colour_elems, slot_map, conn;
     DArr<float> Ke;               // Galerkin element matrices [n_el][24][24]
     std::vector<float> h_pen;     // lumped penalty per DOF (in units of sf)
     DArr<float> pen;
@@ -162,6 +160,9 @@ void launch_k(const Ctx& c, void (*k)(KArgs...), dim3 grid, int block, size_t sm
     cfg.numAttrs = 1;
     ASEND_CUDA(cudaLaunchKernelEx(&cfg, k, std::forward<Args>(args)...));
 }
+// Levels with at least this many node rows run the staged (bulk-copy) row
+// products, one row per lane; smaller ones split each row over T lanes.
+constexpr int kStagedRows = 8192;
 // classes up to which the first coarsening uses projected class matrices
 // (27 x 576 floats each, 62 KB)
 constexpr int kMaxChildClasses = 512;
@@ -194,20 +195,25 @@ __device__ __forceinline__ int find_blk(const int32_t* __restrict__ pre, int n_b
 // ---------------------------------------------------------------------------
 // Galerkin coarsening by elements
 // ---------------------------------------------------------------------------
-// One CTA (512 threads) per coarse element C of level l.  Its <= 8 children
-// (elements of level l-1) are processed together: each child's FP32 stiffness
-// comes from the stored Galerkin matrices of level l-1, or for l = 1 is
-// integrated here from the fine geometry (2x2x2 Gauss points, closed-form
-// isotropic blocks as in the assembly kernel); then T_e = K_e (Q_e x I3) and
-// K_C = sum_e (Q_e x I3)^T T_e.
-__global__ void __launch_bounds__(512)
+// One CTA per coarse element C of level l.  Its <= 8 children (elements of level
+// l-1) are processed together: each child's FP32 stiffness comes from the
+// stored Galerkin matrices of level l-1, or for l = 1 is integrated here from
+// the fine geometry (2x2x2 Gauss points, closed-form isotropic blocks as in
+// the assembly kernel); then T_e = K_e (Q_e x I3) and
+// K_C = sum_e (Q_e x I3)^T T_e.  A thread holds the eight entries of K_e that
+// share its (child, row, component) in registers and forms their eight columns of
+// T_e, then four rows of a column of K_C, so that an operand in shared
+// memory serves 4 to 8 FMAs; one entry a thread (two loads an FMA) was bound by
+// those loads: 750 us over the levels of 128 x 64 x 64 elements, now 304.
+constexpr int kCoarsenThreads = 576;
+constexpr int kTLd = 27;  // row stride of T (24 columns): lanes of 11 rows on different banks
+__global__ void __launch_bounds__(kCoarsenThreads)
 k_coarsen(LevelView cv, const int32_t* __restrict__ pre_el, const float* __restrict__ fine_ke,
           const float* __restrict__ cls_ke, const int32_t* __restrict__ cls_of, const double* __restrict__ xyz,
           const int32_t* __restrict__ conn0, const double* __restrict__ E, const double* __restrict__ nu,
           float* __restrict__ coarse_ke) {
-    __shared__ float Ke[8][576];
-    __shared__ float T[8][576];
-    __shared__ float Q[8][8][8];
+    __shared__ float Ke[8][24 * kTLd];  // the integrated K_e, then T_e
+    __shared__ __align__(16) float Q[8][8][8];
     __shared__ float g[8][8][8][3];
     __shared__ float wdet[8][8];
     __shared__ float xl[8][8][3];
@@ -232,14 +238,7 @@ k_coarsen(LevelView cv, const int32_t* __restrict__ pre_el, const float* __restr
         if (a == 0 && b == 0) fe[ch] = d.fel0 + ((s0 + o0) * d.fny + (s1 + o1)) * d.fnz + (s2 + o2);
     }
     __syncthreads();
-    if (cls_ke) {  // K_e = E_e * (unit-modulus matrix of the element's geometry class)
-        for (int q = t; q < nch * 576; q += blockDim.x) {
-            const int e = fe[q / 576];
-            Ke[q / 576][q % 576] = (float)E[e] * cls_ke[(size_t)cls_of[e] * 576 + q % 576];
-        }
-    } else if (fine_ke) {
-        for (int q = t; q < nch * 576; q += blockDim.x) Ke[q / 576][q % 576] = fine_ke[(size_t)fe[q / 576] * 576 + q % 576];
-    } else {
+    if (!cls_ke && !fine_ke) {
         if (t < nch * 24) {
             const int ch = t / 24, a = (t / 3) % 8, j = t % 3;
             const int e = fe[ch];
@@ -296,28 +295,59 @@ k_coarsen(LevelView cv, const int32_t* __restrict__ pre_el, const float* __restr
             const float tr = mu * (S[0][0] + S[1][1] + S[2][2]);
             for (int i = 0; i < 3; ++i)
                 for (int j = 0; j < 3; ++j)
-                    Ke[ch][(3 * a + i) * 24 + 3 * b + j] = lam * S[i][j] + mu * S[j][i] + ((i == j) ? tr : 0.f);
+                    Ke[ch][(3 * a + i) * kTLd + 3 * b + j] = lam * S[i][j] + mu * S[j][i] + ((i == j) ? tr : 0.f);
         }
     }
     __syncthreads();
-    // T_ch = K_ch (Q_ch x I3)
-    for (int q = t; q < nch * 576; q += blockDim.x) {
-        const int ch = q / 576, r = q % 576, row = r / 24, col = r % 24, b = col / 3, c2 = col % 3;
-        float acc = 0.f;
+    // T_ch = K_ch (Q_ch x I3): this thread's entries (row, 3 a2 + c2) of child ch
+    const int ch = t / 72, row = t % 72 / 3, c2 = t % 3;
+    float kv[8];
+    if (ch < nch) {
+        if (cls_ke) {  // K_e = E_e * (unit-modulus matrix of the element's geometry class)
+            const float Ee = (float)E[fe[ch]];
+            const float* src = cls_ke + (size_t)cls_of[fe[ch]] * 576 + row * 24 + c2;
 #pragma unroll
-        for (int a2 = 0; a2 < 8; ++a2) acc = fmaf(Ke[ch][row * 24 + 3 * a2 + c2], Q[ch][a2][b], acc);
-        T[ch][r] = acc;
+            for (int a2 = 0; a2 < 8; ++a2) kv[a2] = Ee * src[3 * a2];
+        } else if (fine_ke) {
+            const float* src = fine_ke + (size_t)fe[ch] * 576 + row * 24 + c2;
+#pragma unroll
+            for (int a2 = 0; a2 < 8; ++a2) kv[a2] = src[3 * a2];
+        } else {
+#pragma unroll
+            for (int a2 = 0; a2 < 8; ++a2) kv[a2] = Ke[ch][row * kTLd + 3 * a2 + c2];
+        }
+    }
+    __syncthreads();  // K_e is read
+    if (ch < nch) {
+        float acc[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
+#pragma unroll
+        for (int a2 = 0; a2 < 8; ++a2) {
+            const float4 q0 = *reinterpret_cast<const float4*>(Q[ch][a2]);
+            const float4 q1 = *reinterpret_cast<const float4*>(Q[ch][a2] + 4);
+            const float qv[8] = {q0.x, q0.y, q0.z, q0.w, q1.x, q1.y, q1.z, q1.w};
+#pragma unroll
+            for (int b = 0; b < 8; ++b) acc[b] = fmaf(kv[a2], qv[b], acc[b]);
+        }
+#pragma unroll
+        for (int b = 0; b < 8; ++b) Ke[ch][row * kTLd + 3 * b + c2] = acc[b];
     }
     __syncthreads();
-    // K_C = sum_ch (Q_ch x I3)^T T_ch
-    for (int q = t; q < 576; q += blockDim.x) {
-        const int row = q / 24, col = q % 24, b = row / 3, c1 = row % 3;
-        float acc = 0.f;
-        for (int ch = 0; ch < nch; ++ch)
+    // K_C = sum_ch (Q_ch x I3)^T T_ch: rows 3 b + c1, b = b0 .. b0 + 3, of column col
+    if (t >= 144) return;
+    const int b0 = t / 72 * 4, c1 = t % 72 / 24, col = t % 24;
+    float acc[4] = {0.f, 0.f, 0.f, 0.f};
+    for (int h = 0; h < nch; ++h)
 #pragma unroll
-            for (int a = 0; a < 8; ++a) acc = fmaf(Q[ch][a][b], T[ch][(3 * a + c1) * 24 + col], acc);
-        coarse_ke[(size_t)C * 576 + q] = acc;
-    }
+        for (int a = 0; a < 8; ++a) {
+            const float4 qv = *reinterpret_cast<const float4*>(Q[h][a] + b0);
+            const float tv = Ke[h][(3 * a + c1) * kTLd + col];
+            acc[0] = fmaf(qv.x, tv, acc[0]);
+            acc[1] = fmaf(qv.y, tv, acc[1]);
+            acc[2] = fmaf(qv.z, tv, acc[2]);
+            acc[3] = fmaf(qv.w, tv, acc[3]);
+        }
+#pragma unroll
+    for (int b = 0; b < 4; ++b) coarse_ke[(size_t)C * 576 + (3 * (b0 + b) + c1) * 24 + col] = acc[b];
 }
 
 // First coarsening of a level-0 block made of geometry classes: with
@@ -404,49 +434,10 @@ __global__ void __launch_bounds__(144) k_coarsen_lin(LevelView cv, const int32_t
     reinterpret_cast<float4*>(coarse_ke + (size_t)C * 576)[t] = acc;
 }
 
-// Coloured scatter of stored element matrices into a level's FP32 values.
-__global__ void k_scatter_ke(int n, const int32_t* __restrict__ elems, const int32_t* __restrict__ slot_map,
-                             const float* __restrict__ ke, float* __restrict__ vals) {
-    const int t = blockIdx.x * blockDim.x + threadIdx.x;
-    if (t >= n * 64) return;
-    const int e = elems[t >> 6], pr = t & 63, a = pr >> 3, b = pr & 7;
-    const int32_t slot = slot_map[(size_t)e * 64 + pr];
-    const int64_t g = slot >> 5, lane = slot & 31;
-    float* vb = vals + (g * 9) * 32 + lane;
-    const float* K = ke + (size_t)e * 576;
-#pragma unroll
-    for (int i = 0; i < 3; ++i)
-#pragma unroll
-        for (int j = 0; j < 3; ++j) vb[(i * 3 + j) * 32] += K[(3 * a + i) * 24 + 3 * b + j];
-}
-
-// Lumped penalty of a coarse level, scaled by the penalty scale of the
-// node's block (instance).
-__global__ void k_add_pen(int n_rows, const int64_t* __restrict__ slice_off, const uint8_t* __restrict__ diag,
-                          const float* __restrict__ pen, const int32_t* __restrict__ pre_node, int n_blk,
-                          const double* __restrict__ blk_sf, float* __restrict__ vals) {
-    const int row = blockIdx.x * blockDim.x + threadIdx.x;
-    if (row >= n_rows) return;
-    const float sf = (float)blk_sf[find_blk(pre_node, n_blk, row)];
-    const int64_t g = slice_off[row >> 5] + diag[row];
-    const int lane = row & 31;
-#pragma unroll
-    for (int a = 0; a < 3; ++a) vals[(g * 9 + a * 4) * 32 + lane] += sf * pen[3 * row + a];
-}
-
-template <typename TV>
-__global__ void k_smoother_blocks(int n_rows, const int64_t* __restrict__ slice_off, const uint8_t* __restrict__ diag,
-                                  const TV* __restrict__ vals, float omega, float* __restrict__ binv) {
-    const int row = blockIdx.x * blockDim.x + threadIdx.x;
-    if (row >= n_rows) return;
-    const int64_t g = slice_off[row >> 5] + diag[row];
-    const int lane = row & 31;
-    double m[9];
-#pragma unroll
-    for (int q = 0; q < 9; ++q) m[q] = (double)vals[(g * 9 + q) * 32 + lane];
+// binv := omega m^-1 (cofactors in FP64)
+__device__ __forceinline__ void smoother_block(const double (&m)[9], float omega, float* B) {
     const double c00 = m[4] * m[8] - m[5] * m[7], c01 = m[5] * m[6] - m[3] * m[8], c02 = m[3] * m[7] - m[4] * m[6];
     const double id = omega / (m[0] * c00 + m[1] * c01 + m[2] * c02);
-    float* B = binv + 9 * (size_t)row;
     B[0] = (float)(c00 * id);
     B[1] = (float)((m[2] * m[7] - m[1] * m[8]) * id);
     B[2] = (float)((m[1] * m[5] - m[2] * m[4]) * id);
@@ -456,6 +447,142 @@ __global__ void k_smoother_blocks(int n_rows, const int64_t* __restrict__ slice_
     B[6] = (float)(c02 * id);
     B[7] = (float)((m[1] * m[6] - m[0] * m[7]) * id);
     B[8] = (float)((m[0] * m[4] - m[1] * m[3]) * id);
+}
+
+// lo: a split-only assembly whose FP64 diagonal blocks were asked for (nullptr:
+// the values as they are)
+template <typename TV>
+__global__ void k_smoother_blocks(int n_rows, const int64_t* __restrict__ slice_off, const uint8_t* __restrict__ diag,
+                                  const TV* __restrict__ vals, const float* __restrict__ lo, float* __restrict__ binv) {
+    const int row = blockIdx.x * blockDim.x + threadIdx.x;
+    if (row >= n_rows) return;
+    const int64_t g = slice_off[row >> 5] + diag[row];
+    const int lane = row & 31;
+    double m[9];
+#pragma unroll
+    for (int q = 0; q < 9; ++q)
+        m[q] = (double)vals[(g * 9 + q) * 32 + lane] + (lo ? (double)lo[(g * 9 + q) * 32 + lane] : 0.0);
+    smoother_block(m, 1.f, binv + 9 * (size_t)row);
+}
+
+// A coarse level's values from its element matrices, one CTA per slice of 32
+// rows: every row sums its <= 8 elements' three matrix rows (72 consecutive
+// floats each, one warp a row, all of a row's loads in flight) in shared memory
+// in the order of the elements' parities, adds the lumped penalty (scaled by
+// the block's penalty scale), and the slice is written once, with its smoother
+// blocks D^-1 and the bound ||D^-1 A||_inf >= lambda_max (float bits under
+// atomicMax).  Each element matrix is read once and each value written once, so
+// the kernel is bound by those bytes; eight coloured scatters, the clearing, the
+// penalty, the blocks and the bound as kernels of their own took 1.4 ms over the levels of
+// 128 x 64 x 64 elements, this one 245 us.
+constexpr int kValThreads = 256;
+constexpr int kValLd = 33;
+constexpr size_t kValSmem = sizeof(float) * (27 * 9 * kValLd + 9 * kValLd);
+
+__global__ void __launch_bounds__(kValThreads)
+k_level_values(int n_rows, const BlkDev* __restrict__ blk, const int32_t* __restrict__ row_blk, BlkDev one,
+               const float* __restrict__ ke, const float* __restrict__ pen, const double* __restrict__ blk_sf,
+               float* __restrict__ vals, float* __restrict__ binv, unsigned int* __restrict__ bound_bits) {
+    extern __shared__ __align__(16) float vsm[];
+    float* Bs = vsm + 27 * 9 * kValLd;
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    for (int q = threadIdx.x; q < 27 * 9 * kValLd; q += kValThreads) vsm[q] = 0.f;
+    __syncthreads();
+    // this lane's entries of an element's three rows: (i, column corner b, j)
+    int vo[3], co[3][3];
+#pragma unroll
+    for (int w = 0; w < 3; ++w) {
+        const int s = min(lane + 32 * w, 71), b = s % 24 / 3;
+        vo[w] = s / 24 * 3 + s % 3;
+#pragma unroll
+        for (int ax = 0; ax < 3; ++ax) co[w][ax] = c_corner[b][ax];
+    }
+    for (int q = warp; q < 32; q += kValThreads / 32) {
+        const int row = blockIdx.x * 32 + q;
+        if (row >= n_rows) break;
+        const int b = row_blk ? row_blk[row] : 0;
+        const BlkDev d = row_blk ? blk[b] : one;
+        const int l = row - d.node0, sj = d.nz + 1, si = (d.ny + 1) * sj;
+        if (l >= (d.nx + 1) * si) continue;  // padding node between instances
+        const int i = l / si, j = (l - i * si) / sj, k = l - i * si - j * sj;
+        const int i0 = max(i - 1, 0), j0 = max(j - 1, 0), k0 = max(k - 1, 0);
+        const int nj = min(j + 1, d.ny) - j0 + 1, nk = min(k + 1, d.nz) - k0 + 1;
+        float v[8][3];
+#pragma unroll
+        for (int c = 0; c < 8; ++c) {  // the adjacent element of parity c
+            const int ei = ((i & 1) == (c >> 2)) ? i : i - 1, ej = ((j & 1) == ((c >> 1) & 1)) ? j : j - 1,
+                      ek = ((k & 1) == (c & 1)) ? k : k - 1;
+            const bool in = ei >= 0 && ej >= 0 && ek >= 0 && ei < d.nx && ej < d.ny && ek < d.nz;
+            const int di = i - ei, dj = j - ej, a = 4 * (k - ek) + (dj ? 3 - di : di);
+            const float* K = ke + ((size_t)d.el0 + (ei * d.ny + ej) * d.nz + ek) * 576 + 72 * a;
+#pragma unroll
+            for (int w = 0; w < 3; ++w) v[c][w] = in && lane + 32 * w < 72 ? __ldcs(K + lane + 32 * w) : 0.f;
+        }
+#pragma unroll
+        for (int c = 0; c < 8; ++c) {
+            const int ei = ((i & 1) == (c >> 2)) ? i : i - 1, ej = ((j & 1) == ((c >> 1) & 1)) ? j : j - 1,
+                      ek = ((k & 1) == (c & 1)) ? k : k - 1;
+            if (ei >= 0 && ej >= 0 && ek >= 0 && ei < d.nx && ej < d.ny && ek < d.nz) {  // uniform over the warp
+#pragma unroll
+                for (int w = 0; w < 3; ++w)
+                    if (lane + 32 * w < 72) {
+                        const int at = ((ei + co[w][0] - i0) * nj + (ej + co[w][1] - j0)) * nk + (ek + co[w][2] - k0);
+                        vsm[(at * 9 + vo[w]) * kValLd + q] += v[c][w];
+                    }
+            }
+            __syncwarp();
+        }
+        if (lane < 3) {
+            const int at = ((i - i0) * nj + (j - j0)) * nk + (k - k0);
+            const float sf = (float)blk_sf[b];
+            vsm[(at * 9 + 4 * lane) * kValLd + q] += sf * pen[3 * row + lane];
+        }
+        __syncwarp();
+        if (lane < 9) {  // the diagonal block, for the smoother
+            const int at = ((i - i0) * nj + (j - j0)) * nk + (k - k0);
+            Bs[lane * kValLd + q] = vsm[(at * 9 + lane) * kValLd + q];
+        }
+    }
+    __syncthreads();
+    const int row = blockIdx.x * 32 + lane;
+    float* out = vals + (size_t)blockIdx.x * (27 * 9 * 32);
+    for (int x = warp; x < 27 * 9; x += kValThreads / 32) out[(size_t)x * 32 + lane] = vsm[x * kValLd + lane];
+    bool real = row < n_rows;
+    if (real) {
+        const BlkDev d = row_blk ? blk[row_blk[row]] : one;
+        real = row - d.node0 < (d.nx + 1) * (d.ny + 1) * (d.nz + 1);
+    }
+    if (warp == 0 && row < n_rows) {
+        double m[9];
+#pragma unroll
+        for (int q = 0; q < 9; ++q) m[q] = real ? (double)Bs[q * kValLd + lane] : 0.0;
+        float B[9];
+        smoother_block(m, 1.f, B);
+#pragma unroll
+        for (int q = 0; q < 9; ++q) {
+            Bs[q * kValLd + lane] = B[q];
+            binv[9 * (size_t)row + q] = B[q];
+        }
+    }
+    if (!bound_bits) return;
+    __syncthreads();
+    if (warp >= 3) return;
+    float sum = 0.f;  // component `warp` of the row's sum
+    if (real) {
+        float B[3];
+#pragma unroll
+        for (int q = 0; q < 3; ++q) B[q] = Bs[(3 * warp + q) * kValLd + lane];
+#pragma unroll 3
+        for (int j = 0; j < 27; ++j) {
+            const float* m = vsm + j * 9 * kValLd + lane;
+#pragma unroll
+            for (int b = 0; b < 3; ++b)
+                sum += fabsf(B[0] * m[b * kValLd] + B[1] * m[(3 + b) * kValLd] + B[2] * m[(6 + b) * kValLd]);
+        }
+    }
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) sum = fmaxf(sum, __shfl_xor_sync(0xffffffffu, sum, o));
+    if (lane == 0 && sum > 0.f) atomicMax(bound_bits, __float_as_uint(sum));
 }
 
 // Coarsest level: one dense matrix per block (n_b = 3 x the block's nodes,
@@ -482,161 +609,193 @@ __global__ void k_dense_build(int n_rows, const int64_t* __restrict__ slice_off,
     }
 }
 
-// Coarsest inverse: blocked Gauss-Jordan of one block's matrix (n <= 256, which
+// Coarsest inverse: in-place Gauss-Jordan of one block's matrix (n <= 256, which
 // the coarsening rule guarantees) by a cluster of 8 CTAs, CTA r holding rows
-// 32 r .. 32 r + 31 in shared memory.  For panel P (rows / columns k0 .. k0 +
-// 31) its owner forms D = A_PP^-1 (warp 0, in registers, lane = row) and R = D
-// A_P (R_PP = D); the others copy R through distributed shared memory and set
-// A_i = A_i - A_iP R with the panel columns of A_i cleared first, which is the
-// unblocked in-place elimination regrouped.  No pivoting: the coarse operators
-// are SPD.  Bound by the serial panels; one CTA with the whole matrix took 283
-// us at n = 216, and above 234 (no longer in one CTA's shared memory) 3,460 us
-// column by column in global memory at n = 243.
-__device__ __forceinline__ void gj_panel_inverse(const float* __restrict__ rows, int ld, int k0, int kb, float* __restrict__ D) {
-    const int lane = threadIdx.x & 31;
-    float d[32];
-#pragma unroll
-    for (int j = 0; j < 32; ++j) d[j] = (lane < kb && j < kb) ? rows[lane * ld + k0 + j] : (lane == j ? 1.f : 0.f);
-#pragma unroll
-    for (int p = 0; p < 32; ++p) {
-        const float piv = __shfl_sync(0xffffffffu, d[p], p);
-        const float inv = 1.f / piv;
-        const float cp = d[p];  // this row's entry in column p
-        if (lane == p) {
-#pragma unroll
-            for (int j = 0; j < 32; ++j) d[j] = (j == p) ? inv : d[j] * inv;
-        }
-        // row p (already scaled) from lane p, entry by entry; lane p keeps its row
-#pragma unroll
-        for (int j = 0; j < 32; ++j) {
-            const float rpj = __shfl_sync(0xffffffffu, d[j], p);
-            if (lane != p) d[j] = (j == p) ? -cp * inv : fmaf(-cp, rpj, d[j]);
-        }
-    }
-#pragma unroll
-    for (int j = 0; j < 32; ++j) D[lane * 32 + j] = d[j];
-}
-
+// 32 r .. 32 r + 31 in registers (warp w rows 4 w .. 4 w + 3, lane columns lane +
+// 32 j).  For panel P (rows / columns k0 .. k0 + 31) its owner forms the 32 rows
+// R that eliminate it and writes them to the panel's rows of the matrix in
+// global memory (L2: 8 readers of one SM's shared memory took three times as
+// long); after a cluster barrier the others read them and apply A_i = A_i - A_iP R
+// with the panel columns of A_i cleared first.  No pivoting: the coarse
+// operators are SPD.  Up to 234 DOF R = D A_P with D = A_PP^-1 (the elimination
+// regrouped by panels), above it the owner eliminates column by column and the
+// others follow its steps, each size keeping the rounding of its V-cycles.
+// Bound by the serial panels, 32 pivots of one CTA barrier each; rows in
+// registers and one pass over memory a panel instead of shared memory with
+// 8-way conflicts: n = 216 170 -> 99 us, n = 243 636 -> 126 us.
 constexpr int kGjCtas = 8, kGjN = 256, kGjThreads = 256, kGjBlocked = 234;
-constexpr size_t kGjSmem = sizeof(float) * (2 * 32 * kGjN + 32 * 32);
+constexpr int kGjLd = 33;  // transposed copy: 256 columns of 32 rows
+constexpr size_t kGjSmem = sizeof(float) * (32 * kGjN + kGjN * kGjLd);
 
 __global__ void __cluster_dims__(kGjCtas, 1, 1) __launch_bounds__(kGjThreads)
-k_gauss_jordan(LevelView cv, float* __restrict__ Dall) {
+k_gauss_jordan(LevelView cv, float* Dall) {
     extern __shared__ __align__(16) float gj[];
-    float* A = gj;                  // own 32 rows
-    float* R = gj + 32 * kGjN;      // the panel's rows
-    float* D = gj + 2 * 32 * kGjN;
+    float* R = gj;               // the panel's eliminating rows [32][256]
+    float* S = gj + 32 * kGjN;   // the owner's rows / the transposed copy
     cooperative_groups::cluster_group cl = cooperative_groups::this_cluster();
-    const int r = (int)cl.block_rank(), t = threadIdx.x;
+    const int r = (int)cl.block_rank(), t = threadIdx.x, warp = t >> 5, lane = t & 31;
     const BlkDev& dv = cv.blk[blockIdx.x / kGjCtas];
     const int n = 3 * (dv.nx + 1) * (dv.ny + 1) * (dv.nz + 1);
+    const bool blocked = n <= kGjBlocked;
     float* Ag = Dall + dv.dense0;
-    for (int q = t; q < 32 * kGjN; q += kGjThreads) {
-        const int i = 32 * r + q / kGjN, j = q % kGjN;
-        A[q] = (i < n && j < n) ? Ag[(size_t)i * n + j] : 0.f;
-    }
-    __syncthreads();
-    const int i0 = 4 * (t >> 5), j0 = 8 * (t & 31);  // this thread's 4 x 8 tile of the own rows
-    if (n > kGjBlocked) {
-        // the owner of row k stores it into every CTA's copy, two alternating
-        for (int k = 0; k < n; ++k) {
-            float* row = R + (k & 1) * kGjN;
-            if (r == k >> 5) {
-                const float v = A[(k & 31) * kGjN + t];
+    const int row0 = 32 * r + 4 * warp;
+    float a[4][8];
 #pragma unroll
-                for (int q = 0; q < kGjCtas; ++q) cl.map_shared_rank(row, q)[t] = v;
-            }
-            cl.sync();
-            const float inv = 1.f / row[k];
-            float rk[8];
+    for (int u = 0; u < 4; ++u)
 #pragma unroll
-            for (int w = 0; w < 8; ++w) rk[w] = row[j0 + w] * inv;
-            float ci[4];
-#pragma unroll
-            for (int u = 0; u < 4; ++u) ci[u] = A[(i0 + u) * kGjN + k];
-            __syncthreads();  // every thread has read column k
-#pragma unroll
-            for (int u = 0; u < 4; ++u) {
-                const bool pivot = 32 * r + i0 + u == k;
-#pragma unroll
-                for (int w = 0; w < 8; ++w) {
-                    float* e = A + (i0 + u) * kGjN + j0 + w;
-                    if (pivot) *e = j0 + w == k ? inv : rk[w];
-                    else *e = j0 + w == k ? -ci[u] * inv : fmaf(-ci[u], rk[w], *e);
-                }
-            }
-            __syncthreads();
+        for (int j = 0; j < 8; ++j) {
+            const int i = row0 + u, q = lane + 32 * j;
+            a[u][j] = (i < n && q < n) ? Ag[(size_t)i * n + q] : 0.f;
         }
-    }
-    for (int P = 0; n <= kGjBlocked && 32 * P < n; ++P) {
+    cl.sync();  // loaded: the panels' rows in global memory may be written
+    for (int P = 0; 32 * P < n; ++P) {
         const int k0 = 32 * P, kb = min(32, n - k0);
+        float pc[4];  // the panel's columns of the own rows
+#pragma unroll
+        for (int u = 0; u < 4; ++u) {
+            pc[u] = 0.f;
+#pragma unroll
+            for (int j = 0; j < 8; ++j)
+                if (j == P) pc[u] = a[u][j];
+        }
         if (r == P) {
-            if (t < 32) gj_panel_inverse(A, kGjN, k0, kb, D);
-            __syncthreads();
-            float a[32];
+            if (blocked) {
+                // A_PP (its padding the identity) inverted in pc; rows exchanged
+                // through R
 #pragma unroll
-            for (int q = 0; q < 32; ++q) a[q] = A[q * kGjN + t];
-            const bool in_p = t >= k0 && t < k0 + 32;
-#pragma unroll 4
-            for (int p = 0; p < 32; ++p) {
-                float s = 0.f;
-#pragma unroll
-                for (int q = 0; q < 32; ++q) s = fmaf(D[p * 32 + q], a[q], s);
-                R[p * kGjN + t] = in_p ? D[p * 32 + t - k0] : s;
+                for (int u = 0; u < 4; ++u)
+                    if (4 * warp + u >= kb || lane >= kb) pc[u] = 4 * warp + u == lane ? 1.f : 0.f;
             }
-        }
-        cl.sync();  // R is complete
-        if (r != P) {
-            const float4* src = reinterpret_cast<const float4*>(cl.map_shared_rank(R, P));
-#pragma unroll
-            for (int q = 0; q < 32 * kGjN / 4 / kGjThreads; ++q)
-                reinterpret_cast<float4*>(R)[q * kGjThreads + t] = src[q * kGjThreads + t];
-        }
-        cl.sync();  // copied: the owner's R may be overwritten with the next panel's
-        float acc[4][8];
-        if (r == P) {
-#pragma unroll
-            for (int u = 0; u < 4; ++u)
-#pragma unroll
-                for (int w = 0; w < 8; ++w) acc[u][w] = R[(i0 + u) * kGjN + j0 + w];
-        } else {
-#pragma unroll
-            for (int u = 0; u < 4; ++u)
-#pragma unroll
-                for (int w = 0; w < 8; ++w)
-                    acc[u][w] = (j0 + w >= k0 && j0 + w < k0 + 32) ? 0.f : A[(i0 + u) * kGjN + j0 + w];
-#pragma unroll 4
-            for (int q = 0; q < 32; ++q) {
-                const float4 r0 = *reinterpret_cast<const float4*>(R + q * kGjN + j0);
-                const float4 r1 = *reinterpret_cast<const float4*>(R + q * kGjN + j0 + 4);
-                const float rv[8] = {r0.x, r0.y, r0.z, r0.w, r1.x, r1.y, r1.z, r1.w};
+            for (int w = 0; 4 * w < kb; ++w) {
 #pragma unroll
                 for (int u = 0; u < 4; ++u) {
-                    const float av = A[(i0 + u) * kGjN + k0 + q];
+                    const int p = 4 * w + u;
+                    if (p >= kb) break;
+                    float* row = R + p * kGjN;
+                    if (warp == w) {
+                        const float inv = 1.f / __shfl_sync(0xffffffffu, pc[u], p);
+                        const float pm = lane == p ? inv : pc[u] * inv;
+                        if (!blocked) {
 #pragma unroll
-                    for (int w = 0; w < 8; ++w) acc[u][w] = fmaf(-av, rv[w], acc[u][w]);
+                            for (int j = 0; j < 8; ++j) row[lane + 32 * j] = j == P ? pm : a[u][j] * inv;
+                        } else {
+                            row[lane] = pm;
+                        }
+                    }
+                    __syncthreads();
+                    const float pm = row[blocked ? lane : k0 + lane];
+                    float ci[4];
+#pragma unroll
+                    for (int v = 0; v < 4; ++v) {
+                        ci[v] = __shfl_sync(0xffffffffu, pc[v], p);
+                        pc[v] = fmaf(-ci[v], pm, lane == p ? 0.f : pc[v]);
+                        if (v == u && warp == w) pc[v] = pm;
+                    }
+                    if (!blocked) {
+#pragma unroll
+                        for (int j = 0; j < 8; ++j) {
+                            const float m = row[lane + 32 * j];
+#pragma unroll
+                            for (int v = 0; v < 4; ++v)
+                                a[v][j] = (v == u && warp == w) ? m : fmaf(-ci[v], m, a[v][j]);
+                        }
+                    }
                 }
             }
+            if (blocked) {  // R = D A_P, R_PP = D
+#pragma unroll
+                for (int u = 0; u < 4; ++u)
+#pragma unroll
+                    for (int j = 0; j < 8; ++j) S[(4 * warp + u) * kGjN + lane + 32 * j] = a[u][j], a[u][j] = 0.f;
+                __syncthreads();
+#pragma unroll 4
+                for (int q = 0; q < 32; ++q) {
+                    float d[4];
+#pragma unroll
+                    for (int u = 0; u < 4; ++u) d[u] = __shfl_sync(0xffffffffu, pc[u], q);
+#pragma unroll
+                    for (int j = 0; j < 8; ++j) {
+                        const float m = S[q * kGjN + lane + 32 * j];
+#pragma unroll
+                        for (int u = 0; u < 4; ++u) a[u][j] = fmaf(d[u], m, a[u][j]);
+                    }
+                }
+            }
+#pragma unroll
+            for (int u = 0; u < 4; ++u)
+#pragma unroll
+                for (int j = 0; j < 8; ++j) {
+                    if (j == P) a[u][j] = pc[u];
+                    const int i = row0 + u, q = lane + 32 * j;
+                    // unblocked: the rows as they eliminated, not as they ended
+                    if (i < n && q < n) Ag[(size_t)i * n + q] = blocked ? a[u][j] : R[(4 * warp + u) * kGjN + q];
+                }
         }
-        __syncthreads();  // every thread has read the panel columns of A
+        cl.sync();  // R is in global memory
+        if (r == P) continue;
+        if (t < n) {
+#pragma unroll 16
+            for (int q = 0; q < 32; ++q) R[q * kGjN + t] = q < kb ? __ldcg(Ag + (size_t)(k0 + q) * n + t) : 0.f;
+        } else {
+#pragma unroll 16
+            for (int q = 0; q < 32; ++q) R[q * kGjN + t] = 0.f;
+        }
+        __syncthreads();
 #pragma unroll
         for (int u = 0; u < 4; ++u)
 #pragma unroll
-            for (int w = 0; w < 8; ++w) A[(i0 + u) * kGjN + j0 + w] = acc[u][w];
-        __syncthreads();
+            for (int j = 0; j < 8; ++j)
+                if (j == P) a[u][j] = 0.f;
+#pragma unroll 4
+        for (int q = 0; q < 32; ++q) {
+            if (!blocked && q >= kb) break;
+            float ci[4];
+#pragma unroll
+            for (int u = 0; u < 4; ++u) ci[u] = __shfl_sync(0xffffffffu, pc[u], q);
+#pragma unroll
+            for (int j = 0; j < 8; ++j) {
+                const float m = R[q * kGjN + lane + 32 * j];
+#pragma unroll
+                for (int u = 0; u < 4; ++u) a[u][j] = fmaf(-ci[u], m, a[u][j]);
+            }
+            if (!blocked) {
+                const float m = R[q * kGjN + k0 + lane];
+#pragma unroll
+                for (int u = 0; u < 4; ++u) pc[u] = fmaf(-ci[u], m, lane == q ? 0.f : pc[u]);
+            }
+        }
+        if (!blocked) {
+#pragma unroll
+            for (int u = 0; u < 4; ++u)
+#pragma unroll
+                for (int j = 0; j < 8; ++j)
+                    if (j == P) a[u][j] = pc[u];
+        }
+        __syncthreads();  // R is read
     }
     // the exact inverse is symmetric: average the FP32 rounding asymmetry out,
     // so the coarse solve (and with it the V-cycle) is a symmetric operator
+    cl.sync();  // every panel's rows are read
+#pragma unroll
+    for (int u = 0; u < 4; ++u)
+#pragma unroll
+        for (int j = 0; j < 8; ++j) {
+            const int i = row0 + u, q = lane + 32 * j;
+            if (i < n && q < n) Ag[(size_t)i * n + q] = a[u][j];
+        }
     cl.sync();
-    for (int q = t; q < 32 * kGjN; q += kGjThreads) {
-        const int i = 32 * r + q / kGjN, j = q % kGjN;
-        if (i >= n || j >= n || j < i) continue;
-        const float* other = cl.map_shared_rank(A, j >> 5);
-        const float v = 0.5f * (A[q] + other[(j & 31) * kGjN + i]);
-        Ag[(size_t)i * n + j] = v;
-        Ag[(size_t)j * n + i] = v;
+    if (32 * r + lane < n) {
+#pragma unroll 16
+        for (int q = warp; q < n; q += 8) S[q * kGjLd + lane] = __ldcg(Ag + (size_t)q * n + 32 * r + lane);
     }
-    cl.sync();  // the other CTAs may still read this one's rows
+    cl.sync();  // the transposed columns are read
+#pragma unroll
+    for (int u = 0; u < 4; ++u)
+#pragma unroll
+        for (int j = 0; j < 8; ++j) {
+            const int i = row0 + u, q = lane + 32 * j;
+            if (i < n && q < n) Ag[(size_t)i * n + q] = 0.5f * (a[u][j] + S[q * kGjLd + 4 * warp + u]);
+        }
 }
 
 // ---------------------------------------------------------------------------
@@ -1177,6 +1336,74 @@ __global__ void __launch_bounds__(kT) k_pow_step(SbView A, const float* __restri
         const float z2 = inv * (B[6] * y[0] + B[7] * y[1] + B[8] * y[2]);
         y4[row] = make_float4(z0, z1, z2, 0.f);
         acc[0] = (double)z0 * z0 + (double)z1 * z1 + (double)z2 * z2;
+    }
+    block_sum<1>(acc, sm);
+    if (threadIdx.x == 0) {
+        part[blockIdx.x] = acc[0];
+        __threadfence();
+        last = atomicAdd(ticket + k, 1u) == gridDim.x - 1;
+    }
+    __syncthreads();
+    if (!last) return;
+    __threadfence();
+    double s[1] = {0.0};
+#pragma unroll 4
+    for (int b = threadIdx.x; b < (int)gridDim.x; b += blockDim.x) s[0] += __ldcg(part + b);
+    block_sum<1>(s, sm);
+    if (threadIdx.x == 0) nrm[k + 1] = (float)sqrt(s[0]);
+}
+
+// The same step on a coarse level, four lanes a row (a component of the product
+// each, nine columns in flight; the fourth repeats the third's loads): one
+// thread a row left a level of 6,171 rows on 49 CTAs with nine dependent rounds
+// of loads, 13.8 us; now 8.3 (of
+// which the sums in FP64 and the last CTA's part are the most).  Each component's sum is k_pow_step's.
+__global__ void __launch_bounds__(kT) k_pow_rows(GeoView G, const float* __restrict__ dinv, const float4* __restrict__ x,
+                                                 float4* __restrict__ y4, float* __restrict__ nrm, int k,
+                                                 double* __restrict__ part, uint32_t* __restrict__ ticket) {
+    __shared__ double sm[32];
+    __shared__ bool last;
+    const int gt = blockIdx.x * blockDim.x + threadIdx.x;
+    const bool ok = (gt >> 2) < G.n_rows;
+    const int row = ok ? gt >> 2 : 0, comp = min(gt & 3, 2);
+    const float inv = 1.f / nrm[k];
+    const BlkDev d = blk_of(G, row);
+    const int l = row - d.node0, sj = d.nz + 1, si = (d.ny + 1) * sj;
+    const int i = l / si, j = (l - i * si) / sj, kk = l - i * si - j * sj;
+    const int i0 = max(i - 1, 0), j0 = max(j - 1, 0), k0 = max(kk - 1, 0);
+    // padding between instances (i > nx): no columns
+    const int ni = i <= d.nx ? min(i + 1, d.nx) - i0 + 1 : 0;
+    const int nj = min(j + 1, d.ny) - j0 + 1, nk = min(kk + 1, d.nz) - k0 + 1;
+    x += d.node0 + i0 * si + j0 * sj + k0;
+    const float* v = G.v + (size_t)(row >> 5) * (27 * 9 * 32) + comp * 96 + (row & 31);
+    const float B[3] = {dinv[9 * (size_t)row + 3 * comp], dinv[9 * (size_t)row + 3 * comp + 1],
+                        dinv[9 * (size_t)row + 3 * comp + 2]};
+    float y = 0.f;
+#pragma unroll
+    for (int a = 0; a < 3; ++a) {
+        float m[9][3];
+        float4 p[9];
+#pragma unroll
+        for (int u = 0; u < 9; ++u)
+            if (a < ni && u / 3 < nj && u % 3 < nk) {
+                p[u] = x[a * si + (u / 3) * sj + u % 3];
+#pragma unroll
+                for (int w = 0; w < 3; ++w) m[u][w] = v[((a * nj + u / 3) * nk + u % 3) * 288 + w * 32];
+            }
+#pragma unroll
+        for (int u = 0; u < 9; ++u)
+            if (a < ni && u / 3 < nj && u % 3 < nk)
+                y = fmaf(m[u][0], p[u].x, fmaf(m[u][1], p[u].y, fmaf(m[u][2], p[u].z, y)));
+    }
+    const int quad = threadIdx.x & 28;
+    const float a0 = __shfl_sync(0xffffffffu, y, quad), a1 = __shfl_sync(0xffffffffu, y, quad + 1),
+                a2 = __shfl_sync(0xffffffffu, y, quad + 2);
+    const float z = inv * (B[0] * a0 + B[1] * a1 + B[2] * a2);
+    const float z1 = __shfl_sync(0xffffffffu, z, quad + 1), z2 = __shfl_sync(0xffffffffu, z, quad + 2);
+    double acc[1] = {0.0};
+    if (ok) {
+        reinterpret_cast<float*>(y4 + row)[gt & 3] = (gt & 3) == 3 ? 0.f : z;
+        if ((gt & 3) == 0) acc[0] = (double)z * z + (double)z1 * z1 + (double)z2 * z2;
     }
     block_sum<1>(acc, sm);
     if (threadIdx.x == 0) {
@@ -2123,44 +2350,11 @@ void level_pattern(Ctx& c, MgLevel& L) {
             if (j < (int64_t)adj[r].size() && adj[r][j] == r) A.h_diag[r] = (uint8_t)j;
         }
     }
-    // elements, slot map, parity colouring
-    std::vector<int32_t> conn((size_t)L.n_el * 8), slot((size_t)L.n_el * 64);
-    const int co[8][3] = {{0, 0, 0}, {1, 0, 0}, {1, 1, 0}, {0, 1, 0}, {0, 0, 1}, {1, 0, 1}, {1, 1, 1}, {0, 1, 1}};
-    std::vector<std::vector<int32_t>> colour(8);
-    for (const MgBlk& B : L.blk) {
-        auto id = [&](int i, int j, int k) { return B.node0 + (i * (B.ny + 1) + j) * (B.nz + 1) + k; };
-        for (int i = 0; i < B.nx; ++i)
-            for (int j = 0; j < B.ny; ++j)
-                for (int k = 0; k < B.nz; ++k) {
-                    const int e = B.el0 + (i * B.ny + j) * B.nz + k;
-                    for (int a = 0; a < 8; ++a)
-                        conn[(size_t)e * 8 + a] = id(i + co[a][0], j + co[a][1], k + co[a][2]);
-                    for (int a = 0; a < 8; ++a) {
-                        const int ra = conn[(size_t)e * 8 + a];
-                        for (int b = 0; b < 8; ++b) {
-                            const int cb = conn[(size_t)e * 8 + b];
-                            const auto& v = adj[ra];
-                            const int p = (int)(std::lower_bound(v.begin(), v.end(), cb) - v.begin());
-                            slot[(size_t)e * 64 + a * 8 + b] = (int32_t)A.slot(ra, p);
-                        }
-                    }
-                    colour[(i & 1) * 4 + (j & 1) * 2 + (k & 1)].push_back(e);
-                }
-    }
-    std::vector<int32_t> ce;
-    L.colour_ptr.assign(1, 0);
-    for (auto& cl : colour) {
-        ce.insert(ce.end(), cl.begin(), cl.end());
-        L.colour_ptr.push_back((int32_t)ce.size());
-    }
     A.slice_off.upload(A.h_slice_off, c.stream);
     A.col.upload(A.h_col, c.stream);
     A.row_len.upload(A.h_row_len, c.stream);
     A.diag.upload(A.h_diag, c.stream);
     A.v32.alloc((size_t)A.n_groups * 9 * kSlice);
-    L.conn.upload(conn, c.stream);
-    L.slot_map.upload(slot, c.stream);
-    L.colour_elems.upload(ce, c.stream);
     L.A = &L.own;
 }
 
@@ -2439,7 +2633,7 @@ void damp_smoother(Ctx& c, int l) {
     const int steps = warm ? kPowWarmSteps : kPowSteps;
     if (L.pow_vec.n != (size_t)4 * L.n_nodes) L.pow_vec.alloc((size_t)4 * L.n_nodes);
     ASEND_CUDA(cudaMemsetAsync(tk, 0, sizeof(uint32_t) * kPowSteps, c.stream));
-    ASEND_CUDA(cudaMemsetAsync(H.pow_bound.p + l, 0, sizeof(unsigned int), c.stream));
+    if (l == 0) ASEND_CUDA(cudaMemsetAsync(H.pow_bound.p, 0, sizeof(unsigned int), c.stream));
     if (warm)
         ASEND_CUDA(cudaMemcpyAsync(xa, L.pow_vec.p, sizeof(float) * 4 * L.n_nodes, cudaMemcpyDeviceToDevice,
                                    c.stream));
@@ -2447,6 +2641,9 @@ void damp_smoother(Ctx& c, int l) {
     BoxPlan* box = l == 0 ? H.box : nullptr;
     for (int k = 0; k < steps; ++k) {
         if (box) box_power(c, *box, L.binv.p, xa, xb, nrm, k, H.pow_part.p, tk);
+        else if (l > 0 && L.n_nodes < kStagedRows)
+            k_pow_rows<<<grid_of(4 * L.n_nodes), kT, 0, c.stream>>>(geo_of(L, L), L.binv.p, xa, xb, nrm, k,
+                                                                    H.pow_part.p, tk);
         else k_pow_step<<<g, kT, 0, c.stream>>>(sbview(L), L.binv.p, xa, xb, nrm, k, H.pow_part.p, tk);
         std::swap(xa, xb);
     }
@@ -2454,11 +2651,11 @@ void damp_smoother(Ctx& c, int l) {
     L.pow_warm = true;
     L.pow_steps = steps;
     unsigned int* bound = H.pow_bound.p + l;
-    k_inf_bound<<<g, kT, 0, c.stream>>>(sbview(L), L.binv.p, bound);
+    if (l == 0) k_inf_bound<<<g, kT, 0, c.stream>>>(sbview(L), L.binv.p, bound);  // else with the values
     k_scale_blocks<<<(9 * L.n_nodes + 255) / 256, 256, 0, c.stream>>>(L.n_nodes, L.binv.p, nrm, steps, bound,
                                                                        H.safe_damping ? 1 : 0, c.mg_damping,
                                                                        H.pow_omega.p + l);
-    c.launches += steps + 3;
+    c.launches += steps + 2 + (l == 0);
 }
 
 // per-assembly values: Galerkin element matrices, level operators, penalty,
@@ -2468,10 +2665,11 @@ void damp_smoother(Ctx& c, int l) {
 void level0_smoother_blocks(Ctx& c, MgLevel& L0) {
     if (c.v64_valid)
         k_smoother_blocks<double><<<grid_of(L0.n_nodes), kT, 0, c.stream>>>(L0.n_nodes, c.A.slice_off.p, c.A.diag.p,
-                                                                            c.A.v64.p, 1.f, L0.binv.p);
+                                                                            c.A.v64.p, nullptr, L0.binv.p);
     else
         k_smoother_blocks<float><<<grid_of(L0.n_nodes), kT, 0, c.stream>>>(L0.n_nodes, c.A.slice_off.p, c.A.diag.p,
-                                                                           c.A.v32.p, 1.f, L0.binv.p);
+                                                                           c.A.v32.p, c.diag64 ? c.A.v32lo.p : nullptr,
+                                                                           L0.binv.p);
 }
 
 // Per-assembly multigrid values.  skip_l0: the solve takes its finest-level
@@ -2486,7 +2684,10 @@ void setup_values(Ctx& c, bool skip_l0) {
     H.pow_bound.zero(c.stream);
     H.pow_omega.zero(c.stream);
     H.pow_ticket.alloc((size_t)n_lev * kPowSteps);
-    H.pow_part.alloc((size_t)std::max(grid_of(H.L[0]->n_nodes), H.box ? box_ctas(*H.box) : 0));
+    int pow_ctas = std::max(grid_of(H.L[0]->n_nodes), H.box ? box_ctas(*H.box) : 0);
+    for (int l = 1; l < n_lev; ++l)
+        pow_ctas = std::max(pow_ctas, grid_of((H.L[l]->n_nodes < kStagedRows ? 4 : 1) * H.L[l]->n_nodes));
+    H.pow_part.alloc((size_t)pow_ctas);
     {
         std::vector<double> sf(H.n_blk, c.sf);
         if (c.n_inst > 1 && (int)c.sf_inst.size() == H.n_blk) sf = c.sf_inst;
@@ -2529,22 +2730,14 @@ void setup_values(Ctx& c, bool skip_l0) {
             }
             k_coarsen_lin<<<L.n_el, 144, 0, c.stream>>>(view_of(L), L.pre_el.p, c.d_E.p, cls_of, H.child.p, L.Ke.p);
         } else {
-            k_coarsen<<<L.n_el, 512, 0, c.stream>>>(view_of(L), L.pre_el.p, fine_ke, cls_ke, cls_of, c.d_xyz.p,
+            k_coarsen<<<L.n_el, kCoarsenThreads, 0, c.stream>>>(view_of(L), L.pre_el.p, fine_ke, cls_ke, cls_of, c.d_xyz.p,
                                                     c.d_conn.p, c.d_E.p, c.d_nu.p, L.Ke.p);
         }
-        L.own.v32.zero(c.stream);
-        for (size_t k = 0; k + 1 < L.colour_ptr.size(); ++k) {
-            const int n = L.colour_ptr[k + 1] - L.colour_ptr[k];
-            if (!n) continue;
-            k_scatter_ke<<<(n * 64 + 255) / 256, 256, 0, c.stream>>>(n, L.colour_elems.p + L.colour_ptr[k], L.slot_map.p,
-                                                                     L.Ke.p, L.own.v32.p);
-            ++c.launches;
-        }
-        k_add_pen<<<grid_of(L.n_nodes), kT, 0, c.stream>>>(L.n_nodes, L.own.slice_off.p, L.own.diag.p, L.pen.p,
-                                                           L.pre_node.p, (int)L.blk.size(), H.blk_sf.p, L.own.v32.p);
-        k_smoother_blocks<float><<<grid_of(L.n_nodes), kT, 0, c.stream>>>(L.n_nodes, L.own.slice_off.p, L.own.diag.p,
-                                                                          L.own.v32.p, 1.f, L.binv.p);
-        c.launches += 3;
+        const bool lone = L.blk.size() == 1;
+        k_level_values<<<L.own.n_slices, kValThreads, kValSmem, c.stream>>>(
+            L.n_nodes, L.d_blk.p, lone ? nullptr : L.row_blk.p, L.one, L.Ke.p, L.pen.p, H.blk_sf.p, L.own.v32.p,
+            L.binv.p, l + 1 < H.L.size() ? H.pow_bound.p + l : nullptr);
+        c.launches += 2;
         if (l + 1 < H.L.size()) damp_smoother(c, (int)l);  // the coarsest level is solved directly
     }
     MgLevel& Lc = *H.L.back();
@@ -2594,10 +2787,6 @@ int lanes_for(int n_rows) {
     while (t < 16 && (int64_t)n_rows * t < kFill) t *= 2;
     return t;
 }
-
-// Levels with at least this many node rows run the staged (bulk-copy) row
-// products, one row per lane; smaller ones split each row over T lanes.
-constexpr int kStagedRows = 8192;
 
 template <bool POST>
 void launch_rows(Ctx& c, MgLevel& L, int t, const Control* ctl, int nr) {
