@@ -143,7 +143,7 @@ struct Ctx {
     std::shared_ptr<MgHierarchy> mg;
     float mg_damping = 1.5f;  // smoother omega = mg_damping / lambda_max(D^-1 A)
     int product_variant = 0;  // split outer product: ASEND_PRODUCT_* (0 = the default shape)
-    bool mg_tail = true;      // multigrid: fuse the V-cycle's smallest levels into one launch
+    bool mg_tail = true;      // multigrid: the V-cycle's smallest levels as one launch (lone blocks)
     bool time_solves = true;  // record CUDA events around each PCG solve (off inside Newmark runs)
     int64_t dinv_epoch = -1;  // assembly whose point-Jacobi diagonal d_dinv holds
     bool pdl = false;         // multigrid CG: programmatic dependent launch between its kernels

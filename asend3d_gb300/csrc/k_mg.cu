@@ -89,11 +89,38 @@ struct MgLevel {
     int pow_steps = 0;            // steps of the last estimate
 };
 
+// Levels of the V-cycle's fused tail (k_vc_tail)
+constexpr int kTailLevels = 6, kTailThreads = 1024, kTailCtas = 16, kTailSmem = 224 * 1024, kTailRows = 1024;
+constexpr int kTailLd = 249;    // values of a row, 243: 16 lanes x 2 rows on different banks
+constexpr int kTailCols = 28;   // columns of a row and their number
+struct TailView {
+    int n;  // levels, the last one the coarsest
+    struct Level {
+        BlkDev d;
+        const float* v;
+        const float* binv;
+        int n_rows, own;  // rows, rows a CTA
+        // shared memory, in floats
+        int xo, ro;  // the vectors' copies (float4): iterate; residual, then result (the coarsest's xo: b)
+        int so;      // own rows: [own][12] b and smoother block
+        int co;      // own rows' columns, uint16 [own][kTailCols]
+        int po;      // per node, uint16: 8 x first coarse node of its prolongation + axes between two
+        int to;      // own rows' restriction: fine node + 65536 x axis sides that contribute
+        int vo;      // own rows' values [own][kTailLd], or -1: in global memory
+    } L[kTailLevels];
+    const float* b;
+    const float4* x4;
+    float4* y4;
+};
+
 struct MgHierarchy {
     std::vector<std::unique_ptr<MgLevel>> L;
     DArr<float> dense, ainv;      // coarsest operators, one dense block per instance, inverted in place
     int n_coarse = 0;             // largest coarsest block (DOF)
     int n_blk = 1;
+    int tail0 = 0;                // first level of the V-cycle's fused tail (0: no tail)
+    TailView tail;                // its levels
+    int tail_smem = 0;            // bytes
     std::vector<int32_t> h_dense0;  // offset of each block's dense matrix (floats)
     DArr<double> blk_sf;          // penalty scale per block (instance)
     DArr<float> child;            // projected class matrices of the first coarsening [n_cls][27][576]
@@ -1117,10 +1144,10 @@ __device__ __forceinline__ BlkDev blk_of(const GeoView& G, int row) {
     return G.row_blk ? G.blk[G.row_blk[row]] : G.one;
 }
 
-// The share of lane t of T in row `row`'s product; false: no such row.
-template <int T>
-__device__ __forceinline__ void geo_row_part(const GeoView& G, const BlkDev& d, int row, int t,
-                                             const float4* __restrict__ x, float (&y)[3]) {
+// The share of lane t of T in row `row`'s product: v(9 q + w) entry w of its q-th
+// block, x(c) the entry of a column.
+template <int T, typename V, typename X>
+__device__ __forceinline__ void geo_row_part(const BlkDev& d, int row, int t, V&& v, X&& x, float (&y)[3]) {
     const int l = row - d.node0;
     const int sj = d.nz + 1, si = (d.ny + 1) * sj;
     const int i = l / si, j = (l - i * si) / sj, k = l - i * si - j * sj;
@@ -1128,7 +1155,6 @@ __device__ __forceinline__ void geo_row_part(const GeoView& G, const BlkDev& d, 
     const int nj = min(j + 1, d.ny) - j0 + 1, nk = min(k + 1, d.nz) - k0 + 1;
     const int len = (min(i + 1, d.nx) - i0 + 1) * nj * nk;
     const int first = d.node0 + i0 * si + j0 * sj + k0;
-    const float* v = G.v + (size_t)(row >> 5) * (27 * 9 * 32) + (row & 31);
     constexpr int U = (27 + T - 1) / T;
     constexpr int STEP = U < 4 ? U : 4;  // columns in flight
     y[0] = y[1] = y[2] = 0.f;
@@ -1141,9 +1167,9 @@ __device__ __forceinline__ void geo_row_part(const GeoView& G, const BlkDev& d, 
             const int q = t + (u0 + u) * T;
             if (q < len) {
                 const int qk = q / nk, c = first + (qk / nj) * si + (qk % nj) * sj + (q - qk * nk);
-                p[u] = x[c];
+                p[u] = x(c);
 #pragma unroll
-                for (int w = 0; w < 9; ++w) m[u][w] = v[((size_t)q * 9 + w) * 32];
+                for (int w = 0; w < 9; ++w) m[u][w] = v(q * 9 + w);
             }
         }
 #pragma unroll
@@ -1180,7 +1206,10 @@ __global__ void __launch_bounds__(kT) k_vc_rows(GeoView G, const float* __restri
             for (int q = 0; q < 9; ++q) B[q] = binv[9 * (size_t)row + q];
         }
     }
-    if (ok) geo_row_part<T>(G, blk_of(G, row), row, t, x, y);
+    if (ok) {
+        const float* v = G.v + (size_t)(row >> 5) * (27 * 9 * 32) + (row & 31);
+        geo_row_part<T>(blk_of(G, row), row, t, [v](int e) { return v[(size_t)e * 32]; }, [x](int c) { return x[c]; }, y);
+    }
     sum_lanes<T>(y);
     if (!lead) return;
     if constexpr (!POST) {
@@ -1472,20 +1501,12 @@ __global__ void k_scale_blocks(int n, float* __restrict__ binv, const float* __r
 // and weights (1/2 from the neighbours across a cell of two) are computed.
 __device__ __forceinline__ int fine_of(int m, int nc, int nf) { return nc == nf ? m : min(2 * m, nf); }
 
-// x_f[i] += sum_I w_iI y_c[I] over the fine level's nodes (a fine node outside
-// every block -- padding between instances -- is left alone); G describes the
-// coarse level's blocks (with their finer blocks), row_blk the fine rows'.
-__global__ void k_vc_prolong(GeoView G, int n_fine, const float4* yc, float4* xf, const Control* ctl) {
-    pdl_begin();
-    if (vc_idle(ctl)) return;
-    const int f = blockIdx.x * blockDim.x + threadIdx.x;
-    if (f >= n_fine) return;
-    yc = rhs_of(yc, G.n_rows);
-    xf = rhs_of(xf, n_fine);
-    float4 acc = xf[f];
-    const BlkDev d = blk_of(G, f);
-    const int fl = f - d.fnode0, sj = d.fnz + 1, si = (d.fny + 1) * sj;
-    if (fl >= (d.fnx + 1) * si) return;
+// acc += sum_I w_I y_c[I] at node fl of the fine block of coarse block d; y(c) the
+// coarse vector's entry.  false: outside the block.
+template <typename Y>
+__device__ __forceinline__ bool prolong_at(const BlkDev& d, int fl, Y&& yc, float4& acc) {
+    const int sj = d.fnz + 1, si = (d.fny + 1) * sj;
+    if (fl >= (d.fnx + 1) * si) return false;
     const int at[3] = {fl / si, (fl % si) / sj, fl % sj};
     const int nf[3] = {d.fnx, d.fny, d.fnz}, nc[3] = {d.nx, d.ny, d.nz};
     int lo[3];
@@ -1502,7 +1523,7 @@ __global__ void k_vc_prolong(GeoView G, int n_fine, const float4* yc, float4* xf
     for (int q = 0; q < 8; ++q) {
         const int di = q >> 2, dj = (q >> 1) & 1, dk = q & 1;
         if ((!di || mid[0]) && (!dj || mid[1]) && (!dk || mid[2]))
-            y[q] = yc[base + (di * (d.ny + 1) + dj) * (d.nz + 1) + dk];
+            y[q] = yc(base + (di * (d.ny + 1) + dj) * (d.nz + 1) + dk);
     }
 #pragma unroll
     for (int q = 0; q < 8; ++q) {
@@ -1514,13 +1535,46 @@ __global__ void k_vc_prolong(GeoView G, int n_fine, const float4* yc, float4* xf
             acc.z += ww * y[q].z;
         }
     }
-    xf[f] = acc;
+    return true;
+}
+
+// x_f[i] += sum_I w_iI y_c[I] over the fine level's nodes (a fine node outside
+// every block -- padding between instances -- is left alone); G describes the
+// coarse level's blocks (with their finer blocks), row_blk the fine rows'.
+__global__ void k_vc_prolong(GeoView G, int n_fine, const float4* yc, float4* xf, const Control* ctl) {
+    pdl_begin();
+    if (vc_idle(ctl)) return;
+    const int f = blockIdx.x * blockDim.x + threadIdx.x;
+    if (f >= n_fine) return;
+    yc = rhs_of(yc, G.n_rows);
+    xf = rhs_of(xf, n_fine);
+    float4 acc = xf[f];
+    const BlkDev d = blk_of(G, f);
+    if (prolong_at(d, f - d.fnode0, [yc](int c) { return yc[c]; }, acc)) xf[f] = acc;
 }
 
 // Coarsest solve y = A_b^-1 b per block: one warp per row (eight loads a lane
 // in flight: a 256-wide row in one pass), kDenseRows rows a CTA.  y is
 // node-padded.
 constexpr int kDenseRows = 8;
+template <typename B>
+__device__ __forceinline__ float dense_row(const float* ar, int n, B&& b) {
+    const int lane = threadIdx.x & 31;
+    float a[8], bv[8], acc = 0.f;
+#pragma unroll
+    for (int t = 0; t < 8; ++t) {
+        const int j = lane + 32 * t;
+        a[t] = j < n ? ar[j] : 0.f;
+        bv[t] = j < n ? b(j) : 0.f;
+    }
+#pragma unroll
+    for (int t = 0; t < 8; ++t)
+        if (lane + 32 * t < n) acc = fmaf(a[t], bv[t], acc);
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, o);
+    return acc;
+}
+
 __global__ void __launch_bounds__(32 * kDenseRows) k_vc_dense(GeoView G, const float* __restrict__ ainv, const float* b,
                                                               float* y4, const Control* ctl) {
     pdl_begin();
@@ -1530,20 +1584,40 @@ __global__ void __launch_bounds__(32 * kDenseRows) k_vc_dense(GeoView G, const f
     const int n = 3 * (d.nx + 1) * (d.ny + 1) * (d.nz + 1);
     if (row >= n) return;
     const float* bb = rhs_of(b, 3 * (size_t)G.n_rows) + 3 * (size_t)d.node0;
-    const float* ar = ainv + d.dense0 + (size_t)row * n;
-    float a[8], bv[8], acc = 0.f;
-#pragma unroll
-    for (int t = 0; t < 8; ++t) {
-        const int j = lane + 32 * t;
-        a[t] = j < n ? ar[j] : 0.f;
-        bv[t] = j < n ? bb[j] : 0.f;
-    }
-#pragma unroll
-    for (int t = 0; t < 8; ++t)
-        if (lane + 32 * t < n) acc = fmaf(a[t], bv[t], acc);
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, o);
+    const float acc = dense_row(ainv + d.dense0 + (size_t)row * n, n, [bb](int j) { return bb[j]; });
     if (lane == 0) rhs_of(y4, 4 * (size_t)G.n_rows)[4 * ((size_t)d.node0 + row / 3) + row % 3] = acc;
+}
+
+// sum over the fine nodes f of w_x w_y w_z r(f) at node ol of coarse block d
+template <typename R>
+__device__ __forceinline__ float restrict_at(const BlkDev& d, int ol, R&& r) {
+    const int sj = d.nz + 1, si = (d.ny + 1) * sj;
+    const int m[3] = {ol / si, (ol % si) / sj, ol % sj};
+    const int nf[3] = {d.fnx, d.fny, d.fnz}, nc[3] = {d.nx, d.ny, d.nz};
+    int x[3];
+    bool on[3][3];  // axis, tap x - 1, x, x + 1
+#pragma unroll
+    for (int ax = 0; ax < 3; ++ax) {
+        x[ax] = fine_of(m[ax], nc[ax], nf[ax]);
+        on[ax][0] = m[ax] > 0 && x[ax] - fine_of(m[ax] - 1, nc[ax], nf[ax]) == 2;
+        on[ax][1] = true;
+        on[ax][2] = m[ax] < nc[ax] && fine_of(m[ax] + 1, nc[ax], nf[ax]) - x[ax] == 2;
+    }
+    float v[27];
+#pragma unroll
+    for (int q = 0; q < 27; ++q) {
+        const int a = q / 9, b = q / 3 % 3, c = q % 3;
+        const size_t src = d.fnode0 + ((size_t)(x[0] + a - 1) * (d.fny + 1) + (x[1] + b - 1)) * (d.fnz + 1) + (x[2] + c - 1);
+        v[q] = on[0][a] && on[1][b] && on[2][c] ? r(src) : 0.f;
+    }
+    float s = 0.f;
+#pragma unroll
+    for (int q = 0; q < 27; ++q) {
+        const int a = q / 9, b = q / 3 % 3, c = q % 3;
+        const float ww = (a == 1 ? 1.f : 0.5f) * (b == 1 ? 1.f : 0.5f) * (c == 1 ? 1.f : 0.5f);
+        if (on[0][a] && on[1][b] && on[2][c]) s = fmaf(ww, v[q], s);
+    }
+    return s;
 }
 
 // Trilinear restriction R = P^T over every block at once, four lanes per coarse
@@ -1566,32 +1640,7 @@ __global__ void __launch_bounds__(kT) k_vc_restrict(GeoView G, int n_fine, const
         for (int q = 0; q < 3; ++q) B[q] = binv[9 * (size_t)o + 3 * comp + q];
     }
     const BlkDev d = blk_of(G, o);
-    const int ol = o - d.node0, sj = d.nz + 1, si = (d.ny + 1) * sj;
-    const int m[3] = {ol / si, (ol % si) / sj, ol % sj};
-    const int nf[3] = {d.fnx, d.fny, d.fnz}, nc[3] = {d.nx, d.ny, d.nz};
-    int x[3];
-    bool on[3][3];  // axis, tap x - 1, x, x + 1
-#pragma unroll
-    for (int ax = 0; ax < 3; ++ax) {
-        x[ax] = fine_of(m[ax], nc[ax], nf[ax]);
-        on[ax][0] = m[ax] > 0 && x[ax] - fine_of(m[ax] - 1, nc[ax], nf[ax]) == 2;
-        on[ax][1] = true;
-        on[ax][2] = m[ax] < nc[ax] && fine_of(m[ax] + 1, nc[ax], nf[ax]) - x[ax] == 2;
-    }
-    float v[27];
-#pragma unroll
-    for (int q = 0; q < 27; ++q) {
-        const int a = q / 9, b = q / 3 % 3, c = q % 3;
-        const size_t src = d.fnode0 + ((size_t)(x[0] + a - 1) * (d.fny + 1) + (x[1] + b - 1)) * (d.fnz + 1) + (x[2] + c - 1);
-        v[q] = on[0][a] && on[1][b] && on[2][c] ? in[3 * src] : 0.f;
-    }
-    float s = 0.f;
-#pragma unroll
-    for (int q = 0; q < 27; ++q) {
-        const int a = q / 9, b = q / 3 % 3, c = q % 3;
-        const float ww = (a == 1 ? 1.f : 0.5f) * (b == 1 ? 1.f : 0.5f) * (c == 1 ? 1.f : 0.5f);
-        if (on[0][a] && on[1][b] && on[2][c]) s = fmaf(ww, v[q], s);
-    }
+    const float s = restrict_at(d, o - d.node0, [in](size_t f) { return in[3 * f]; });
     const int lane0 = (threadIdx.x & 31) & ~3;
     const float s0 = __shfl_sync(0xffffffffu, s, lane0), s1 = __shfl_sync(0xffffffffu, s, lane0 + 1),
                 s2 = __shfl_sync(0xffffffffu, s, lane0 + 2);
@@ -1599,6 +1648,261 @@ __global__ void __launch_bounds__(kT) k_vc_restrict(GeoView G, int n_fine, const
     rhs_of(out, 3 * (size_t)G.n_rows)[3 * (size_t)o + comp] = s;
     if (binv)
         reinterpret_cast<float*>(rhs_of(x4, G.n_rows) + o)[comp] = B[0] * s0 + B[1] * s1 + B[2] * s2;
+}
+
+// The V-cycle's smallest levels (down to the coarsest and back) of a lone block as
+// one launch, a cluster of 16 CTAs per right-hand side.  A step on these levels is
+// a few hundred cycles of work that a launch of its own turns into 3 us (and
+// a step through global memory with a cluster barrier into 2.5, most of it the
+// fence), so the vectors live in every CTA's shared memory: a CTA stores its rows'
+// results into the other copies, and a cluster barrier ends the step.  Each CTA owns a run of rows of every level.  What does not change
+// between V-cycles -- the own rows' values, columns and smoother blocks, the rows
+// of the coarsest inverse, the transfers' indices -- is laid out before the wait
+// for the kernel that restricts to the first level (nothing in between writes
+// any of it).  The prolongation is made by every CTA for its whole copy.  The
+// sums and their order are those of the separate kernels.  Bound by the barriers (1,500
+// cycles with the stores before them) and short dependent chains: 100 x 20 x 20
+// elements, levels of 936, 180 and 72 rows: nine launches of 28 us -> 19.5 serialised,
+// 12 with its loads under the kernel before it; 57 x 13 x 11: 16 -> 11.
+__device__ __forceinline__ void tail_tables(const TailView& V, int l, float* tsm, int r0, int mine) {
+    const TailView::Level& L = V.L[l];
+    const BlkDev& d = L.d;
+    const int tid = threadIdx.x, sj = d.nz + 1, si = (d.ny + 1) * sj;
+    if (l < V.n - 1) {
+        uint16_t* col = reinterpret_cast<uint16_t*>(tsm + L.co);
+        for (int q = tid; q < mine * kTailCols; q += kTailThreads) {
+            const int lr = q / kTailCols, e = q % kTailCols, row = r0 + lr;
+            const int i = row / si, j = (row - i * si) / sj, k = row - i * si - j * sj;
+            const int i0 = max(i - 1, 0), j0 = max(j - 1, 0), k0 = max(k - 1, 0);
+            const int nj = min(j + 1, d.ny) - j0 + 1, nk = min(k + 1, d.nz) - k0 + 1;
+            const int len = (min(i + 1, d.nx) - i0 + 1) * nj * nk;
+            const int ek = e / nk;
+            col[q] = (uint16_t)(e == 27 ? len : e < len ? (i0 + ek / nj) * si + (j0 + ek % nj) * sj + k0 + e - ek * nk : row);
+            if (e < 9) tsm[L.so + 12 * lr + 3 + e] = L.binv[9 * (size_t)row + e];
+        }
+        const BlkDev& c = V.L[l + 1].d;
+        uint16_t* pro = reinterpret_cast<uint16_t*>(tsm + L.po);
+        for (int f = tid; f < L.n_rows; f += kTailThreads) {
+            const int at[3] = {f / si, (f % si) / sj, f % sj};
+            const int nf[3] = {c.fnx, c.fny, c.fnz}, nc[3] = {c.nx, c.ny, c.nz};
+            int lo[3], mid = 0;
+#pragma unroll
+            for (int ax = 0; ax < 3; ++ax) {
+                const bool two = nc[ax] != nf[ax];
+                lo[ax] = !two ? at[ax] : (at[ax] == nf[ax] ? nc[ax] : at[ax] >> 1);
+                mid |= (two && (at[ax] & 1) && at[ax] < nf[ax]) << ax;
+            }
+            pro[f] = (uint16_t)(8 * nid(lo[0], lo[1], lo[2], c.ny, c.nz) + mid);
+        }
+    }
+    if (l > 0) {
+        int* res = reinterpret_cast<int*>(tsm + L.to);
+        for (int q = tid; q < mine; q += kTailThreads) {
+            const int o = r0 + q, m[3] = {o / si, (o % si) / sj, o % sj};
+            const int nf[3] = {d.fnx, d.fny, d.fnz}, nc[3] = {d.nx, d.ny, d.nz};
+            int x[3], on = 0;
+#pragma unroll
+            for (int ax = 0; ax < 3; ++ax) {
+                x[ax] = fine_of(m[ax], nc[ax], nf[ax]);
+                on |= (m[ax] > 0 && x[ax] - fine_of(m[ax] - 1, nc[ax], nf[ax]) == 2) << (2 * ax);
+                on |= (m[ax] < nc[ax] && fine_of(m[ax] + 1, nc[ax], nf[ax]) - x[ax] == 2) << (2 * ax + 1);
+            }
+            res[q] = nid(x[0], x[1], x[2], d.fny, d.fnz) + (on << 16);
+        }
+    }
+}
+
+__global__ void __launch_bounds__(kTailThreads) k_vc_tail(const __grid_constant__ TailView V,
+                                                          const float* __restrict__ ainv, const Control* ctl) {
+    extern __shared__ __align__(16) float tsm[];
+    cooperative_groups::cluster_group cl = cooperative_groups::this_cluster();
+    const int rank = (int)cl.block_rank(), tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    const int last = V.n - 1;
+    auto vec = [&](int off) { return reinterpret_cast<float4*>(tsm + off); };
+    for (int l = 0; l <= last; ++l) {
+        const TailView::Level& L = V.L[l];
+        const int r0 = rank * L.own, mine = max(0, min(L.own, L.n_rows - r0));
+        if (l < last && L.vo >= 0)  // a warp reads an entry of 32 rows at a time
+            for (int p = 0; p < mine; p += 32) {
+                const int lr = min(p + lane, mine - 1), row = r0 + lr;
+                const float* src = L.v + (size_t)(row >> 5) * (27 * 9 * 32) + (row & 31);
+                float* dst = tsm + L.vo + lr * kTailLd;
+#pragma unroll 8
+                for (int e = warp; e < 27 * 9; e += kTailThreads / 32) dst[e] = src[(size_t)e * 32];
+            }
+        tail_tables(V, l, tsm, r0, mine);
+    }
+    // the coarsest inverse: one warp a row
+    const int nd = 3 * V.L[last].n_rows, drow = warp * kTailCtas + rank;
+    float ai[8];
+#pragma unroll
+    for (int t = 0; t < 8; ++t)
+        ai[t] = drow < nd && lane + 32 * t < nd ? ainv[(size_t)drow * nd + lane + 32 * t] : 0.f;
+    cl.sync();  // every CTA runs: its shared memory may be written
+    pdl_begin();
+    if (vc_idle(ctl)) return;  // the same for the whole cluster
+    {
+        const TailView::Level& L = V.L[0];
+        const int r0 = rank * L.own, mine = max(0, min(L.own, L.n_rows - r0));
+        const float4* x = rhs_of(V.x4, L.n_rows);
+        const float* b = rhs_of(V.b, 3 * (size_t)L.n_rows) + 3 * r0;
+        for (int q = tid; q < L.n_rows; q += kTailThreads) vec(L.xo)[q] = x[q];
+        for (int q = tid; q < 3 * mine; q += kTailThreads) tsm[L.so + q / 3 * 12 + q % 3] = b[q];
+    }
+    __syncthreads();
+    // residuals b - A x of the own rows of level l, 16 lanes a row (all get the sums)
+    auto rows = [&](int l, auto&& epi) {
+        const TailView::Level& L = V.L[l];
+        const float4* x = vec(L.xo);
+        const int t = tid & 15, r0 = rank * L.own, mine = min(L.own, L.n_rows - r0);
+        for (int p = 0; p < L.own; p += kTailThreads / 16) {
+            const int lr = p + (tid >> 4), row = r0 + lr;
+            const bool ok = lr < mine;
+            const float* own = tsm + L.so + lr * 12;
+            float y[3] = {0.f, 0.f, 0.f};
+            if (ok) {
+                const uint16_t* col = reinterpret_cast<const uint16_t*>(tsm + L.co) + lr * kTailCols;
+                const int len = col[27];
+                auto part = [&](auto&& v) {
+                    float m[2][9];
+                    float4 xv[2];
+#pragma unroll
+                    for (int u = 0; u < 2; ++u)
+                        if (t + 16 * u < len) {
+                            xv[u] = x[col[t + 16 * u]];
+#pragma unroll
+                            for (int w = 0; w < 9; ++w) m[u][w] = v((t + 16 * u) * 9 + w);
+                        }
+#pragma unroll
+                    for (int u = 0; u < 2; ++u)
+                        if (t + 16 * u < len)
+#pragma unroll
+                            for (int a = 0; a < 3; ++a)
+                                y[a] = fmaf(m[u][a * 3], xv[u].x,
+                                            fmaf(m[u][a * 3 + 1], xv[u].y, fmaf(m[u][a * 3 + 2], xv[u].z, y[a])));
+                };
+                if (L.vo >= 0) {
+                    const float* v = tsm + L.vo + lr * kTailLd;
+                    part([v](int e) { return v[e]; });
+                } else {
+                    const float* v = L.v + (size_t)(row >> 5) * (27 * 9 * 32) + (row & 31);
+                    part([v](int e) { return v[e * 32]; });
+                }
+            }
+            sum_lanes<16>(y);
+            if (ok) {
+                const float r[3] = {own[0] - y[0], own[1] - y[1], own[2] - y[2]};
+                epi(row, t, own + 3, r);
+            }
+        }
+    };
+    // own rows of a vector to the other CTAs' copies: two warps a CTA, 512 bytes a store
+    auto publish = [&](int off, int own, int n) {
+        __syncthreads();
+        const int r0 = rank * own, mine = min(own, n - r0), to = warp & (kTailCtas - 1);
+        const float4* src = vec(off) + r0;
+        float4* dst = cl.map_shared_rank(vec(off), to) + r0;
+        if (to != rank)
+            for (int q = lane + 32 * (warp / kTailCtas); q < mine; q += 32 * (kTailThreads / 32 / kTailCtas)) dst[q] = src[q];
+        cl.sync();
+    };
+    for (int l = 0; l < last; ++l) {
+        const TailView::Level &L = V.L[l], &C = V.L[l + 1];
+        rows(l, [&](int row, int t, const float*, const float (&r)[3]) {
+            if (t == 0) vec(L.ro)[row] = make_float4(r[0], r[1], r[2], 0.f);
+        });
+        publish(L.ro, L.own, L.n_rows);
+        // restriction and the coarse level's first sweep, four lanes a node
+        const float* r = reinterpret_cast<const float*>(vec(L.ro));
+        const int sj = C.d.fnz + 1, si = (C.d.fny + 1) * sj;
+        const int comp = min(tid & 3, 2), quad = lane & ~3, r0 = rank * C.own, mine = min(C.own, C.n_rows - r0);
+        for (int p = 0; p < C.own; p += kTailThreads / 4) {
+            if (p + 8 * warp >= mine) continue;  // the warp's nodes
+            const int lo = p + (tid >> 2);
+            const bool ok = lo < mine;
+            const int at = reinterpret_cast<const int*>(tsm + C.to)[min(lo, mine - 1)], on = at >> 16;
+            const float* rc = r + 4 * (at & 0xffff) + comp;
+            float v[27], s = 0.f;
+#pragma unroll
+            for (int q = 0; q < 27; ++q) {  // all in flight; the sides that do not contribute add 0
+                const int i = q / 9, j = q / 3 % 3, k = q % 3;
+                const int need = (i == 1 ? 0 : 1 << (i / 2)) | (j == 1 ? 0 : 4 << (j / 2)) | (k == 1 ? 0 : 16 << (k / 2));
+                const bool in = (on & need) == need;
+                v[q] = rc[in ? 4 * ((i - 1) * si + (j - 1) * sj + k - 1) : 0];
+                v[q] = in ? v[q] : 0.f;
+            }
+#pragma unroll
+            for (int q = 0; q < 27; ++q)
+                s = fmaf((q / 9 == 1 ? 1.f : 0.5f) * (q / 3 % 3 == 1 ? 1.f : 0.5f) * (q % 3 == 1 ? 1.f : 0.5f), v[q], s);
+            const float s0 = __shfl_sync(0xffffffffu, s, quad), s1 = __shfl_sync(0xffffffffu, s, quad + 1),
+                        s2 = __shfl_sync(0xffffffffu, s, quad + 2);
+            float4 out = make_float4(s0, s1, s2, 0.f);
+            if (l + 1 < last) {
+                float* own = tsm + C.so + min(lo, mine - 1) * 12;
+                const float* B = own + 3 + 3 * comp;
+                const float x = B[0] * s0 + B[1] * s1 + B[2] * s2;
+                if (ok && (tid & 3) != 3) own[comp] = s;
+                out.x = __shfl_sync(0xffffffffu, x, quad);
+                out.y = __shfl_sync(0xffffffffu, x, quad + 1);
+                out.z = __shfl_sync(0xffffffffu, x, quad + 2);
+            }
+            if (ok && (tid & 3) == 0) vec(C.xo)[r0 + lo] = out;
+        }
+        publish(C.xo, C.own, C.n_rows);
+    }
+    {
+        const TailView::Level& L = V.L[last];
+        const float* b = reinterpret_cast<const float*>(vec(L.xo));
+        if (drow < nd) {
+            float bv[8], acc = 0.f;
+#pragma unroll
+            for (int t = 0; t < 8; ++t) {
+                const int j = lane + 32 * t;
+                bv[t] = j < nd ? b[4 * (j / 3) + j % 3] : 0.f;
+            }
+#pragma unroll
+            for (int t = 0; t < 8; ++t)
+                if (lane + 32 * t < nd) acc = fmaf(ai[t], bv[t], acc);
+#pragma unroll
+            for (int o = 16; o > 0; o >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, o);
+            if (lane < kTailCtas)
+                reinterpret_cast<float*>(cl.map_shared_rank(vec(L.ro), lane) + drow / 3)[drow % 3] = acc;
+        }
+        cl.sync();
+    }
+    for (int l = last - 1; l >= 0; --l) {
+        const TailView::Level &L = V.L[l], &C = V.L[l + 1];
+        float4* x = vec(L.xo);
+        const float4* yc = vec(C.ro);
+        const int sj = C.d.nz + 1, si = (C.d.ny + 1) * sj;
+        for (int f = tid; f < L.n_rows; f += kTailThreads) {
+            const int at = reinterpret_cast<const uint16_t*>(tsm + L.po)[f], mid = at & 7;
+            const float ww = (mid & 1 ? 0.5f : 1.f) * (mid & 2 ? 0.5f : 1.f) * (mid & 4 ? 0.5f : 1.f);
+            const float4* y = yc + (at >> 3);
+            float4 acc = x[f];
+#pragma unroll
+            for (int q = 0; q < 8; ++q) {
+                const int need = (q >> 2) | (q & 2) | (q & 1) << 2;  // q = 4 di + 2 dj + dk
+                if ((mid & need) == need) {
+                    const float4 v = y[(q >> 2) * si + (q >> 1 & 1) * sj + (q & 1)];
+                    acc.x += ww * v.x;
+                    acc.y += ww * v.y;
+                    acc.z += ww * v.z;
+                }
+            }
+            x[f] = acc;
+        }
+        __syncthreads();
+        float4* y4 = rhs_of(V.y4, L.n_rows);
+        rows(l, [&](int row, int t, const float* B, const float (&e)[3]) {
+            const float4 xv = x[row];
+            const float4 y = make_float4(xv.x + B[0] * e[0] + B[1] * e[1] + B[2] * e[2],
+                                         xv.y + B[3] * e[0] + B[4] * e[1] + B[5] * e[2],
+                                         xv.z + B[6] * e[0] + B[7] * e[1] + B[8] * e[2], 0.f);
+            if (t == 0) (l > 0 ? vec(L.ro) : y4)[row] = y;
+        });
+        if (l > 0) publish(L.ro, L.own, L.n_rows);
+    }
 }
 
 // ---------------------------------------------------------------------------
@@ -2472,6 +2776,55 @@ std::vector<MgBlk> level0_blocks(const Ctx& c) {
     return out;
 }
 
+// The fused tail takes every level below the finest whose vectors fit in a CTA's
+// shared memory; values go there from the coarsest level up while they fit.
+// Stacks keep one launch per level and step: a cluster per block needs more
+// SMs than there are, and the blocks' rows fill them as it is.
+void plan_tail(MgHierarchy& H) {
+    const int nl = (int)H.L.size();
+    if (H.n_blk != 1 || nl < 3) return;
+    constexpr int kFloats = kTailSmem / 4;
+    auto own = [&](int l) { return (H.L[l]->n_nodes + kTailCtas - 1) / kTailCtas; };
+    auto up4 = [](int n) { return (n + 3) / 4 * 4; };
+    int at = 0;
+    TailView& V = H.tail;
+    V = TailView{};
+    std::vector<TailView::Level> lv;  // from the coarsest up
+    for (int l = nl - 1; l >= 1 && nl - l <= kTailLevels; --l) {
+        MgLevel& M = *H.L[l];
+        const int n = M.n_nodes, o = own(l);
+        TailView::Level L{M.one, M.own.v32.p, M.binv.p, n, o, 0, 0, 0, 0, 0, 0, -1};
+        int off = at;
+        auto take = [&](int floats) { const int p = off; off += up4(floats); return p; };
+        L.xo = take(4 * n);
+        L.ro = take(4 * n);
+        L.to = take(o);
+        if (l + 1 < nl) {
+            L.so = take(12 * o);
+            L.co = take((kTailCols * o + 1) / 2);
+            L.po = take((n + 1) / 2);
+        }
+        if (off > kFloats || n > kTailRows) break;
+        at = off;
+        lv.push_back(L);
+    }
+    V.n = (int)lv.size();
+    if (V.n < 2) return;
+    for (int q = 0; q < V.n; ++q) {
+        TailView::Level& L = V.L[V.n - 1 - q];
+        L = lv[q];
+        const int need = up4(L.own * kTailLd);
+        if (q > 0 && at + need <= kFloats) {
+            L.vo = at;
+            at += need;
+        }
+    }
+    H.tail0 = nl - V.n;
+    H.tail_smem = 4 * at;
+    ASEND_CUDA(cudaFuncSetAttribute(k_vc_tail, cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
+    ASEND_CUDA(cudaFuncSetAttribute(k_vc_tail, cudaFuncAttributeMaxDynamicSharedMemorySize, kTailSmem));
+}
+
 void build_hierarchy(Ctx& c) {
     if (c.type != 8 && c.type != 81)
         throw InputError("multigrid needs structured hex8 / brickIM blocks (asend_set_block_structure or "
@@ -2615,6 +2968,7 @@ void build_hierarchy(Ctx& c) {
     if (dense_tot > (size_t)INT32_MAX) throw InputError("multigrid coarsest blocks too large");
     H->dense.alloc(dense_tot);
     for (int l = 0; l < (int)H->L.size(); ++l) level_tables(c, *H, l);
+    plan_tail(*H);
     ASEND_CUDA(cudaStreamSynchronize(c.stream));
     c.mg = H;
 }
@@ -2840,6 +3194,28 @@ void level_rows(Ctx& c, int l, bool post, const Control* ctl, int nr = 1) {
     else launch_k(c, k_vc_resid_staged, grid, kT, smem, sbview(L), L.b.p, x, L.r.p, ctl);
 }
 
+void fused_tail(Ctx& c, const Control* ctl, int nr) {
+    MgHierarchy& H = *c.mg;
+    TailView V = H.tail;
+    MgLevel& T = *H.L[H.tail0];
+    V.b = T.b.p;
+    V.x4 = reinterpret_cast<const float4*>(T.x4.p);
+    V.y4 = reinterpret_cast<float4*>(T.y4.p);
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(kTailCtas, (unsigned)nr);
+    cfg.blockDim = dim3(kTailThreads);
+    cfg.dynamicSmemBytes = (size_t)H.tail_smem;
+    cfg.stream = c.stream;
+    cudaLaunchAttribute at[2];
+    at[0].id = cudaLaunchAttributeClusterDimension;
+    at[0].val.clusterDim = {kTailCtas, 1, 1};
+    at[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    at[1].val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = at;
+    cfg.numAttrs = c.pdl ? 2 : 1;
+    ASEND_CUDA(cudaLaunchKernelEx(&cfg, k_vc_tail, V, (const float*)H.dense.p, ctl));
+}
+
 void vcycle(Ctx& c, const Control* ctl, bool fused0, int nr = 1) {
     MgHierarchy& H = *c.mg;
     const int nl = (int)H.L.size();
@@ -2848,18 +3224,22 @@ void vcycle(Ctx& c, const Control* ctl, bool fused0, int nr = 1) {
         launch_k(c, k_vc_smooth0, dim3(grid_of(L.n_nodes), nr), kT, 0, L.n_nodes, L.binv.p, L.b.p,
                  reinterpret_cast<float4*>(L.x4.p), ctl);
     }
-    for (int l = 0; l < nl - 1; ++l) {
+    const int top = c.mg_tail && H.tail0 ? H.tail0 : nl - 1;
+    for (int l = 0; l < top; ++l) {
         level_rows(c, l, false, ctl, nr);
         restrict_to(c, l, ctl, nr);
     }
-    coarsest_solve(c, ctl, nr);
-    for (int l = nl - 2; l >= 0; --l) {
+    if (top < nl - 1) fused_tail(c, ctl, nr);
+    else coarsest_solve(c, ctl, nr);
+    for (int l = top - 1; l >= 0; --l) {
         prolong_from(c, l, ctl, nr);
         level_rows(c, l, true, ctl, nr);
     }
 }
 
-int vcycle_launches(const Ctx& c) { return 4 * ((int)c.mg->L.size() - 1) + 1; }
+int vcycle_launches(const Ctx& c) {
+    return 4 * (c.mg_tail && c.mg->tail0 ? c.mg->tail0 : (int)c.mg->L.size() - 1) + 1;
+}
 
 // Level vectors for nr right-hand sides (grow only; the captured graphs hold
 // their addresses).
@@ -3301,12 +3681,12 @@ int pcg_solve_mg_once(Ctx& c, const asend_solve_opts& o, asend_solve_stats* st, 
         // G iterations as one graph, kept with the hierarchy and reused while
         // the launch arguments are the same (they fully define the graph)
         // (with everything else that changes the captured sequence: the
-        // method, the chunk length, the product shape, the launch overlap and
-        // the matrix-free plan)
+        // method, the chunk length, the product shape, the launch overlap, the
+        // fused tail and the matrix-free plan)
         std::vector<uint8_t> key(sizeof(MgPcg) + 4 * sizeof(int) + sizeof(void*));
         std::memcpy(key.data(), &M, sizeof(MgPcg));
         std::memcpy(key.data() + sizeof(MgPcg) + 4 * sizeof(int), &H.box, sizeof(void*));
-        const int extra[4] = {o.method, G, c.product_variant, (H.box_cycle ? 1 : 0) | (c.pdl ? 2 : 0)};
+        const int extra[4] = {o.method, G, c.product_variant, (H.box_cycle ? 1 : 0) | (c.pdl ? 2 : 0) | (c.mg_tail ? 4 : 0)};
         std::memcpy(key.data() + sizeof(MgPcg), extra, sizeof(extra));
         cudaGraphExec_t exec = nullptr;
         for (auto& g : H.graphs)

@@ -522,12 +522,13 @@ class GpuSolver:
 
     def set_product_variant(self, variant):
         """Shape of the multigrid CG's split outer product (_lib.PRODUCT_*):
-        register-fed or staged through shared memory; results are identical."""
+        matrix-free where the model allows (default), register-fed or
+        staged through shared memory; the last two give identical results."""
         self._check(self.lib.asend_set_product_variant(self.ctx, int(variant)), "set_product_variant")
 
     def mg_set_fused_tail(self, enable=True):
-        """Multigrid: the smallest levels as one fused launch (default) or one
-        launch per level and step; same arithmetic."""
+        """Multigrid: the smallest levels of a lone block as one fused launch
+        (default) or one launch per level and step; same arithmetic."""
         self._check(self.lib.asend_mg_set_fused_tail(self.ctx, int(bool(enable))), "mg_set_fused_tail")
 
     def set_launch_overlap(self, enable=True):

@@ -150,10 +150,10 @@ int asend_mg_set_damping(asend_ctx* ctx, double factor);
 #define ASEND_PRODUCT_STAGED_2x2 4
 #define ASEND_PRODUCT_STAGED_4x2 5
 int asend_set_product_variant(asend_ctx* ctx, int32_t variant);
-/* Multigrid V-cycle: the deepest levels as one fused launch (enable = 1, the
- * default) or as one launch per level and step (enable = 0), the same
- * arithmetic either way.  The separate launches have become the faster form on
- * every model, so both settings now run them; the call keeps its checks.
+/* Multigrid V-cycle: the deepest levels of a lone block as one fused launch
+ * (enable = 1, the default) or as one launch per level and step (enable = 0),
+ * the same arithmetic either way.  Stacks of instances, whose levels fill the
+ * GPU, always take separate launches; the call keeps its checks.
  * No counterpart in the reference (it has no multigrid); a tuning and
  * diagnostic switch of the preconditioner that replaces the reference's
  * block-LDL^T (lower_tri_mat_meth.rs:15-241). */
