@@ -327,10 +327,23 @@ __device__ __forceinline__ void block_sum(double (&v)[K], double* smem /* [32*K]
     if (warp == 0) {
 #pragma unroll
         for (int k = 0; k < K; ++k) {
-            double t = (lane < nw) ? smem[lane * K + k] : 0.0;
-            v[k] = warp_sum(t);
+            v[k] = (lane < nw) ? smem[lane * K + k] : 0.0;
+            // the stages that would only add zeros are skipped (an FP64 addition
+            // is 107 cycles of a chain that every CG scalar waits for)
+#pragma unroll
+            for (int o = 16; o > 0; o >>= 1)
+                if (o < nw) v[k] += __shfl_xor_sync(0xffffffffu, v[k], o);
         }
     }
+}
+
+// One more CTA done: what this thread wrote before is visible to whoever takes a
+// later ticket (after a barrier to its whole CTA).  One release / acquire
+// atomic instead of two full fences around a relaxed one.
+__device__ __forceinline__ uint32_t take_ticket(uint32_t* ticket) {
+    uint32_t t;
+    asm volatile("atom.add.acq_rel.gpu.global.u32 %0, [%1], 1;" : "=r"(t) : "l"(ticket) : "memory");
+    return t;
 }
 
 // host-side helpers implemented in the .cu files

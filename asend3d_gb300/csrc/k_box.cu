@@ -436,6 +436,7 @@ __global__ void __launch_bounds__(kBoxThreads, 1) k_box_power(BoxArgs X, const f
                                                               const float4* __restrict__ x, float4* __restrict__ y4,
                                                               float* __restrict__ nrm, int k, double* __restrict__ part,
                                                               uint32_t* __restrict__ ticket) {
+    pdl_begin();
     extern __shared__ __align__(16) unsigned char smem[];
     __shared__ double sm[32];
     __shared__ bool last;
@@ -453,12 +454,10 @@ __global__ void __launch_bounds__(kBoxThreads, 1) k_box_power(BoxArgs X, const f
     block_sum<1>(a, sm);
     if (threadIdx.x == 0) {
         part[blockIdx.x] = a[0];
-        __threadfence();
-        last = atomicAdd(ticket + k, 1u) == gridDim.x - 1;
+        last = take_ticket(ticket + k) == gridDim.x - 1;
     }
     __syncthreads();
     if (!last) return;
-    __threadfence();
     double s[1] = {0.0};
 #pragma unroll 4
     for (int b = threadIdx.x; b < (int)gridDim.x; b += blockDim.x) s[0] += __ldcg(part + b);
@@ -580,7 +579,17 @@ template <typename T, typename... K, typename... Args>
 void launch(Ctx& c, const BoxPlan& P, int nr, void (*k)(K...), Args... args) {
     const size_t smem = box_smem<T>(P.threads, P.halo);
     ASEND_CUDA(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-    k<<<dim3(P.n_items, nr), P.threads, smem, c.stream>>>(args...);
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3((unsigned)P.n_items, (unsigned)nr);
+    cfg.blockDim = dim3((unsigned)P.threads);
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = c.stream;
+    cudaLaunchAttribute at[1];
+    at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    at[0].val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = at;
+    cfg.numAttrs = c.pdl ? 1 : 0;
+    ASEND_CUDA(cudaLaunchKernelEx(&cfg, k, K(args)...));
 }
 
 }  // namespace

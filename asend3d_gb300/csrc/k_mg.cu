@@ -188,7 +188,8 @@ void launch_k(const Ctx& c, void (*k)(KArgs...), dim3 grid, int block, size_t sm
     ASEND_CUDA(cudaLaunchKernelEx(&cfg, k, std::forward<Args>(args)...));
 }
 // Levels with at least this many node rows run the staged (bulk-copy) row
-// products, one row per lane; smaller ones split each row over T lanes.
+// products, one row per lane; smaller ones split each row over 16 lanes (with
+// fewer, 8,192 rows leave SMs idle).
 constexpr int kStagedRows = 8192;
 // classes up to which the first coarsening uses projected class matrices
 // (27 x 576 floats each, 62 KB)
@@ -1369,12 +1370,10 @@ __global__ void __launch_bounds__(kT) k_pow_step(SbView A, const float* __restri
     block_sum<1>(acc, sm);
     if (threadIdx.x == 0) {
         part[blockIdx.x] = acc[0];
-        __threadfence();
-        last = atomicAdd(ticket + k, 1u) == gridDim.x - 1;
+        last = take_ticket(ticket + k) == gridDim.x - 1;
     }
     __syncthreads();
     if (!last) return;
-    __threadfence();
     double s[1] = {0.0};
 #pragma unroll 4
     for (int b = threadIdx.x; b < (int)gridDim.x; b += blockDim.x) s[0] += __ldcg(part + b);
@@ -1437,12 +1436,10 @@ __global__ void __launch_bounds__(kT) k_pow_rows(GeoView G, const float* __restr
     block_sum<1>(acc, sm);
     if (threadIdx.x == 0) {
         part[blockIdx.x] = acc[0];
-        __threadfence();
-        last = atomicAdd(ticket + k, 1u) == gridDim.x - 1;
+        last = take_ticket(ticket + k) == gridDim.x - 1;
     }
     __syncthreads();
     if (!last) return;
-    __threadfence();
     double s[1] = {0.0};
 #pragma unroll 4
     for (int b = threadIdx.x; b < (int)gridDim.x; b += blockDim.x) s[0] += __ldcg(part + b);
@@ -1977,6 +1974,7 @@ __device__ __forceinline__ void fused_smooth0(const MgPcg& M, int row, const dou
 
 template <typename TV, typename TP>
 __global__ void __launch_bounds__(kThreads) k_mg_spmv_dot(MgPcg M) {
+    pdl_begin();
     using PV = typename ApOf<TP>::T;
     M = rhs_view<sizeof(TV) == 4 && std::is_same<TP, float>::value>(M);
     const PcgArgs& A = M.a;
@@ -2006,24 +2004,29 @@ __global__ void __launch_bounds__(kThreads) k_mg_spmv_dot(MgPcg M) {
     }
 }
 
-// The FP64 product with T lanes a row, for single models whose rows alone leave
+// The FP64 product with four lanes a row, for single models whose rows alone leave
 // SMs idle: one thread a row walked 27 columns one step after the other (7,930
-// rows: 52.6 us), T lanes share them.
-template <int T>
+// rows: 52.6 us).  FP64 issue (64 cycles a warp instruction) bounds it from there:
+// the lanes' sums are exchanged so that each lane ends with one component (3
+// additions, where eight lanes with the whole sum each took 9 for half the rows)
+// and makes that component's share of p.Ap; 7,930
+// rows, two right-hand sides: eight lanes 19.7 us, now 13.4.
+constexpr int kLaneRows = 152 * 1024 / 4;  // rows whose lanes fill the GPU
 __global__ void __launch_bounds__(kThreads) k_mg_spmv_dot_lanes(MgPcg M) {
+    pdl_begin();
     M = rhs_view<false>(M);
     const PcgArgs& A = M.a;
     RhsScalars* S = A.sc;
     if (mg_done(A, S)) return;
     const int gt = blockIdx.x * blockDim.x + threadIdx.x;
-    const int row = gt / T, t = gt % T;
+    const int row = gt / 4, t = gt % 4;
     const bool ok = row < A.n_rows;
     double y[3] = {0.0, 0.0, 0.0}, d[1][1] = {{0.0}};
     if (ok) {
         const int lane = row & 31, len = A.row_len[row];
         const int64_t g0 = A.slice_off[row >> 5];
 #pragma unroll 2
-        for (int j = t; j < len; j += T) {
+        for (int j = t; j < len; j += 4) {
             const int64_t g = g0 + j;
             double m[9], p[3];
             PadVec<double>::load(A.p, (size_t)A.col[g * 32 + lane], p);
@@ -2033,19 +2036,15 @@ __global__ void __launch_bounds__(kThreads) k_mg_spmv_dot_lanes(MgPcg M) {
             for (int a = 0; a < 3; ++a) y[a] = fma(m[3 * a], p[0], fma(m[3 * a + 1], p[1], fma(m[3 * a + 2], p[2], y[a])));
         }
     }
-#pragma unroll
-    for (int o = T / 2; o >= 1; o >>= 1)
-#pragma unroll
-        for (int a = 0; a < 3; ++a) y[a] += __shfl_xor_sync(0xffffffffu, y[a], o);
-    if (ok && t == 0) {
+    const bool up = t & 2, odd = t & 1;
+    double lo = (up ? y[2] : y[0]) + __shfl_xor_sync(0xffffffffu, up ? y[0] : y[2], 2);
+    const double hi = (up ? 0.0 : y[1]) + __shfl_xor_sync(0xffffffffu, up ? y[1] : 0.0, 2);
+    lo = (odd ? hi : lo) + __shfl_xor_sync(0xffffffffu, odd ? lo : hi, 1);  // component t
+    if (ok && t < 3) {
         double pv[3];
         PadVec<double>::load(A.p, row, pv);
-        double* ap = reinterpret_cast<double*>(A.ap) + 3 * (size_t)row;
-#pragma unroll
-        for (int q = 0; q < 3; ++q) {
-            ap[q] = y[q];
-            d[0][0] += pv[q] * y[q];
-        }
+        reinterpret_cast<double*>(A.ap)[3 * (size_t)row + t] = lo;
+        d[0][0] = (t == 0 ? pv[0] : t == 1 ? pv[1] : pv[2]) * lo;
     }
     double tot[1][1];
     if (last_block_reduce<1, 1>(A, d, 0, tot) && threadIdx.x == 0) {
@@ -2428,6 +2427,7 @@ void launch_split_product(Ctx& c, const MgPcg& M, dim3 grid) {
 
 template <typename TP>
 __global__ void __launch_bounds__(kThreads) k_mg_update_xr(MgPcg M) {
+    pdl_begin();
     using PV = typename ApOf<TP>::T;
     M = rhs_view<std::is_same<TP, float>::value>(M);
     const PcgArgs& A = M.a;
@@ -2475,6 +2475,7 @@ __global__ void __launch_bounds__(kThreads) k_mg_update_xr(MgPcg M) {
 //         flag is set (initialisation, or convergence of the recurrence)
 template <typename TP>
 __global__ void __launch_bounds__(kThreads) k_mg_rz(MgPcg M, int mode) {
+    pdl_begin();
     using PV = typename ApOf<TP>::T;
     M = rhs_view<std::is_same<TP, float>::value>(M);
     const PcgArgs& A = M.a;
@@ -2516,6 +2517,7 @@ __global__ void __launch_bounds__(kThreads) k_mg_rz(MgPcg M, int mode) {
 
 template <typename TP>
 __global__ void __launch_bounds__(kThreads) k_mg_update_p(MgPcg M) {
+    pdl_begin();
     using PV = typename ApOf<TP>::T;
     M = rhs_view<std::is_same<TP, float>::value>(M);
     const PcgArgs& A = M.a;
@@ -3132,31 +3134,6 @@ void prolong_from(Ctx& c, int l, const Control* ctl, int nr = 1) {
 
 // One V(1,1) cycle on level 0's b.  With fused0, the caller has already
 // written level 0's first sweep x4 = B^-1 b (fused into the PCG update).
-// Lanes per row of a level's products: one per row while the rows alone
-// fill the GPU (about 152 SMs x 1024 threads), else the smallest power of two
-// up to 16 that does.
-int lanes_for(int n_rows) {
-    constexpr int kFill = 152 * 1024;
-    int t = 1;
-    while (t < 16 && (int64_t)n_rows * t < kFill) t *= 2;
-    return t;
-}
-
-template <bool POST>
-void launch_rows(Ctx& c, MgLevel& L, int t, const Control* ctl, int nr) {
-    const dim3 grid((unsigned)(((int64_t)L.n_nodes * t + kT - 1) / kT), nr);
-    const GeoView G = geo_of(L, L);
-    const float4* x = reinterpret_cast<const float4*>(L.x4.p);
-    float4* y = reinterpret_cast<float4*>(L.y4.p);
-    auto go = [&](auto k) { launch_k(c, k, grid, kT, 0, G, L.binv.p, L.b.p, x, L.r.p, y, ctl); };
-    switch (t) {
-        case 2: go(k_vc_rows<2, POST>); break;
-        case 4: go(k_vc_rows<4, POST>); break;
-        case 8: go(k_vc_rows<8, POST>); break;
-        default: go(k_vc_rows<16, POST>); break;
-    }
-}
-
 // Residual r = b - A x (post = false) or post-smoothing y4 = x + B^-1 (b - A x) of
 // level l for nr right-hand sides: matrix-free on the finest level of a box
 // model inside the CG, staged for many rows, several lanes a row for few.
@@ -3170,21 +3147,16 @@ void level_rows(Ctx& c, int l, bool post, const Control* ctl, int nr = 1) {
         else box_resid(c, *H.box, L.b.p, x, L.r.p, ctl, nr);
         return;
     }
-    const int t = L.n_nodes >= kStagedRows ? 1 : lanes_for(L.n_nodes);
-    if (t > 1 && l > 0) {
-        if (post) launch_rows<true>(c, L, t, ctl, nr);
-        else launch_rows<false>(c, L, t, ctl, nr);
-        return;
-    }
-    if (t > 1) {  // a small finest level: any pattern
-        const SbView A = sbview(L);
-        const dim3 grid((unsigned)(((int64_t)L.n_nodes * t + kT - 1) / kT), nr);
-        auto go = [&](auto k) { launch_k(c, k, grid, kT, 0, A, L.binv.p, L.b.p, x, L.r.p, y, ctl); };
-        switch (t) {
-            case 2: post ? go(k_vc_rows_any<2, true>) : go(k_vc_rows_any<2, false>); break;
-            case 4: post ? go(k_vc_rows_any<4, true>) : go(k_vc_rows_any<4, false>); break;
-            case 8: post ? go(k_vc_rows_any<8, true>) : go(k_vc_rows_any<8, false>); break;
-            default: post ? go(k_vc_rows_any<16, true>) : go(k_vc_rows_any<16, false>); break;
+    if (L.n_nodes < kStagedRows) {  // 16 lanes a row
+        const dim3 g((unsigned)grid_of(16 * L.n_nodes), nr);
+        if (l > 0) {
+            const GeoView G = geo_of(L, L);
+            if (post) launch_k(c, k_vc_rows<16, true>, g, kT, 0, G, L.binv.p, L.b.p, x, L.r.p, y, ctl);
+            else launch_k(c, k_vc_rows<16, false>, g, kT, 0, G, L.binv.p, L.b.p, x, L.r.p, y, ctl);
+        } else {  // a small finest level: any pattern
+            const SbView A = sbview(L);
+            if (post) launch_k(c, k_vc_rows_any<16, true>, g, kT, 0, A, L.binv.p, L.b.p, x, L.r.p, y, ctl);
+            else launch_k(c, k_vc_rows_any<16, false>, g, kT, 0, A, L.binv.p, L.b.p, x, L.r.p, y, ctl);
         }
         return;
     }
@@ -3556,8 +3528,8 @@ int pcg_solve_mg_once(Ctx& c, const asend_solve_opts& o, asend_solve_stats* st, 
     c.d_r.alloc(std::max(c.d_r.n, (size_t)nrhs_all * nd));
     const int grid = grid_of(n);
     // eight lanes a row where one thread a row leaves more than half the GPU idle
-    const bool fp64_lanes = !mixed && !split && c.n_inst <= 1 && lanes_for(n) > 2;
-    const size_t n_part = (size_t)std::max({grid, H.box ? box_ctas(*H.box) : 0, fp64_lanes ? grid_of(8 * n) : 0});
+    const bool fp64_lanes = !mixed && !split && c.n_inst <= 1 && n <= kLaneRows;
+    const size_t n_part = (size_t)std::max({grid, H.box ? box_ctas(*H.box) : 0, fp64_lanes ? grid_of(4 * n) : 0});
     const int nr_max = std::min(nrhs_all, kMaxRhs);
     c.d_partials.alloc(std::max(c.d_partials.n, nr_max * n_part * kMaxRhs * 3));
     if (mixed) {
@@ -3644,35 +3616,35 @@ int pcg_solve_mg_once(Ctx& c, const asend_solve_opts& o, asend_solve_stats* st, 
         };
         auto launch_iteration = [&]() {
             if (mixed) {
-                k_mg_spmv_dot<float, float><<<dim3(grid, nr), kThreads, 0, c.stream>>>(M);
-                k_mg_update_xr<float><<<dim3(grid, nr), kThreads, 0, c.stream>>>(M);
+                launch_k(c, k_mg_spmv_dot<float, float>, dim3(grid, nr), kThreads, 0, M);
+                launch_k(c, k_mg_update_xr<float>, dim3(grid, nr), kThreads, 0, M);
             } else if (split) {
                 launch_split_product(c, M, dim3(grid_cg, nr));
                 launch_k(c, k_mg_update_xr_pair, dim3(grid_cg, nr), kThreads, 0, M);
             } else {
-                if (fp64_lanes) k_mg_spmv_dot_lanes<8><<<dim3(grid_of(8 * n), nr), kThreads, 0, c.stream>>>(M);
-                else k_mg_spmv_dot<double, double><<<dim3(grid, nr), kThreads, 0, c.stream>>>(M);
-                k_mg_update_xr<double><<<dim3(grid, nr), kThreads, 0, c.stream>>>(M);
+                if (fp64_lanes) launch_k(c, k_mg_spmv_dot_lanes, dim3(grid_of(4 * n), nr), kThreads, 0, M);
+                else launch_k(c, k_mg_spmv_dot<double, double>, dim3(grid, nr), kThreads, 0, M);
+                launch_k(c, k_mg_update_xr<double>, dim3(grid, nr), kThreads, 0, M);
             }
             vcycle(c, a.ctl, true, nr);
             if (mixed) {
-                k_mg_rz<float><<<dim3(grid, nr), kThreads, 0, c.stream>>>(M, 0);
-                k_mg_update_p<float><<<dim3(grid, nr), kThreads, 0, c.stream>>>(M);
+                launch_k(c, k_mg_rz<float>, dim3(grid, nr), kThreads, 0, M, 0);
+                launch_k(c, k_mg_update_p<float>, dim3(grid, nr), kThreads, 0, M);
             } else if (split) {
                 launch_k(c, k_mg_rz_pair, dim3(grid_cg, nr), kThreads, 0, M, 0);
                 launch_k(c, k_mg_update_p_pair, dim3(grid_cg, nr), kThreads, 0, M);
             } else {
-                k_mg_rz<double><<<dim3(grid, nr), kThreads, 0, c.stream>>>(M, 0);
-                k_mg_update_p<double><<<dim3(grid, nr), kThreads, 0, c.stream>>>(M);
+                launch_k(c, k_mg_rz<double>, dim3(grid, nr), kThreads, 0, M, 0);
+                launch_k(c, k_mg_update_p<double>, dim3(grid, nr), kThreads, 0, M);
             }
         };
         // V-cycle of every instance's current b0, then rz (and p = z on a
         // restart) for the instances the residual kernel marked
         auto launch_start = [&]() {
             vcycle(c, nullptr, false, nr);
-            if (mixed) k_mg_rz<float><<<dim3(grid, nr), kThreads, 0, c.stream>>>(M, 1);
+            if (mixed) launch_k(c, k_mg_rz<float>, dim3(grid, nr), kThreads, 0, M, 1);
             else if (split) launch_k(c, k_mg_rz_pair, dim3(grid_cg, nr), kThreads, 0, M, 1);
-            else k_mg_rz<double><<<dim3(grid, nr), kThreads, 0, c.stream>>>(M, 1);
+            else launch_k(c, k_mg_rz<double>, dim3(grid, nr), kThreads, 0, M, 1);
             c.launches += vcycle_launches(c) + 2;
         };
         launch_residual(warm ? 1 : kZeroStart);

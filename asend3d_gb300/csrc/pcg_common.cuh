@@ -558,13 +558,11 @@ __device__ __forceinline__ bool last_block_reduce(const PcgArgs& A, double (&val
     if (threadIdx.x == 0) {
 #pragma unroll
         for (int q = 0; q < NR * NV; ++q) A.partials[(size_t)blockIdx.x * (kMaxRhs * 3) + q] = flat[q];
-        __threadfence();
-        const uint32_t t = atomicAdd(ticket, 1u);
+        const uint32_t t = take_ticket(ticket);
         is_last = (t == (uint32_t)nb - 1);
     }
     __syncthreads();
     if (!is_last) return false;
-    __threadfence();
     double acc[NR * NV];
 #pragma unroll
     for (int q = 0; q < NR * NV; ++q) acc[q] = 0.0;
