@@ -125,6 +125,10 @@ struct MgHierarchy {
     DArr<double> blk_sf;          // penalty scale per block (instance)
     DArr<float> child;            // projected class matrices of the first coarsening [n_cls][27][576]
     bool child_ready = false;
+    // stacks: CTAs of the pair method's vector kernels (instance, rows; first
+    // CTA and their number per instance)
+    DArr<int32_t> cg_inst, cg_cta0, cg_ncta;
+    DArr<int2> cg_rows;
     // captured outer iterations, reused while the launch arguments match
     std::vector<std::pair<std::vector<uint8_t>, cudaGraphExec_t>> graphs;
     ~MgHierarchy() {
@@ -1586,7 +1590,10 @@ __global__ void __launch_bounds__(32 * kDenseRows) k_vc_dense(GeoView G, const f
 }
 
 // sum over the fine nodes f of w_x w_y w_z r(f) at node ol of coarse block d
-template <typename R>
+// LARGE: plane by plane, skipping the planes of an axis that is not coarsened
+// (there are enough nodes to hide the rounds of loads; the first coarsenings of a
+// stretched grid leave an axis as it is: 9 taps of 27; 140,000 nodes 12.8 -> 9.1 us).
+template <bool LARGE, typename R>
 __device__ __forceinline__ float restrict_at(const BlkDev& d, int ol, R&& r) {
     const int sj = d.nz + 1, si = (d.ny + 1) * sj;
     const int m[3] = {ol / si, (ol % si) / sj, ol % sj};
@@ -1599,6 +1606,26 @@ __device__ __forceinline__ float restrict_at(const BlkDev& d, int ol, R&& r) {
         on[ax][0] = m[ax] > 0 && x[ax] - fine_of(m[ax] - 1, nc[ax], nf[ax]) == 2;
         on[ax][1] = true;
         on[ax][2] = m[ax] < nc[ax] && fine_of(m[ax] + 1, nc[ax], nf[ax]) - x[ax] == 2;
+    }
+    if constexpr (LARGE) {
+        float s = 0.f;
+#pragma unroll
+        for (int a = 0; a < 3; ++a) {
+            if (!on[0][a]) continue;
+            float v[9];
+#pragma unroll
+            for (int q = 0; q < 9; ++q) {
+                const int b = q / 3, c = q % 3;
+                const size_t src = d.fnode0 + ((size_t)(x[0] + a - 1) * (d.fny + 1) + (x[1] + b - 1)) * (d.fnz + 1) + (x[2] + c - 1);
+                v[q] = on[1][b] && on[2][c] ? r(src) : 0.f;
+            }
+#pragma unroll
+            for (int q = 0; q < 9; ++q) {
+                const int b = q / 3, c = q % 3;
+                if (on[1][b] && on[2][c]) s = fmaf((a == 1 ? 1.f : 0.5f) * (b == 1 ? 1.f : 0.5f) * (c == 1 ? 1.f : 0.5f), v[q], s);
+            }
+        }
+        return s;
     }
     float v[27];
 #pragma unroll
@@ -1623,6 +1650,7 @@ __device__ __forceinline__ float restrict_at(const BlkDev& d, int ol, R&& r) {
 // contribute with 1/2 when they lie across a cell of two.  Fixed slots let the
 // 27 loads of a lane issue together.  The coarse level's first smoothing sweep
 // x4 = B^-1 b is fused in (binv non-null).
+template <bool LARGE>
 __global__ void __launch_bounds__(kT) k_vc_restrict(GeoView G, int n_fine, const float* in, float* out,
                                                     const float* __restrict__ binv, float4* x4, const Control* ctl) {
     pdl_begin();
@@ -1637,7 +1665,7 @@ __global__ void __launch_bounds__(kT) k_vc_restrict(GeoView G, int n_fine, const
         for (int q = 0; q < 3; ++q) B[q] = binv[9 * (size_t)o + 3 * comp + q];
     }
     const BlkDev d = blk_of(G, o);
-    const float s = restrict_at(d, o - d.node0, [in](size_t f) { return in[3 * f]; });
+    const float s = restrict_at<LARGE>(d, o - d.node0, [in](size_t f) { return in[3 * f]; });
     const int lane0 = (threadIdx.x & 31) & ~3;
     const float s0 = __shfl_sync(0xffffffffu, s, lane0), s1 = __shfl_sync(0xffffffffu, s, lane0 + 1),
                 s2 = __shfl_sync(0xffffffffu, s, lane0 + 2);
@@ -1918,7 +1946,20 @@ struct MgPcg {
     float4* x40;          // x4 = B^-1 r is fused into the kernels writing b0
     int n_inst;           // instances (1: a single model)
     int part_stride;      // CTAs of the partials array per right-hand side
+    const int2* cg_rows;  // stacks: rows of each CTA of the vector kernels (else nullptr)
 };
+
+// The rows of a thread of the pair method's vector kernels.
+struct RowRange {
+    int begin, end, step;
+};
+__device__ __forceinline__ RowRange cg_range(const MgPcg& M) {
+    if (M.cg_rows) {
+        const int2 q = M.cg_rows[blockIdx.x];
+        return {q.x + (int)threadIdx.x, q.y, (int)blockDim.x};
+    }
+    return {(int)(blockIdx.x * blockDim.x + threadIdx.x), M.a.n_rows, (int)(gridDim.x * blockDim.x)};
+}
 
 // The kernels' second grid dimension is the right-hand side: its slice of every
 // vector, scalar set, ticket and partials array (F32: the mixed method's FP32
@@ -2124,7 +2165,8 @@ __global__ void __launch_bounds__(kThreads) k_fold_pairs(MgPcg M, int all) {
     const PcgArgs& A = M.a;
     const RhsScalars* S = A.sc + cta_instance(A) * kMaxRhs;
     if (!all && !S[0].replace) return;
-    for (int row = blockIdx.x * blockDim.x + threadIdx.x; row < A.n_rows; row += gridDim.x * blockDim.x) {
+    const RowRange rows = cg_range(M);
+    for (int row = rows.begin; row < rows.end; row += rows.step) {
         F2 e[3];
         ld_pad_pair(M.xp, row, e);
         float t[3][3];
@@ -2250,7 +2292,8 @@ __global__ void __launch_bounds__(kThreads) k_mg_update_xr_pair(MgPcg M) {
     if (mg_done(A, S)) return;
     F2 rr{0.f, 0.f};
     const F2 alpha{S[0].alpha2[0], S[0].alpha2[1]};
-    for (int row = blockIdx.x * blockDim.x + threadIdx.x; row < A.n_rows; row += gridDim.x * blockDim.x) {
+    const RowRange rows = cg_range(M);
+    for (int row = rows.begin; row < rows.end; row += rows.step) {
         F2 pv[3], xv[3];
         ld_pad_pair(A.p, row, pv);
         ld_pad_pair(M.xp, row, xv);
@@ -2300,7 +2343,8 @@ __global__ void __launch_bounds__(kThreads) k_mg_rz_pair(MgPcg M, int mode) {
     if (mode == 1 && !S[0].refresh) return;
     const bool restart = mode == 1 && S[0].restart;
     F2 a0{0.f, 0.f}, a1{0.f, 0.f};
-    for (int row = blockIdx.x * blockDim.x + threadIdx.x; row < A.n_rows; row += gridDim.x * blockDim.x) {
+    const RowRange rows = cg_range(M);
+    for (int row = rows.begin; row < rows.end; row += rows.step) {
         const float4 z = M.z[row];
         const float zz[3] = {z.x, z.y, z.z};
         const float2* r = reinterpret_cast<const float2*>(A.r);
@@ -2350,7 +2394,8 @@ __global__ void __launch_bounds__(kThreads) k_mg_update_p_pair(MgPcg M) {
     RhsScalars* S = A.sc + cta_instance(A) * kMaxRhs;
     if (mg_done(A, S)) return;
     const F2 beta{S[0].beta2[0], S[0].beta2[1]};
-    for (int row = blockIdx.x * blockDim.x + threadIdx.x; row < A.n_rows; row += gridDim.x * blockDim.x) {
+    const RowRange rows = cg_range(M);
+    for (int row = rows.begin; row < rows.end; row += rows.step) {
         const float4 z = M.z[row];
         F2 pv[3];
         ld_pad_pair(A.p, row, pv);
@@ -2827,6 +2872,33 @@ void plan_tail(MgHierarchy& H) {
     ASEND_CUDA(cudaFuncSetAttribute(k_vc_tail, cudaFuncAttributeMaxDynamicSharedMemorySize, kTailSmem));
 }
 
+// CTAs of the pair method's vector kernels on a stack: whole tiles of 128 rows of
+// one instance, up to eight once that leaves two CTAs an SM.  A CTA's FP64
+// sums hold the FP64 pipe for some 50 x 64 cycles whatever its rows: with a tile
+// each, 1,606 tiles x 4 right-hand sides, they were two thirds of the kernels
+// (r.z 28.1 us, now 16.3; x, r update 30.7, now 25.3).  Not a function of the number
+// of right-hand sides: the sums' order is a case's own.
+void vector_ctas(Ctx& c, MgHierarchy& H) {
+    const int tiles = (c.n_nodes + kThreads - 1) / kThreads;
+    const int per = std::max(1, std::min(8, tiles / (2 * 152))) * kThreads;
+    std::vector<int32_t> inst, first, count;
+    std::vector<int2> rows;
+    for (int i = 0; i < c.n_inst; ++i) {
+        const int end = i + 1 < c.n_inst ? c.inst_node_ptr[i + 1] : c.n_nodes;
+        first.push_back((int32_t)rows.size());
+        for (int r = c.inst_node_ptr[i]; r < end; r += per) {
+            inst.push_back(i);
+            rows.push_back(make_int2(r, std::min(r + per, end)));
+        }
+        count.push_back((int32_t)rows.size() - first.back());
+    }
+    H.cg_inst.upload(inst, c.stream);
+    H.cg_cta0.upload(first, c.stream);
+    H.cg_ncta.upload(count, c.stream);
+    H.cg_rows.upload(rows, c.stream);
+    ASEND_CUDA(cudaStreamSynchronize(c.stream));  // the host tables go out of scope
+}
+
 void build_hierarchy(Ctx& c) {
     if (c.type != 8 && c.type != 81)
         throw InputError("multigrid needs structured hex8 / brickIM blocks (asend_set_block_structure or "
@@ -2971,6 +3043,7 @@ void build_hierarchy(Ctx& c) {
     H->dense.alloc(dense_tot);
     for (int l = 0; l < (int)H->L.size(); ++l) level_tables(c, *H, l);
     plan_tail(*H);
+    if (c.n_inst > 1) vector_ctas(c, *H);
     ASEND_CUDA(cudaStreamSynchronize(c.stream));
     c.mg = H;
 }
@@ -3113,8 +3186,8 @@ void restrict_to(Ctx& c, int l, const Control* ctl, int nr = 1) {
     MgLevel& L = *H.L[l];
     MgLevel& C = *H.L[l + 1];
     const bool last = (l + 2 == (int)H.L.size());  // the coarsest level is solved directly: no sweep
-    launch_k(c, k_vc_restrict, dim3(grid_of(4 * C.n_nodes), nr), kT, 0, geo_of(C, C), L.n_nodes, L.r.p, C.b.p,
-             last ? nullptr : C.binv.p, reinterpret_cast<float4*>(C.x4.p), ctl);
+    launch_k(c, C.n_nodes >= kStagedRows ? k_vc_restrict<true> : k_vc_restrict<false>, dim3(grid_of(4 * C.n_nodes), nr), kT,
+             0, geo_of(C, C), L.n_nodes, L.r.p, C.b.p, last ? nullptr : C.binv.p, reinterpret_cast<float4*>(C.x4.p), ctl);
 }
 
 void coarsest_solve(Ctx& c, const Control* ctl, int nr = 1) {
@@ -3545,8 +3618,9 @@ int pcg_solve_mg_once(Ctx& c, const asend_solve_opts& o, asend_solve_stats* st, 
     // one scalar set per instance and right-hand side, persistent so the
     // captured iteration graphs stay valid across solves
     const int NI = c.n_inst > 1 ? c.n_inst : 1;
-    // a batched stack keeps one CTA per 128 rows (its reductions are per instance)
+    // a batched stack's reductions are per instance: its own row ranges
     const int grid_cg = (split && NI == 1) ? std::min(grid, kPersistCtas) : grid;
+    const int grid_v = (split && NI > 1) ? (int)H.cg_rows.n : grid_cg;
     const size_t sc_need = sizeof(RhsScalars) * NI * kMaxRhs, tk_need = sizeof(uint32_t) * NI * 4 * kMaxRhs;
     if (c.pcg_sc.n < sc_need) c.pcg_sc.alloc(sc_need);
     if (c.pcg_ctl.n < sizeof(Control)) c.pcg_ctl.alloc(sizeof(Control));
@@ -3601,9 +3675,16 @@ int pcg_solve_mg_once(Ctx& c, const asend_solve_opts& o, asend_solve_stats* st, 
         }
         ASEND_CUDA(cudaMemsetAsync(d_sc, 0, sc_need, c.stream));
         ASEND_CUDA(cudaMemsetAsync(d_ctl, 0, sizeof(Control), c.stream));
+        MgPcg V = M;  // the pair method's vector kernels
+        if (split && NI > 1) {
+            V.cg_rows = H.cg_rows.p;
+            V.a.cta_inst = H.cg_inst.p;
+            V.a.inst_cta0 = H.cg_cta0.p;
+            V.a.inst_ncta = H.cg_ncta.p;
+        }
         auto launch_residual = [&](int init) {
             if (split) {  // x64 += e first (the instances being replaced), then r = f - A64 x64
-                launch_k(c, k_fold_pairs, dim3(grid_cg, nr), kThreads, 0, M, init);
+                launch_k(c, k_fold_pairs, dim3(grid_v, nr), kThreads, 0, V, init);
                 if (split_only)
                     launch_k(c, k_mg_residual_split, dim3(grid, nr), kThreads, 0, M, init, o.rel_tol * o.rel_tol);
                 else  // FP64-pipe bound: all 4 warps of every row tile in flight
@@ -3620,7 +3701,7 @@ int pcg_solve_mg_once(Ctx& c, const asend_solve_opts& o, asend_solve_stats* st, 
                 launch_k(c, k_mg_update_xr<float>, dim3(grid, nr), kThreads, 0, M);
             } else if (split) {
                 launch_split_product(c, M, dim3(grid_cg, nr));
-                launch_k(c, k_mg_update_xr_pair, dim3(grid_cg, nr), kThreads, 0, M);
+                launch_k(c, k_mg_update_xr_pair, dim3(grid_v, nr), kThreads, 0, V);
             } else {
                 if (fp64_lanes) launch_k(c, k_mg_spmv_dot_lanes, dim3(grid_of(4 * n), nr), kThreads, 0, M);
                 else launch_k(c, k_mg_spmv_dot<double, double>, dim3(grid, nr), kThreads, 0, M);
@@ -3631,8 +3712,8 @@ int pcg_solve_mg_once(Ctx& c, const asend_solve_opts& o, asend_solve_stats* st, 
                 launch_k(c, k_mg_rz<float>, dim3(grid, nr), kThreads, 0, M, 0);
                 launch_k(c, k_mg_update_p<float>, dim3(grid, nr), kThreads, 0, M);
             } else if (split) {
-                launch_k(c, k_mg_rz_pair, dim3(grid_cg, nr), kThreads, 0, M, 0);
-                launch_k(c, k_mg_update_p_pair, dim3(grid_cg, nr), kThreads, 0, M);
+                launch_k(c, k_mg_rz_pair, dim3(grid_v, nr), kThreads, 0, V, 0);
+                launch_k(c, k_mg_update_p_pair, dim3(grid_v, nr), kThreads, 0, V);
             } else {
                 launch_k(c, k_mg_rz<double>, dim3(grid, nr), kThreads, 0, M, 0);
                 launch_k(c, k_mg_update_p<double>, dim3(grid, nr), kThreads, 0, M);
@@ -3643,7 +3724,7 @@ int pcg_solve_mg_once(Ctx& c, const asend_solve_opts& o, asend_solve_stats* st, 
         auto launch_start = [&]() {
             vcycle(c, nullptr, false, nr);
             if (mixed) launch_k(c, k_mg_rz<float>, dim3(grid, nr), kThreads, 0, M, 1);
-            else if (split) launch_k(c, k_mg_rz_pair, dim3(grid_cg, nr), kThreads, 0, M, 1);
+            else if (split) launch_k(c, k_mg_rz_pair, dim3(grid_v, nr), kThreads, 0, V, 1);
             else launch_k(c, k_mg_rz<double>, dim3(grid, nr), kThreads, 0, M, 1);
             c.launches += vcycle_launches(c) + 2;
         };
@@ -3718,7 +3799,7 @@ int pcg_solve_mg_once(Ctx& c, const asend_solve_opts& o, asend_solve_stats* st, 
             since_repl += G;
         }
         if (split) {  // the solution: x64 + e
-            launch_k(c, k_fold_pairs, dim3(grid_cg, nr), kThreads, 0, M, 1);
+            launch_k(c, k_fold_pairs, dim3(grid_v, nr), kThreads, 0, V, 1);
             ++c.launches;
         }
         ASEND_CUDA(cudaMemcpyAsync(h, d_sc, sc_bytes, cudaMemcpyDeviceToHost, c.stream));
