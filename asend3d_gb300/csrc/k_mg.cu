@@ -966,8 +966,10 @@ struct F32Stage {
 };
 constexpr int kVcG = 4, kVcS = 2;  // stage shape of the finest level's products
 
-template <int G, int S, typename Epi>
-__device__ __forceinline__ bool f32_staged_slices(const SbView& A, const float4* __restrict__ x, unsigned char* smem,
+// y_k = A x_k for the right-hand sides k of the mask `on` (NR at most), whose
+// vectors are n_rows apart: a slice's values are staged once for all of them.
+template <int G, int S, int NR, typename Epi>
+__device__ __forceinline__ bool f32_staged_slices(const SbView& A, const float4* x, unsigned on, unsigned char* smem,
                                                   Epi&& epi) {
     using St = F32Stage<G, S>;
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -1017,7 +1019,9 @@ __device__ __forceinline__ bool f32_staged_slices(const SbView& A, const float4*
         const int ng = (int)(A.slice_off[sl + 1] - g0);
         const int len = row < A.n_rows ? A.row_len[row] : 0;
         const int nst = (ng + G - 1) / G;
-        float y[3] = {0.f, 0.f, 0.f};
+        float y[NR][3];
+#pragma unroll
+        for (int k = 0; k < NR; ++k) y[k][0] = y[k][1] = y[k][2] = 0.f;
         for (int k = 0; k < nst; ++k) {
             const int s = used % S;
             if (!__all_sync(0xffffffffu, mbar_wait(bars + s, (uint32_t)((used / S) & 1)))) {
@@ -1027,18 +1031,27 @@ __device__ __forceinline__ bool f32_staged_slices(const SbView& A, const float4*
             const float* hv = reinterpret_cast<const float*>(ring + s * St::kStage);
             const int* cv = reinterpret_cast<const int*>(hv + G * St::kVal);
             const int cnt = min(G, ng - k * G);
-            float4 p[G];
+            float4 p[G][NR];
 #pragma unroll
             for (int u = 0; u < G; ++u)
-                if (u < cnt && k * G + u < len) p[u] = x[cv[u * 32 + lane]];
+                if (u < cnt && k * G + u < len) {
+                    const float4* xc = x + cv[u * 32 + lane];
+#pragma unroll
+                    for (int h = 0; h < NR; ++h)
+                        if (NR == 1 || (on >> h & 1)) p[u][h] = xc[(size_t)h * A.n_rows];
+                }
 #pragma unroll
             for (int u = 0; u < G; ++u) {
                 if (u < cnt && k * G + u < len) {
                     const float* m = hv + u * St::kVal + lane;
 #pragma unroll
-                    for (int a = 0; a < 3; ++a)
-                        y[a] = fmaf(m[(a * 3) * 32], p[u].x,
-                                    fmaf(m[(a * 3 + 1) * 32], p[u].y, fmaf(m[(a * 3 + 2) * 32], p[u].z, y[a])));
+                    for (int a = 0; a < 3; ++a) {
+                        const float m0 = m[(a * 3) * 32], m1 = m[(a * 3 + 1) * 32], m2 = m[(a * 3 + 2) * 32];
+#pragma unroll
+                        for (int h = 0; h < NR; ++h)
+                            if (NR == 1 || (on >> h & 1))
+                                y[h][a] = fmaf(m0, p[u][h].x, fmaf(m1, p[u][h].y, fmaf(m2, p[u][h].z, y[h][a])));
+                    }
                 }
             }
             ++used;
@@ -1049,7 +1062,10 @@ __device__ __forceinline__ bool f32_staged_slices(const SbView& A, const float4*
             }
         }
         if (!ok) break;
-        if (row < A.n_rows) epi(row, y);
+        if (row < A.n_rows)
+#pragma unroll
+            for (int h = 0; h < NR; ++h)
+                if (NR == 1 || (on >> h & 1)) epi(row, h, y[h]);
     }
     if (!ok) {
         const int upto = __shfl_sync(0xffffffffu, issued, 0);
@@ -1059,41 +1075,62 @@ __device__ __forceinline__ bool f32_staged_slices(const SbView& A, const float4*
         // poison this warp's first row: the V-cycle output turns non-finite
         // and the solve reports it
         const int row = sl0 * 32 + lane;
-        if (row < A.n_rows) epi(row, {__int_as_float(0x7fc00000), 0.f, 0.f});
+        const float nan[3] = {__int_as_float(0x7fc00000), 0.f, 0.f};
+        for (int h = 0; row < A.n_rows && h < NR; ++h)
+            if (NR == 1 || (on >> h & 1)) epi(row, h, nan);
     }
     return ok;
 }
 
+// right-hand sides with an instance that still iterates, of nr (NR == 1: this one's)
+template <int NR>
+__device__ __forceinline__ unsigned vc_on(const Control* ctl, int nr) {
+    if constexpr (NR == 1) return !vc_idle(ctl);
+    unsigned on = 0;
+    for (int k = 0; k < nr; ++k) on |= (!ctl || ctl->active[k] != 0) << k;
+    return on;
+}
+
 // r = b - A x over the level's rows (staged)
+template <int NR>
 __global__ void __launch_bounds__(kT) k_vc_resid_staged(SbView A, const float* b, const float4* x, float* r,
-                                                        const Control* ctl) {
+                                                        const Control* ctl, int nr) {
     pdl_begin();
-    if (vc_idle(ctl)) return;
-    b = rhs_of(b, 3 * (size_t)A.n_rows);
-    x = rhs_of(x, A.n_rows);
-    r = rhs_of(r, 3 * (size_t)A.n_rows);
+    const unsigned on = vc_on<NR>(ctl, nr);
+    if (!on) return;
+    if constexpr (NR == 1) {
+        b = rhs_of(b, 3 * (size_t)A.n_rows);
+        x = rhs_of(x, A.n_rows);
+        r = rhs_of(r, 3 * (size_t)A.n_rows);
+    }
     extern __shared__ __align__(128) unsigned char vc_smem[];
-    f32_staged_slices<kVcG, kVcS>(A, x, vc_smem, [&](int row, const float (&y)[3]) {
+    f32_staged_slices<kVcG, kVcS, NR>(A, x, on, vc_smem, [&](int row, int h, const float (&y)[3]) {
+        const size_t at = 3 * ((size_t)h * A.n_rows + row);
 #pragma unroll
-        for (int a = 0; a < 3; ++a) r[3 * row + a] = b[3 * row + a] - y[a];
+        for (int a = 0; a < 3; ++a) r[at + a] = b[at + a] - y[a];
     });
 }
 
 // y4 = x + B^-1 (b - A x) over the level's rows (staged)
+template <int NR>
 __global__ void __launch_bounds__(kT) k_vc_post_staged(SbView A, const float* __restrict__ binv, const float* b,
-                                                       const float4* x, float4* y4, const Control* ctl) {
+                                                       const float4* x, float4* y4, const Control* ctl, int nr) {
     pdl_begin();
-    if (vc_idle(ctl)) return;
-    b = rhs_of(b, 3 * (size_t)A.n_rows);
-    x = rhs_of(x, A.n_rows);
-    y4 = rhs_of(y4, A.n_rows);
+    const unsigned on = vc_on<NR>(ctl, nr);
+    if (!on) return;
+    if constexpr (NR == 1) {
+        b = rhs_of(b, 3 * (size_t)A.n_rows);
+        x = rhs_of(x, A.n_rows);
+        y4 = rhs_of(y4, A.n_rows);
+    }
     extern __shared__ __align__(128) unsigned char vc_smem[];
-    f32_staged_slices<kVcG, kVcS>(A, x, vc_smem, [&](int row, const float (&y)[3]) {
-        const float d0 = b[3 * row] - y[0], d1 = b[3 * row + 1] - y[1], d2 = b[3 * row + 2] - y[2];
+    f32_staged_slices<kVcG, kVcS, NR>(A, x, on, vc_smem, [&](int row, int h, const float (&y)[3]) {
+        const size_t at = (size_t)h * A.n_rows + row;
+        const float d0 = b[3 * at] - y[0], d1 = b[3 * at + 1] - y[1], d2 = b[3 * at + 2] - y[2];
         const float* B = binv + 9 * (size_t)row;
-        const float4 xv = x[row];
-        y4[row] = make_float4(xv.x + B[0] * d0 + B[1] * d1 + B[2] * d2, xv.y + B[3] * d0 + B[4] * d1 + B[5] * d2,
-                              xv.z + B[6] * d0 + B[7] * d1 + B[8] * d2, 0.f);
+        const float4 xv = x[at];
+        y4[at] = make_float4(xv.x + B[0] * d0 + B[1] * d1 + B[2] * d2, xv.y + B[3] * d0 + B[4] * d1 + B[5] * d2,
+                             xv.z + B[6] * d0 + B[7] * d1 + B[8] * d2, 0.f);
     });
 }
 
@@ -3233,10 +3270,19 @@ void level_rows(Ctx& c, int l, bool post, const Control* ctl, int nr = 1) {
         }
         return;
     }
-    const dim3 grid(std::min(grid_of(L.n_nodes), kPersistCtas), nr);
+    // four right-hand sides by one reading of the values once every warp of the
+    // persistent grid has a slice (91,000 rows: a residual 44 -> 35 us, a
+    // post-smoothing 39 -> 32), else by a grid each (16,500 rows: 9.8 us, by one
+    // reading 14.9: a quarter of the warps)
+    const bool together = nr > 1 && L.n_nodes >= kPersistCtas * kT;
+    const dim3 grid(std::min(grid_of(L.n_nodes), kPersistCtas), together ? 1 : nr);
     const size_t smem = (size_t)F32Stage<kVcG, kVcS>::smem(kT);
-    if (post) launch_k(c, k_vc_post_staged, grid, kT, smem, sbview(L), L.binv.p, L.b.p, x, y, ctl);
-    else launch_k(c, k_vc_resid_staged, grid, kT, smem, sbview(L), L.b.p, x, L.r.p, ctl);
+    if (post)
+        launch_k(c, together ? k_vc_post_staged<kMaxRhs> : k_vc_post_staged<1>, grid, kT, smem, sbview(L), L.binv.p, L.b.p, x, y,
+                 ctl, nr);
+    else
+        launch_k(c, together ? k_vc_resid_staged<kMaxRhs> : k_vc_resid_staged<1>, grid, kT, smem, sbview(L), L.b.p, x, L.r.p, ctl,
+                 nr);
 }
 
 void fused_tail(Ctx& c, const Control* ctl, int nr) {
