@@ -313,11 +313,12 @@ __device__ __forceinline__ double warp_max(double v) {
     return v;
 }
 
-// Block-wide sum of K values per thread (K small); result valid in thread 0.
+// Block-wide sum of K values per thread (K small) over the first nt threads (the
+// others, whole warps, have returned); result valid in thread 0.
 template <int K>
-__device__ __forceinline__ void block_sum(double (&v)[K], double* smem /* [32*K] */) {
+__device__ __forceinline__ void block_sum(double (&v)[K], double* smem /* [32*K] */, int nt) {
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    const int nw = (blockDim.x + 31) >> 5;
+    const int nw = (nt + 31) >> 5;
 #pragma unroll
     for (int k = 0; k < K; ++k) v[k] = warp_sum(v[k]);
     if (lane == 0)
@@ -335,6 +336,11 @@ __device__ __forceinline__ void block_sum(double (&v)[K], double* smem /* [32*K]
                 if (o < nw) v[k] += __shfl_xor_sync(0xffffffffu, v[k], o);
         }
     }
+}
+
+template <int K>
+__device__ __forceinline__ void block_sum(double (&v)[K], double* smem) {
+    block_sum<K>(v, smem, blockDim.x);
 }
 
 // One more CTA done: what this thread wrote before is visible to whoever takes a

@@ -2256,51 +2256,63 @@ constexpr int kZeroStart = 2;  // init: the start is x = 0, so r = f
 
 // True residual r = f - A x from the operator's hi / lo values (split-only
 // assembly: no FP64 values) and the three FP32 parts of x written by the
-// fold, each term by res_term.
-__global__ void __launch_bounds__(kThreads) k_mg_residual_split(MgPcg M, int init, double tol2) {
+// fold, each term by res_term.  Three threads a row, a component each, in warps
+// of 32 rows (coalesced as one thread a row would be): with one thread a row a model
+// of 44,541 rows had 21 KB of loads in flight an SM (a solve's three evaluations 186 us,
+// now 106).  The first 128 threads then sum their rows' squares in the components'
+// order and make the reduction.
+constexpr int kResThreads = 3 * kThreads;
+__global__ void __launch_bounds__(kResThreads) k_mg_residual_split(MgPcg M, int init, double tol2) {
+    __shared__ F2 sq[3][kThreads];
     pdl_begin();
     M = rhs_view<false>(M);
     const PcgArgs& A = M.a;
     RhsScalars* S = A.sc + cta_instance(A) * kMaxRhs;
     if (!init && !S[0].replace) return;
-    F2 rr{0.f, 0.f};
-    double ff = 0.0;
-    for (int row = blockIdx.x * blockDim.x + threadIdx.x; row < A.n_rows; row += gridDim.x * blockDim.x) {
+    const int a = threadIdx.x / kThreads, rl = threadIdx.x % kThreads, row = blockIdx.x * kThreads + rl;
+    F2 q{0.f, 0.f};
+    if (row < A.n_rows) {
         const int lane = row & 31;
-        float Sm[3] = {0.f, 0.f, 0.f}, Cc[3] = {0.f, 0.f, 0.f}, Dd[3] = {0.f, 0.f, 0.f};
+        float Sm = 0.f, Cc = 0.f, Dd = 0.f;
         const int64_t g0 = A.slice_off[row >> 5];
         const int len = init == kZeroStart ? 0 : A.row_len[row];
+#pragma unroll 2
         for (int j = 0; j < len; ++j) {
             const int64_t g = g0 + j;
             const int c = A.col[g * 32 + lane];
             const float4 xh = M.xt[3 * (size_t)c], xl = M.xt[3 * (size_t)c + 1], xr = M.xt[3 * (size_t)c + 2];
-            const float* hv = A.v32 + (g * 9) * 32 + lane;
-            const float* lv = A.v32lo + (g * 9) * 32 + lane;
+            const float* hv = A.v32 + (g * 9 + 3 * a) * 32 + lane;
+            const float* lv = A.v32lo + (g * 9 + 3 * a) * 32 + lane;
+            res_term(hv[0], lv[0], xh.x, xl.x, xr.x, Sm, Cc, Dd);
+            res_term(hv[32], lv[32], xh.y, xl.y, xr.y, Sm, Cc, Dd);
+            res_term(hv[64], lv[64], xh.z, xl.z, xr.z, Sm, Cc, Dd);
+        }
+        const size_t o = 3 * (size_t)row + a;
+        // f - (S + C + D): the leading cancellation against f is exact in
+        // the pairs' TwoSum; C and D enter below it
+        const F2 y = f2_add(two_sum(Sm, Cc), F2{Dd, 0.f});
+        const F2 rv = f2_add(f2_of(A.f[o]), f2_neg(y));
+        st_pair(reinterpret_cast<float2*>(A.r), o, rv);
+        M.b0[o] = rv.h;
+        q = f2_mul(rv, rv);
+    }
+    sq[a][rl] = q;
+    __syncthreads();
+    if (a > 0) return;
+    F2 rr{0.f, 0.f};
+    double ff = 0.0;
+    if (row < A.n_rows)
 #pragma unroll
-            for (int a = 0; a < 3; ++a) {
-                res_term(hv[(3 * a) * 32], lv[(3 * a) * 32], xh.x, xl.x, xr.x, Sm[a], Cc[a], Dd[a]);
-                res_term(hv[(3 * a + 1) * 32], lv[(3 * a + 1) * 32], xh.y, xl.y, xr.y, Sm[a], Cc[a], Dd[a]);
-                res_term(hv[(3 * a + 2) * 32], lv[(3 * a + 2) * 32], xh.z, xl.z, xr.z, Sm[a], Cc[a], Dd[a]);
+        for (int k = 0; k < 3; ++k) {
+            rr = f2_add(rr, sq[k][rl]);
+            if (init) {
+                const double f = A.f[3 * (size_t)row + k];
+                ff += f * f;
             }
         }
-        float2* r = reinterpret_cast<float2*>(A.r);
-#pragma unroll
-        for (int a = 0; a < 3; ++a) {
-            const size_t o = 3 * (size_t)row + a;
-            const double f = A.f[o];
-            // f - (S + C + D): the leading cancellation against f is exact in
-            // the pairs' TwoSum; C and D enter below it
-            const F2 y = f2_add(two_sum(Sm[a], Cc[a]), F2{Dd[a], 0.f});
-            const F2 rv = f2_add(f2_of(f), f2_neg(y));
-            st_pair(r, o, rv);
-            M.b0[o] = rv.h;
-            rr = f2_add(rr, f2_mul(rv, rv));
-            if (init) ff += f * f;
-        }
-    }
     double d[1][2] = {{f2_dbl(rr), ff}};
     double tot[1][2];
-    if (last_block_reduce<1, 2>(A, d, 3, tot) && threadIdx.x == 0) {
+    if (last_block_reduce<1, 2>(A, d, 3, tot, kThreads) && threadIdx.x == 0) {
         RhsScalars& s = S[0];
         s.rr = tot[0][0];
         s.rr_last_true = tot[0][0];
@@ -3732,7 +3744,7 @@ int pcg_solve_mg_once(Ctx& c, const asend_solve_opts& o, asend_solve_stats* st, 
             if (split) {  // x64 += e first (the instances being replaced), then r = f - A64 x64
                 launch_k(c, k_fold_pairs, dim3(grid_v, nr), kThreads, 0, V, init);
                 if (split_only)
-                    launch_k(c, k_mg_residual_split, dim3(grid, nr), kThreads, 0, M, init, o.rel_tol * o.rel_tol);
+                    launch_k(c, k_mg_residual_split, dim3(grid, nr), kResThreads, 0, M, init, o.rel_tol * o.rel_tol);
                 else  // FP64-pipe bound: all 4 warps of every row tile in flight
                     launch_k(c, k_mg_residual<true>, dim3(grid, nr), kThreads, 0, M, init, o.rel_tol * o.rel_tol);
                 c.launches += 2;

@@ -538,10 +538,11 @@ __device__ __forceinline__ void precond(const PcgArgs& A, int row, const double 
 }
 
 // Last-CTA reduction of NV values per RHS; returns true in the last CTA
-// (all its threads) with tot[k][v] valid in every thread.
+// (all its threads) with tot[k][v] valid in every thread.  nt: the threads that
+// take part (the first; the other warps have returned).
 template <int NR, int NV>
 __device__ __forceinline__ bool last_block_reduce(const PcgArgs& A, double (&val)[NR][NV], int ticket_id,
-                                  double (&tot)[NR][NV]) {
+                                  double (&tot)[NR][NV], int nt) {
     __shared__ double sm[32 * NR * NV];
     __shared__ bool is_last;
     double flat[NR * NV];
@@ -549,7 +550,7 @@ __device__ __forceinline__ bool last_block_reduce(const PcgArgs& A, double (&val
     for (int k = 0; k < NR; ++k)
 #pragma unroll
         for (int v = 0; v < NV; ++v) flat[k * NV + v] = val[k][v];
-    block_sum<NR * NV>(flat, sm);
+    block_sum<NR * NV>(flat, sm, nt);
     // the CTAs of this CTA's instance reduce together (whole grid if single)
     const int inst = cta_instance(A);
     const int b0 = A.cta_inst ? A.inst_cta0[inst] : 0;
@@ -569,13 +570,13 @@ __device__ __forceinline__ bool last_block_reduce(const PcgArgs& A, double (&val
     // L2 reads (ld.global.cg: no stale L1 line after the fence) that may all
     // be in flight together, unlike volatile loads, which issue one by one
 #pragma unroll 4
-    for (int b = b0 + threadIdx.x; b < b0 + nb; b += blockDim.x) {
+    for (int b = b0 + threadIdx.x; b < b0 + nb; b += nt) {
         const double* pp = A.partials + (size_t)b * (kMaxRhs * 3);
 #pragma unroll
         for (int q = 0; q < NR * NV; ++q) acc[q] += __ldcg(pp + q);
     }
     __syncthreads();
-    block_sum<NR * NV>(acc, sm);
+    block_sum<NR * NV>(acc, sm, nt);
     if (threadIdx.x == 0) {
 #pragma unroll
         for (int q = 0; q < NR * NV; ++q) sm[q] = acc[q];
@@ -587,6 +588,11 @@ __device__ __forceinline__ bool last_block_reduce(const PcgArgs& A, double (&val
 #pragma unroll
         for (int v = 0; v < NV; ++v) tot[k][v] = sm[k * NV + v];
     return true;
+}
+template <int NR, int NV>
+__device__ __forceinline__ bool last_block_reduce(const PcgArgs& A, double (&val)[NR][NV], int ticket_id,
+                                  double (&tot)[NR][NV]) {
+    return last_block_reduce<NR, NV>(A, val, ticket_id, tot, (int)blockDim.x);
 }
 
 
