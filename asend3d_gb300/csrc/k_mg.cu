@@ -53,7 +53,7 @@ struct MgBlk {
     int nx = 0, ny = 0, nz = 0;   // cells
     int node0 = 0, el0 = 0;       // first node / element in the level numbering
     MgAxis ax[3];                 // maps from the finer level's block (levels >= 1)
-    int ox[3] = {0, 0, 0}, ol[3] = {0, 0, 0};  // offsets into the level's packed xs / lo, w
+    int ox[3] = {0, 0, 0};        // offsets into the level's packed xs
     double h[3] = {0, 0, 0};      // cell spacing per axis
     bool done = false;            // coarse enough: identity maps below this level
     int n_nodes() const { return (nx + 1) * (ny + 1) * (nz + 1); }
@@ -65,8 +65,8 @@ struct MgBlk {
 struct BlkDev {
     int nx, ny, nz, node0, el0;
     int fnx, fny, fnz, fnode0, fel0;
-    int ox0, ox1, ox2, ol0, ol1, ol2;
-    int dense0, pad;
+    int ox0, ox1, ox2;
+    int dense0;
 };
 
 struct MgLevel {
@@ -76,8 +76,7 @@ struct MgLevel {
     DArr<int32_t> pre_node, pre_el;  // per-block starts (+ total)
     DArr<int32_t> row_blk;        // block of each row (stacks of blocks)
     BlkDev one;                   // the descriptor of a lone block
-    DArr<int32_t> d_xs, d_lo;     // packed per block and axis
-    DArr<float> d_w;
+    DArr<int32_t> d_xs;           // packed per block and axis
     Sbell own;                    // pattern + FP32 values (levels >= 1)
     Sbell* A = nullptr;
     DArr<float> Ke;               // Galerkin element matrices [n_el][24][24]
@@ -209,8 +208,6 @@ struct LevelView {  // kernel-side view of a coarse level's blocks and maps from
     int n_blk;
     const BlkDev* blk;
     const int32_t* xs;
-    const int32_t* lo;
-    const float* w;
 };
 
 // Block of index idx: the largest b with pre[b] <= idx (pre ascending).
@@ -2786,9 +2783,6 @@ void level_tables(Ctx& c, MgHierarchy& H, int l) {
         d.ox0 = B.ox[0];
         d.ox1 = B.ox[1];
         d.ox2 = B.ox[2];
-        d.ol0 = B.ol[0];
-        d.ol1 = B.ol[1];
-        d.ol2 = B.ol[2];
         d.dense0 = (l + 1 == (int)H.L.size() && !H.h_dense0.empty()) ? H.h_dense0[b] : 0;
         pn[b] = B.node0;
         pe[b] = B.el0;
@@ -2823,8 +2817,6 @@ LevelView view_of(const MgLevel& L) {
     v.n_blk = (int)L.blk.size();
     v.blk = L.d_blk.p;
     v.xs = L.d_xs.p;
-    v.lo = L.d_lo.p;
-    v.w = L.d_w.p;
     return v;
 }
 
@@ -2872,8 +2864,10 @@ std::vector<MgBlk> level0_blocks(const Ctx& c) {
     return out;
 }
 
-// The fused tail takes every level below the finest whose vectors fit in a CTA's
-// shared memory; values go there from the coarsest level up while they fit.
+// The fused tail takes the levels below the finest of at most kTailRows rows whose
+// vectors fit in a CTA's shared memory (1,680 rows: 26 us in the tail, 23 as
+// launches of their own); values go there from the coarsest level up while
+// they fit.
 // Stacks keep one launch per level and step: a cluster per block needs more
 // SMs than there are, and the blocks' rows fill them as it is.
 void plan_tail(MgHierarchy& H) {
@@ -3000,8 +2994,7 @@ void build_hierarchy(Ctx& c) {
         }
         if (!any_block) break;
         auto L = std::make_unique<MgLevel>();
-        std::vector<int32_t> xs, lo;
-        std::vector<float> w;
+        std::vector<int32_t> xs;
         int node0 = 0, el0 = 0;
         for (int b = 0; b < nb; ++b) {
             const MgBlk& P = F.blk[b];
@@ -3023,10 +3016,7 @@ void build_hierarchy(Ctx& c) {
             el0 += B.n_el();
             for (int ax = 0; ax < 3; ++ax) {
                 B.ox[ax] = (int)xs.size();
-                B.ol[ax] = (int)lo.size();
                 xs.insert(xs.end(), B.ax[ax].xs.begin(), B.ax[ax].xs.end());
-                lo.insert(lo.end(), B.ax[ax].lo.begin(), B.ax[ax].lo.end());
-                w.insert(w.end(), B.ax[ax].w.begin(), B.ax[ax].w.end());
             }
             L->blk.push_back(B);
         }
@@ -3034,8 +3024,6 @@ void build_hierarchy(Ctx& c) {
         L->n_el = el0;
         L->n_dof = 3 * node0;
         L->d_xs.upload(xs, c.stream);
-        L->d_lo.upload(lo, c.stream);
-        L->d_w.upload(w, c.stream);
         // lumped Galerkin penalty: pen_c[I] = sum_i w_iI pen_f[i]
         L->h_pen.assign(L->n_dof, 0.f);
         for (int b = 0; b < nb; ++b) {
