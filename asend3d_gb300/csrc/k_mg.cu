@@ -1721,8 +1721,7 @@ __global__ void __launch_bounds__(kT) k_vc_restrict(GeoView G, int n_fine, const
 // any of it).  The prolongation is made by every CTA for its whole copy.  The
 // sums and their order are those of the separate kernels.  Bound by the barriers (1,500
 // cycles with the stores before them) and short dependent chains: 100 x 20 x 20
-// elements, levels of 936, 180 and 72 rows: nine launches of 28 us -> 19.5 serialised,
-// 12 with its loads under the kernel before it; 57 x 13 x 11: 16 -> 11.
+// elements (nine launches of 28 us) 19.5 us serialised, 57 x 13 x 11 (16 us) 11.2.
 __device__ __forceinline__ void tail_tables(const TailView& V, int l, float* tsm, int r0, int mine) {
     const TailView::Level& L = V.L[l];
     const BlkDev& d = L.d;
@@ -2865,9 +2864,9 @@ std::vector<MgBlk> level0_blocks(const Ctx& c) {
 }
 
 // The fused tail takes the levels below the finest of at most kTailRows rows whose
-// vectors fit in a CTA's shared memory (1,680 rows: 26 us in the tail, 23 as
-// launches of their own); values go there from the coarsest level up while
-// they fit.
+// vectors fit in a CTA's shared memory (a step on 57 x 13 x 11 brickIM elements takes
+// 8.2 ms with its level of 1,680 rows in the tail, 7.7 with launches of its own);
+// values go there from the coarsest level up while they fit.
 // Stacks keep one launch per level and step: a cluster per block needs more
 // SMs than there are, and the blocks' rows fill them as it is.
 void plan_tail(MgHierarchy& H) {
