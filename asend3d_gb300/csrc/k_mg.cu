@@ -3776,37 +3776,53 @@ int pcg_solve_mg_once(Ctx& c, const asend_solve_opts& o, asend_solve_stats* st, 
         launch_residual(warm ? 1 : kZeroStart);
         launch_start();
         ASEND_CUDA(cudaGetLastError());
-        // G iterations as one graph, kept with the hierarchy and reused while
-        // the launch arguments are the same (they fully define the graph)
+        // A chunk of iterations as one graph, kept with the hierarchy and reused
+        // while the launch arguments are the same (they fully define the graph)
         // (with everything else that changes the captured sequence: the
         // method, the chunk length, the product shape, the launch overlap, the
         // fused tail and the matrix-free plan)
-        std::vector<uint8_t> key(sizeof(MgPcg) + 4 * sizeof(int) + sizeof(void*));
-        std::memcpy(key.data(), &M, sizeof(MgPcg));
-        std::memcpy(key.data() + sizeof(MgPcg) + 4 * sizeof(int), &H.box, sizeof(void*));
-        const int extra[4] = {o.method, G, c.product_variant, (H.box_cycle ? 1 : 0) | (c.pdl ? 2 : 0) | (c.mg_tail ? 4 : 0)};
-        std::memcpy(key.data() + sizeof(MgPcg), extra, sizeof(extra));
-        cudaGraphExec_t exec = nullptr;
-        for (auto& g : H.graphs)
-            if (g.first == key) exec = g.second;
-        if (!exec) {
+        auto chunk = [&](int iterations) {
+            std::vector<uint8_t> key(sizeof(MgPcg) + 4 * sizeof(int) + sizeof(void*));
+            std::memcpy(key.data(), &M, sizeof(MgPcg));
+            std::memcpy(key.data() + sizeof(MgPcg) + 4 * sizeof(int), &H.box, sizeof(void*));
+            const int extra[4] = {o.method, iterations, c.product_variant,
+                                  (H.box_cycle ? 1 : 0) | (c.pdl ? 2 : 0) | (c.mg_tail ? 4 : 0)};
+            std::memcpy(key.data() + sizeof(MgPcg), extra, sizeof(extra));
+            for (auto& g : H.graphs)
+                if (g.first == key) return g.second;
             cudaGraph_t graph;
+            cudaGraphExec_t exec = nullptr;
             ASEND_CUDA(cudaStreamBeginCapture(c.stream, cudaStreamCaptureModeThreadLocal));
             launch_k(c, k_mg_count_active, nr, 32, 0, M);
-            for (int i = 0; i < G; ++i) launch_iteration();
+            for (int i = 0; i < iterations; ++i) launch_iteration();
             ASEND_CUDA(cudaStreamEndCapture(c.stream, &graph));
             ASEND_CUDA(cudaGraphInstantiate(&exec, graph, 0));
             ASEND_CUDA(cudaGraphDestroy(graph));
-            if (H.graphs.size() >= 8) {
+            if (H.graphs.size() >= 16) {
                 ASEND_CUDA(cudaGraphExecDestroy(H.graphs.front().second));
                 H.graphs.erase(H.graphs.begin());
             }
             H.graphs.emplace_back(key, exec);
-        }
+            return exec;
+        };
         const int per_iter = 4 + vcycle_launches(c);
         const size_t sc_bytes = sizeof(RhsScalars) * NI * kMaxRhs;
         int since_repl = 0;
+        // Expected number of iterations left, from each case's rate between two
+        // reads of its residual (0: not known).  A chunk runs to its end whatever
+        // converges in it, at some 13 empty launches an iteration, and the last one
+        // or two iterations after a true residual would be a chunk of their own:
+        // a short last stretch is launched as chunks of kShort (100 x 20 x 20 elements, 30
+        // iterations: 40 launched, now 32; the step 4.21 -> 4.06 ms.  Launched without a graph
+        // the stretch was slower, 4.37 ms: 13 launches an iteration are host-bound).
+        // Not where the chunks' ends decide more than the stop (mixed: the drop that
+        // asks for a true residual; replace_every).
+        constexpr int kShort = 2;
+        std::vector<double> rr_prev((size_t)NI * kMaxRhs, 0.0), log_rate((size_t)NI * kMaxRhs, 0.0);
+        int since_read = 0;
         for (;;) {
+            double left = 0.0;
+            bool known = !mixed && o.replace_every == 0;
             ASEND_CUDA(cudaMemcpyAsync(h, d_sc, sc_bytes, cudaMemcpyDeviceToHost, c.stream));
             ASEND_CUDA(cudaStreamSynchronize(c.stream));
             bool all_finished = true, any_replace = false, any_nonfinite = false;
@@ -3818,6 +3834,10 @@ int pcg_solve_mg_once(Ctx& c, const asend_solve_opts& o, asend_solve_stats* st, 
                 if (s.nonfinite) { any_nonfinite = true; continue; }
                 if (s.finished) continue;
                 all_finished = false;
+                if (since_read > 0 && rr_prev[q] > 0.0 && s.rr > 0.0) log_rate[q] = std::log(s.rr / rr_prev[q]) / since_read;
+                rr_prev[q] = s.done ? 0.0 : s.rr;
+                if (log_rate[q] < 0.0 && s.rr > s.target) left = std::max(left, std::log(s.target / s.rr) / log_rate[q]);
+                else known = false;
                 const bool drop = mixed && s.rr < 1e-4 * s.rr_last_true;
                 const bool periodic = o.replace_every > 0 && since_repl >= o.replace_every;
                 if (s.done || drop || periodic) {
@@ -3837,11 +3857,17 @@ int pcg_solve_mg_once(Ctx& c, const asend_solve_opts& o, asend_solve_stats* st, 
                 launch_start();
                 ++repl;
                 since_repl = 0;
+                since_read = 0;
                 continue;
             }
-            ASEND_CUDA(cudaGraphLaunch(exec, c.stream));
-            c.launches += (int64_t)per_iter * G + 1;
-            since_repl += G;
+            const int rest = known && left < G ? ((int)std::ceil(left) + kShort) / kShort * kShort : G;
+            const bool some = rest + kShort <= G && it_now + rest < max_it;
+            since_read = some ? rest : G;
+            for (int i = 0; i < since_read; i += some ? kShort : G) {
+                ASEND_CUDA(cudaGraphLaunch(chunk(some ? kShort : G), c.stream));
+                c.launches += (int64_t)per_iter * (some ? kShort : G) + 1;
+            }
+            since_repl += since_read;
         }
         if (split) {  // the solution: x64 + e
             launch_k(c, k_fold_pairs, dim3(grid_v, nr), kThreads, 0, V, 1);
