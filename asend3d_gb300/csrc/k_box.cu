@@ -247,6 +247,7 @@ __device__ __forceinline__ void box_march(const BoxArgs& A, const float4* __rest
     float2 e = has_el && first < it.nx ? A.E[el + (size_t)first * el_step] : make_float2(0.f, 0.f);
     __syncthreads();
     patterns(first, own, low);
+    __syncthreads();  // plane first is read: the first layer stores plane first + 2 over it
 #pragma unroll
     for (int c = 0; c < 3; ++c)
 #pragma unroll
