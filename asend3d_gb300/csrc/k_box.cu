@@ -579,7 +579,10 @@ BoxArgs args_of(const BoxPlan& P) { return BoxArgs{P.items.p, P.B[P.pairs].p, P.
 template <typename T, typename... K, typename... Args>
 void launch(Ctx& c, const BoxPlan& P, int nr, void (*k)(K...), Args... args) {
     const size_t smem = box_smem<T>(P.threads, P.halo);
-    ASEND_CUDA(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    // the attribute is the kernel's, not the context's: the largest launch's, so that
+    // threads with contexts of their own do not lower it under each other's launches
+    ASEND_CUDA(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                    (int)box_smem<T>(kBoxThreads, kBoxThreads / 2)));
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3((unsigned)P.n_items, (unsigned)nr);
     cfg.blockDim = dim3((unsigned)P.threads);

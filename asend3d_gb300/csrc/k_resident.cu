@@ -906,7 +906,8 @@ void launch_resident(Ctx& c, const asend_solve_opts& o, ResArgs a, const DynArgs
     std::memset(&none, 0, sizeof(none));
     const void* k = resident_kernel(mixed, nr, P.T >= 4, D != nullptr);
     const int threads = std::max({kResMinThreads, (P.VT + 31) / 32 * 32, (3 * P.rows + 31) / 32 * 32});
-    ASEND_CUDA(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)L.bytes));
+    // not this launch's size: the attribute is the kernel's, whichever context's thread sets it
+    ASEND_CUDA(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)P.smem));
     void* args[] = {&a, D ? const_cast<DynArgs*>(D) : &none};
     ASEND_CUDA(cudaLaunchCooperativeKernel(k, dim3(P.grid), dim3(threads), args, L.bytes, c.stream));
     ++c.launches;
