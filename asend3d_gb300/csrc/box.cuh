@@ -23,6 +23,7 @@ void box_post(Ctx& c, const BoxPlan& P, const float* binv, const float* b, const
               const pcg::Control* ctl, int nr);
 void box_power(Ctx& c, const BoxPlan& P, const float* dinv, const float4* x, float4* y4, float* nrm, int k,
                double* part, uint32_t* ticket);
+const void* box_patterns(const BoxPlan& P);  // pattern blocks the launches read (a captured graph keeps them)
 int box_ctas(const BoxPlan& P);  // CTAs of one launch (entries of a partials array)
 double box_product_bytes(const Ctx& c);
 

@@ -690,6 +690,7 @@ BoxPlan* box_plan(Ctx& c, const std::vector<std::array<int, 5>>& blocks) {
     return &P;
 }
 
+const void* box_patterns(const BoxPlan& P) { return P.B[P.pairs].p; }
 int box_ctas(const BoxPlan& P) { return P.n_items; }
 
 void box_product(Ctx& c, const BoxPlan& P, PcgArgs a, int nr, int part_stride) {

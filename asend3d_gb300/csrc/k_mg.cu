@@ -3780,11 +3780,12 @@ int pcg_solve_mg_once(Ctx& c, const asend_solve_opts& o, asend_solve_stats* st, 
         // while the launch arguments are the same (they fully define the graph)
         // (with everything else that changes the captured sequence: the
         // method, the chunk length, the product shape, the launch overlap, the
-        // fused tail and the matrix-free plan)
+        // fused tail, the matrix-free plan and which of its pattern blocks)
         auto chunk = [&](int iterations) {
-            std::vector<uint8_t> key(sizeof(MgPcg) + 4 * sizeof(int) + sizeof(void*));
+            const void* box[2] = {H.box, H.box ? box_patterns(*H.box) : nullptr};
+            std::vector<uint8_t> key(sizeof(MgPcg) + 4 * sizeof(int) + sizeof(box));
             std::memcpy(key.data(), &M, sizeof(MgPcg));
-            std::memcpy(key.data() + sizeof(MgPcg) + 4 * sizeof(int), &H.box, sizeof(void*));
+            std::memcpy(key.data() + sizeof(MgPcg) + 4 * sizeof(int), box, sizeof(box));
             const int extra[4] = {o.method, iterations, c.product_variant,
                                   (H.box_cycle ? 1 : 0) | (c.pdl ? 2 : 0) | (c.mg_tail ? 4 : 0)};
             std::memcpy(key.data() + sizeof(MgPcg), extra, sizeof(extra));
