@@ -3808,7 +3808,7 @@ int pcg_solve_mg_once(Ctx& c, const asend_solve_opts& o, asend_solve_stats* st, 
         };
         const int per_iter = 4 + vcycle_launches(c);
         const size_t sc_bytes = sizeof(RhsScalars) * NI * kMaxRhs;
-        int since_repl = 0;
+        int since_repl[kMaxRhs] = {};
         // Expected number of iterations left, from each case's rate between two
         // reads of its residual (0: not known).  A chunk runs to its end whatever
         // converges in it, at some 13 empty launches an iteration, and the last one
@@ -3821,43 +3821,68 @@ int pcg_solve_mg_once(Ctx& c, const asend_solve_opts& o, asend_solve_stats* st, 
         constexpr int kShort = 2;
         std::vector<double> rr_prev((size_t)NI * kMaxRhs, 0.0), log_rate((size_t)NI * kMaxRhs, 0.0);
         int since_read = 0;
+        // A load case ends by itself, as if it were alone: converged, non-finite in one
+        // of its instances, or at the cap.  From there its kernels have nothing to do.
+        bool ended[kMaxRhs] = {};
         for (;;) {
             double left = 0.0;
             bool known = !mixed && o.replace_every == 0;
             ASEND_CUDA(cudaMemcpyAsync(h, d_sc, sc_bytes, cudaMemcpyDeviceToHost, c.stream));
             ASEND_CUDA(cudaStreamSynchronize(c.stream));
-            bool all_finished = true, any_replace = false, any_nonfinite = false;
-            int it_now = 0;
-            for (int q = 0; q < NI * kMaxRhs; ++q) {
-                if (q % kMaxRhs >= nr) continue;
-                RhsScalars& s = h[q];
-                it_now = std::max(it_now, (int)s.iter);
-                if (s.nonfinite) { any_nonfinite = true; continue; }
-                if (s.finished) continue;
-                all_finished = false;
-                if (since_read > 0 && rr_prev[q] > 0.0 && s.rr > 0.0) log_rate[q] = std::log(s.rr / rr_prev[q]) / since_read;
-                rr_prev[q] = s.done ? 0.0 : s.rr;
-                if (log_rate[q] < 0.0 && s.rr > s.target) left = std::max(left, std::log(s.target / s.rr) / log_rate[q]);
-                else known = false;
-                const bool drop = mixed && s.rr < 1e-4 * s.rr_last_true;
-                const bool periodic = o.replace_every > 0 && since_repl >= o.replace_every;
-                if (s.done || drop || periodic) {
-                    s.replace = 1;
-                    any_replace = true;
+            bool any_replace = false, stopped = false, all_ended = true;
+            int it_now = 0;  // of the cases that go on
+            for (int k = 0; k < nr; ++k) {
+                if (ended[k]) continue;
+                bool open = false, bad = false;
+                int it_k = 0;
+                for (int q = k; q < NI * kMaxRhs; q += kMaxRhs) {
+                    it_k = std::max(it_k, (int)h[q].iter);
+                    bad |= h[q].nonfinite != 0;
+                    open |= !h[q].finished;
+                }
+                if (bad) status = std::max(status, (int)ASEND_NONFINITE);
+                else if (open && it_k >= max_it) status = std::max(status, (int)ASEND_MAX_ITER);
+                else if (open) {
+                    all_ended = false;
+                    it_now = std::max(it_now, it_k);
+                    continue;
+                }
+                ended[k] = true;
+                for (int q = k; q < NI * kMaxRhs; q += kMaxRhs) {
+                    stopped |= !h[q].done;
+                    h[q].done = 1;
                 }
             }
-            if (any_nonfinite) { status = ASEND_NONFINITE; break; }
-            if (all_finished) break;
-            if (it_now >= max_it) { status = std::max(status, (int)ASEND_MAX_ITER); break; }
+            if (all_ended) break;
+            for (int k = 0; k < nr; ++k) {
+                if (ended[k]) continue;
+                const bool periodic = o.replace_every > 0 && since_repl[k] >= o.replace_every;
+                bool replace = false;
+                for (int q = k; q < NI * kMaxRhs; q += kMaxRhs) {
+                    RhsScalars& s = h[q];
+                    if (s.finished) continue;
+                    if (since_read > 0 && rr_prev[q] > 0.0 && s.rr > 0.0)
+                        log_rate[q] = std::log(s.rr / rr_prev[q]) / since_read;
+                    rr_prev[q] = s.done ? 0.0 : s.rr;
+                    if (log_rate[q] < 0.0 && s.rr > s.target) left = std::max(left, std::log(s.target / s.rr) / log_rate[q]);
+                    else known = false;
+                    const bool drop = mixed && s.rr < 1e-4 * s.rr_last_true;
+                    if (s.done || drop || periodic) {
+                        s.replace = 1;
+                        replace = true;
+                    }
+                }
+                if (replace) since_repl[k] = 0;
+                any_replace |= replace;
+            }
+            if (any_replace || stopped) ASEND_CUDA(cudaMemcpyAsync(d_sc, h, sc_bytes, cudaMemcpyHostToDevice, c.stream));
             if (any_replace) {
                 // after convergence of the recurrence the last p update was
                 // skipped: the instance restarts its direction (p = z);
                 // otherwise p is kept
-                ASEND_CUDA(cudaMemcpyAsync(d_sc, h, sc_bytes, cudaMemcpyHostToDevice, c.stream));
                 launch_residual(0);
                 launch_start();
                 ++repl;
-                since_repl = 0;
                 since_read = 0;
                 continue;
             }
@@ -3868,7 +3893,7 @@ int pcg_solve_mg_once(Ctx& c, const asend_solve_opts& o, asend_solve_stats* st, 
                 ASEND_CUDA(cudaGraphLaunch(chunk(some ? kShort : G), c.stream));
                 c.launches += (int64_t)per_iter * (some ? kShort : G) + 1;
             }
-            since_repl += since_read;
+            for (int& n : since_repl) n += since_read;
         }
         if (split) {  // the solution: x64 + e
             launch_k(c, k_fold_pairs, dim3(grid_v, nr), kThreads, 0, V, 1);
