@@ -442,16 +442,16 @@ __global__ void __launch_bounds__(kBoxThreads, 1) k_box_power(BoxArgs X, const f
     __shared__ double sm[32];
     __shared__ bool last;
     const float inv = 1.f / nrm[k];
-    float acc = 0.f;  // of a few rows a thread; the sums over threads are FP64
+    double acc = 0.0;
     box_march<float>(X, x, smem, [&](int row, const float (&y)[3], const float (&)[3]) {
         const float* B = dinv + 9 * (size_t)row;
         const float z0 = inv * (B[0] * y[0] + B[1] * y[1] + B[2] * y[2]);
         const float z1 = inv * (B[3] * y[0] + B[4] * y[1] + B[5] * y[2]);
         const float z2 = inv * (B[6] * y[0] + B[7] * y[1] + B[8] * y[2]);
         y4[row] = make_float4(z0, z1, z2, 0.f);
-        acc += z0 * z0 + z1 * z1 + z2 * z2;
+        acc += (double)z0 * z0 + (double)z1 * z1 + (double)z2 * z2;
     });
-    double a[1] = {(double)acc};
+    double a[1] = {acc};
     block_sum<1>(a, sm);
     if (threadIdx.x == 0) {
         part[blockIdx.x] = a[0];

@@ -159,3 +159,13 @@ def test_rows(lib, dims, pad, sms):
     grow = np.abs(c.binv).sum(2)
     size = np.abs(c.b).max() + scale
     assert (np.abs(c.run(lib, POST, sms)[0][:, :3] - post) <= grow * (tol + 2.0**-22 * size) + 2.0**-23 * 5).all()
+
+
+@pytest.mark.parametrize("dims,pad,sms", CASES)
+def test_power_step_sums_in_64_bits(lib, dims, pad, sms):
+    """The CTAs' sums of the new vector's squares, positive terms: each addition
+    and product rounds by 2^-53."""
+    c = Case(dims, pad)
+    y, part, _ = c.run(lib, POWER, sms)
+    exact = (y[:, :3].astype(np.longdouble) ** 2).sum()
+    assert abs(part.sum(dtype=np.longdouble) - exact) <= 2 * y.size * 2.0**-53 * exact
