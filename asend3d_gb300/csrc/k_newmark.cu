@@ -218,7 +218,7 @@ int newmark_run(Ctx& c, const asend_solve_opts& o, int n_steps, const double* am
         ~TimeSolves() { c.time_solves = saved; }
     } time_guard{c, c.time_solves};
     c.time_solves = false;
-    // small enough for the resident PCG: the whole time loop in one launch
+    // small enough for the resident PCG: the time loop in the kernel, too
     const bool jac = o.precond == ASEND_PC_JACOBI || o.precond == ASEND_PC_BLOCK;
     const bool on_device = n_steps > 0 && jac && o.rel_tol > 0.0 && resident_usable(c, o, 1);
     if (on_device) {

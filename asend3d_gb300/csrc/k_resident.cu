@@ -39,6 +39,13 @@ using namespace pcg;
 
 constexpr int kMaxCtas = 160;       // CTAs at most: five words a polling lane
 constexpr int kPollLimit = 1 << 21; // polls (about 0.5 us each) before a wait gives up
+// Exchanges (two an iteration, two a step) after which a Newmark run's launch ends.
+// A launch takes every SM, so work of another context (another host thread's)
+// waits for its end: a 9 ms solve beside a run of 21,948 steps waited for all of it
+// (3.4 s) when the run was one launch, now 4 ms (the run on 525 rows) to 15 ms (on
+// 9,744).  The launches' starts cost nothing to be seen (60 time steps of 10,201 shell
+// rows, 40 of 1,225 hex8 rows: the times of one launch).
+constexpr unsigned long long kLaunchExchanges = 2048;
 
 struct ResArgs {
     int n_rows, n_dof, rows, T, K, KR, VT, next, cap, pc, zero_x, replace_every;
@@ -67,9 +74,10 @@ struct ResArgs {
 };
 
 // The Newmark loop of k_newmark.cu in the same kernel (DYN): its state vectors,
-// mass and damping values, and its records.
+// mass and damping values, and its records.  A launch goes on from step0 until
+// the last step or, after a whole step, kLaunchExchanges exchanges.
 struct DynArgs {
-    int n_steps, extrapolate, probe, hist_fields;
+    int n_steps, extrapolate, probe, hist_fields, step0;
     const double *m64, *d64, *f0, *pen, *amp;
     double cM, cD, dt, gamma, c1, c2;
     double *u, *v, *a, *up, *vp, *ap, *du_prev;
@@ -328,6 +336,7 @@ __global__ void __launch_bounds__(res_threads(NR), 1) k_resident_pcg(ResArgs A, 
         }
     for (int q = tid; q < NR * A.next * 3; q += blockDim.x) pe[q] = (TV)0;
     if (tid == 0) S.bad = 0;
+    if (DYN && blockIdx.x == 0 && tid == 0) D.out->next_step = D.n_steps;
     double x[NR], r[NR], di = 0.0;
     float bi[3] = {0.f, 0.f, 0.f};
     if (A.pc == ASEND_PC_JACOBI) {
@@ -482,9 +491,9 @@ __global__ void __launch_bounds__(res_threads(NR), 1) k_resident_pcg(ResArgs A, 
 
     int iter[NR], n_repl = 0, since = 0;
     bool fin[NR], nonfinite = false, timed_out = false;  // the same in every thread
-    int run_iters = 0, run_capped = 0;                   // DYN: over the steps
+    int run_iters = 0, run_capped = 0;                   // DYN: over the launch's steps
     double run_rel2 = 0.0;
-    for (int step = 0; step < (DYN ? D.n_steps : 1); ++step) {
+    for (int step = DYN ? D.step0 : 0; step < (DYN ? D.n_steps : 1); ++step) {
     // ---- right-hand side and initial residual
     since = 0;
     {
@@ -685,6 +694,10 @@ __global__ void __launch_bounds__(res_threads(NR), 1) k_resident_pcg(ResArgs A, 
             A.x[dof] = x[0];
         }
         if (step + 1 < D.n_steps) {
+            if (epoch - A.epoch0 >= kLaunchExchanges) {  // the state is stored: the next launch goes on from it
+                if (blockIdx.x == 0 && tid == 0) D.out->next_step = step + 1;
+                break;
+            }
             const double none[1] = {0.0};
             timed_out = !exchange<1, 1, kSum, true, false>(A, S, ndw, none, ++epoch, nothing);
             if (timed_out) break;
@@ -694,10 +707,10 @@ __global__ void __launch_bounds__(res_threads(NR), 1) k_resident_pcg(ResArgs A, 
     if (timed_out && tid == 0) *A.err = 1;
     if constexpr (DYN) {
         if (blockIdx.x == 0 && tid == 0) {
-            D.out->iterations = run_iters;
-            D.out->capped = run_capped;
+            D.out->iterations += run_iters;
+            D.out->capped |= run_capped;
             D.out->nonfinite = nonfinite || timed_out;
-            D.out->rel_residual = sqrt(run_rel2);
+            D.out->rel_residual = fmax(D.out->rel_residual, sqrt(run_rel2));
         }
         return;
     }
@@ -964,12 +977,16 @@ ResidentRun resident_newmark(Ctx& c, const asend_solve_opts& o, const NewmarkSta
     D.probe_hist = N.probe_hist;
     D.hist = N.hist;
     D.out = out.p;
-    launch_resident(c, o, a, &D, 1);
-    ResidentRun r;
-    ASEND_CUDA(cudaMemcpyAsync(&r, out.p, sizeof(r), cudaMemcpyDeviceToHost, c.stream));
-    ASEND_CUDA(cudaStreamSynchronize(c.stream));
-    if (r.nonfinite && resident_timed_out(c)) throw CudaError("a grid-wide wait of the resident PCG ran out");
-    return r;
+    for (;;) {
+        launch_resident(c, o, a, &D, 1);
+        ResidentRun r;
+        ASEND_CUDA(cudaMemcpyAsync(&r, out.p, sizeof(r), cudaMemcpyDeviceToHost, c.stream));
+        ASEND_CUDA(cudaStreamSynchronize(c.stream));
+        if (r.nonfinite && resident_timed_out(c)) throw CudaError("a grid-wide wait of the resident PCG ran out");
+        if (r.nonfinite || r.next_step >= N.n_steps) return r;
+        D.step0 = r.next_step;
+        a.zero_x = 0;
+    }
 }
 
 }  // namespace asend

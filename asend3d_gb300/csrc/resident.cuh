@@ -35,9 +35,9 @@ struct NewmarkState {
 };
 struct ResidentRun {
     double rel_residual;
-    int iterations, capped, nonfinite, pad;
+    int iterations, capped, nonfinite, next_step;
 };
-// The whole run in one launch (after resident_usable and pcg_precondition).
+// The whole run in a few launches (after resident_usable and pcg_precondition).
 ResidentRun resident_newmark(Ctx& c, const asend_solve_opts& o, const NewmarkState& N);
 
 }  // namespace asend
