@@ -880,6 +880,11 @@ void launch_resident(Ctx& c, const asend_solve_opts& o, ResArgs a, const DynArgs
         P.z.alloc((size_t)nr * c.n_dof);
         P.z.zero(c.stream);
     }
+    if (P.epoch >= 1ull << 63) {  // after 8.4 million launches: no word of the first ones may match again
+        P.words.zero(c.stream);
+        P.z.zero(c.stream);
+        P.epoch = 0;
+    }
     const int G = o.graph_iters > 0 ? o.graph_iters : 16, max_it = o.max_iter > 0 ? o.max_iter : c.n_dof;
     a.n_rows = c.A.n_rows;
     a.n_dof = c.n_dof;
