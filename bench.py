@@ -512,6 +512,31 @@ def ncu_traffic(kernel: int):
     return None
 
 
+def finest_product(kernel, shape, ms, nbytes, n_el, n_nodes, peak, peak_kind):
+    """One finest-level product of the multigrid CG (0: outer product, 1: V-cycle
+    residual, 2: post-smoothing) as time_mg_kernel measured it, under the name
+    of the kernel that ran: the library takes matrix-free kernels on blocks of
+    equal boxes (0 with the default shape only) and counts their compulsory bytes
+    (moduli and vectors) instead of the stored operator's.  Those are bound by
+    instruction issue (0) or latency: the bytes a second are given, but no share
+    of a peak, and the ncu traffic on record is the stored operator's."""
+    n_dof = 3 * n_nodes
+    box_bytes = 8 * n_el + (32 * n_nodes + 8 * n_dof, 16 * n_nodes + 8 * n_dof, 68 * n_nodes + 4 * n_dof)[kernel]
+    box = nbytes == box_bytes and (kernel > 0 or shape == 0)
+    if kernel == 0:
+        name = ("k_box_product" if box else PRODUCT_KERNEL[shape or 2]) + \
+            " (outer FP64-accurate product in FP32 pairs, + p.Ap)"
+    else:
+        form = "k_box_{}" if box else "k_vc_{}_staged" if n_nodes >= 8192 else "k_vc_rows_any ({})"
+        name = form.format(("resid", "post")[kernel - 1]) + \
+            (" (finest-level V-cycle residual, FP32)", " (finest-level post-smoothing, FP32, block Jacobi)")[kernel - 1]
+    gbps = nbytes / (ms * 1e-3) / 1e9
+    return {"kernel": name, "bound": ("issue" if kernel == 0 else "latency") if box else "hbm", "ms_per_launch": ms,
+            "algorithmic_bytes_per_launch": nbytes, "achieved": gbps, "unit": "GB/s", "peak": None if box else peak,
+            "peak_kind": None if box else f"of {peak_kind}", "frac": None if box else gbps / peak,
+            "traffic": None if box else ncu_traffic(kernel)}
+
+
 class ClockSampler:
     def __init__(self, gpu_index: int):
         self.proc = None
@@ -810,30 +835,14 @@ def run_ours(a):
     ms_plain = max_over_ranks(ms_plain, world)
     plain_value = replicas_value(n_dof, world, ms_plain)
 
-    # ---- roofline: the three kernels of every multigrid-CG iteration that
-    # read a full finest-level operator (each launched once per iteration),
-    # timed as they run in the step; the slowest is reported
+    # ---- roofline: the three finest-level products of every multigrid-CG
+    # iteration (each launched once per iteration), timed as they run in the
+    # step; the slowest is reported
     peak, peak_kind = measured_peak()
-    kern = {}
-    names = {0: f"{PRODUCT_KERNEL[shape]} (outer FP64-accurate product in FP32 pairs, + p.Ap)",
-             1: "k_box_resid (finest-level V-cycle residual, FP32)",
-             2: "k_box_post (finest-level post-smoothing, FP32, block Jacobi)"}
-    for k in (0, 1, 2):
-        ms_k, by_k = g.time_mg_kernel(k, _lib.METHOD_SPLIT, 30)
-        kern[k] = {"kernel": names[k], "ms_per_launch": ms_k, "algorithmic_bytes_per_launch": by_k,
-                   "achieved_GBps": by_k / (ms_k * 1e-3) / 1e9}
+    kern = [finest_product(k, shape, *g.time_mg_kernel(k, _lib.METHOD_SPLIT, 30), n_el, n_dof // 3, peak, peak_kind)
+            for k in (0, 1, 2)]
     ms64, by64 = g.time_mg_kernel(0, _lib.METHOD_FP64, 20)
-    top = max(kern, key=lambda k: kern[k]["ms_per_launch"])
-    achieved = kern[top]["achieved_GBps"]
-    # the matrix-free kernels (shape 0) are bound by instruction issue; the ncu
-    # traffic on record is the stored operator's
-    traffic = ncu_traffic if shape else lambda k: None
-    roof = {"bound": "hbm" if shape else "issue", "kernel": kern[top]["kernel"], "achieved": achieved, "peak": peak, "unit": "GB/s",
-            "frac": achieved / peak, "peak_kind": f"of {peak_kind}", "traffic": traffic(top),
-            "algorithmic_bytes_per_launch": kern[top]["algorithmic_bytes_per_launch"],
-            "ms_per_launch": kern[top]["ms_per_launch"],
-            "per_iteration_kernels": [dict(kern[k], frac=kern[k]["achieved_GBps"] / peak,
-                                           traffic=traffic(k)) for k in (0, 1, 2)],
+    roof = {**max(kern, key=lambda e: e["ms_per_launch"]), "per_iteration_kernels": kern,
             "fp64_outer_product": {"kernel": "k_mg_spmv_dot<double,double> (native FP64 values)",
                                    "ms_per_launch": ms64, "achieved_GBps": by64 / (ms64 * 1e-3) / 1e9},
             "product_shapes_ms_per_launch": {PRODUCT_KERNEL[v]: t for v, t in shape_ms.items()}}
