@@ -42,7 +42,7 @@
 // carried in the low parts: its error against 64 bits is 0.5 to 1.4e-15 of |K|
 // |u| (the assembled pair product's 2.7 to 9.5e-15).  Measured, product /
 // residual, against the assembled ones: 200 x 40 x 40: 36.8 / 12.3 us (118 /
-// 60); 128 x 64 x 64: 57 / 18.4 us (200 / 98); 100 x 20 x 20: 18.5 / 6.2 us (21
+// 60); 128 x 64 x 64: 57 / 18.4 us (200 / 98); 100 x 20 x 20: 16.5 / 6.2 us (21
 // / 10).  FP32 issue bounds the pair product (12 warps an SM at the registers
 // it needs; 62 % of the issue slots of the busy SMs), latency the FP32 ones.
 #include <algorithm>
@@ -526,7 +526,12 @@ void pattern_blocks(const double* K, float2* out) {
 // Shares of the blocks: the CTA size and the planes a CTA takes that finish
 // first.  A CTA's layers come one after the other (a layer below its first plane
 // is computed twice: + 1, and the first loads: + 0.5); a layer takes longer the
-// more warps share the SM, from about 0.45 of its time at kBoxThreads up.
+// more warps share the SM: the pair product of ten planes 26.7 us with 64 to 128
+// threads an SM, 35 to 36.5 with 192 to 256, 47.2 with 384 (one CTA or three), which
+// 0.45 + 0.55 of the full SM's threads follows within 0.07.  What it picks was
+// the fastest of the shares tried: 100 x 20 x 20 elements 96 threads x 1 plane 16.5 us
+// (384 x 3 22.6, 96 x 12 28.7), 200 x 40 x 40 384 x 7 36.9 us (384 x 8 40.6, 192 x 25
+// 71.2, 256 x 25 71.8).
 void make_items(BoxPlan& P, const std::vector<std::array<int, 5>>& blocks, const std::vector<int>& cls, int n_nodes,
                 int sms, std::vector<BoxItem>& items, std::vector<int32_t>& blk_of) {
     P.halo = 0;

@@ -1714,14 +1714,17 @@ __global__ void __launch_bounds__(kT) k_vc_restrict(GeoView G, int n_fine, const
 // a few hundred cycles of work that a launch of its own turns into 3 us (and
 // a step through global memory with a cluster barrier into 2.5, most of it the
 // fence), so the vectors live in every CTA's shared memory: a CTA stores its rows'
-// results into the other copies, and a cluster barrier ends the step.  Each CTA owns a run of rows of every level.  What does not change
-// between V-cycles -- the own rows' values, columns and smoother blocks, the rows
-// of the coarsest inverse, the transfers' indices -- is laid out before the wait
-// for the kernel that restricts to the first level (nothing in between writes
-// any of it).  The prolongation is made by every CTA for its whole copy.  The
+// results into the other copies, and a cluster barrier ends the step.  Each CTA owns
+// a run of rows of every level.  What does not change between V-cycles -- the own
+// rows' values, columns and smoother blocks, the rows of the coarsest inverse, the
+// transfers' indices -- is laid out before the wait for the kernel that restricts
+// to the first level (nothing in between writes any of it); that hides these loads
+// with launch overlap only, which is off by default (a 100 x 20 x 20 solve 3.10 ms,
+// with overlap 3.17).  The prolongation is made by every CTA for its whole copy.  The
 // sums and their order are those of the separate kernels.  Bound by the barriers (1,500
 // cycles with the stores before them) and short dependent chains: 100 x 20 x 20
-// elements (nine launches of 28 us) 19.5 us serialised, 57 x 13 x 11 (16 us) 11.2.
+// elements (nine launches of 28 us) 19.5 us launched alone, 23.9 among a step's
+// kernels; 57 x 13 x 11 (16 us) 11.2 alone.
 __device__ __forceinline__ void tail_tables(const TailView& V, int l, float* tsm, int r0, int mine) {
     const TailView::Level& L = V.L[l];
     const BlkDev& d = L.d;
@@ -2864,9 +2867,12 @@ std::vector<MgBlk> level0_blocks(const Ctx& c) {
 }
 
 // The fused tail takes the levels below the finest of at most kTailRows rows whose
-// vectors fit in a CTA's shared memory (a step on 57 x 13 x 11 brickIM elements takes
-// 8.2 ms with its level of 1,680 rows in the tail, 7.7 with launches of its own);
-// values go there from the coarsest level up while they fit.
+// vectors fit in a CTA's shared memory; values go there from the coarsest level up
+// while they fit.  1,024 rows are one pass of the cluster's CTAs (64 rows of 16
+// lanes each); a level that needs a second one is slower there than as launches:
+// solves with a level of 595, 684, 882, 1,008 rows in the tail 1.17, 1.39, 1.39, 1.52
+// ms (as launches 1.23, 1.46, 1.45, 1.57), of 1,056, 1,176, 1,392, 1,512, 1,680 rows
+// 1.58, 1.51, 1.75, 1.52, 2.31 ms (1.58, 1.49, 1.72, 1.48, 2.18).
 // Stacks keep one launch per level and step: a cluster per block needs more
 // SMs than there are, and the blocks' rows fill them as it is.
 void plan_tail(MgHierarchy& H) {
@@ -3645,7 +3651,7 @@ int pcg_solve_mg_once(Ctx& c, const asend_solve_opts& o, asend_solve_stats* st, 
     if (!warm) ASEND_CUDA(cudaMemsetAsync(d_x, 0, (size_t)nrhs_all * nd * sizeof(double), c.stream));
     c.d_r.alloc(std::max(c.d_r.n, (size_t)nrhs_all * nd));
     const int grid = grid_of(n);
-    // eight lanes a row where one thread a row leaves more than half the GPU idle
+    // four lanes a row where one thread a row leaves SMs idle
     const bool fp64_lanes = !mixed && !split && c.n_inst <= 1 && n <= kLaneRows;
     const size_t n_part = (size_t)std::max({grid, H.box ? box_ctas(*H.box) : 0, fp64_lanes ? grid_of(4 * n) : 0});
     const int nr_max = std::min(nrhs_all, kMaxRhs);
